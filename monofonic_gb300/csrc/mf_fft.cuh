@@ -283,13 +283,31 @@ __host__ __device__ constexpr int plan_lcur(int L, int maxr, int s) {
 // radix-8-first plans of lengths 16..384 that are multiples of 16, where
 // layout 1 takes up to twice as many for some exchanges.
 template <int LAYOUT>
-__device__ __forceinline__ int pidx(int e) {
+__host__ __device__ __forceinline__ constexpr int pidx(int e) {
   if constexpr (LAYOUT == 1) return e + (e >> 4);
   else if constexpr (LAYOUT == 2) return e ^ ((e >> 3) & 1);
   else if constexpr (LAYOUT == 12) return e ^ ((e >> 2) & 15);
   else if constexpr (LAYOUT == 13) return e ^ ((e >> 3) & 15);
   else return e;
 }
+// the slot of element r + c, where r depends on the thread and c is a constant
+// once the surrounding loop is unrolled; rbits: the bits that r can have set.
+// Written as (value that depends on r) + constant, so that the accesses of one
+// thread become immediate offsets from a few registers instead of one chain
+// of index arithmetic per element: the XOR layouts are linear over bits and
+// change only the low four, so with r and c disjoint the slot is
+// (pidx(r) ^ low bits of pidx(c)) + high bits of c
+template <int LAYOUT>
+__device__ __forceinline__ int pidx_split(int r, int c, int rbits) {
+  if constexpr (LAYOUT == 0) {
+    return r + c;
+  } else if constexpr (LAYOUT == 1) {
+    return (c & 15) == 0 ? pidx<1>(r) + (c + (c >> 4)) : pidx<1>(r + c);
+  } else {
+    return (rbits & c) == 0 ? (pidx<LAYOUT>(r) ^ (pidx<LAYOUT>(c) & 15)) + (c & ~15) : pidx<LAYOUT>(r + c);
+  }
+}
+__host__ __device__ constexpr bool is_pow2(int x) { return x > 0 && (x & (x - 1)) == 0; }
 __host__ __device__ constexpr int padded_len(int L, int layout) { return layout == 1 ? L + (L >> 4) + 1 : L; }
 // exchange layout of a contiguous line of length L
 __host__ __device__ constexpr int zlayout(int L) {
@@ -333,13 +351,35 @@ struct LineFFT {
   static constexpr int R0 = plan_radix(L, MAXR, 0);
   static constexpr int RL = plan_radix(L, MAXR, NS - 1);
 
-  // stage-0 input element index of register slot (m*R0 + p)
-  __device__ static __forceinline__ int in_index(int t, int slot) {
-    return t + (slot / R0) * TPL + (slot % R0) * (L / R0);
+  // Element indices are a part that depends on the thread plus a constant of
+  // the register slot (a constant once the slot loops are unrolled).
+  // stage-0 input element index of register slot (m*R0 + p): t + in_const(slot)
+  __device__ static __forceinline__ constexpr int in_const(int slot) {
+    return (slot / R0) * TPL + (slot % R0) * (L / R0);
   }
-  // last-stage output element index of register slot (m*RL + q)
-  __device__ static __forceinline__ int out_index(int t, int slot) {
-    return t + (slot / RL) * TPL + (slot % RL) * (L / RL);
+  __device__ static __forceinline__ int in_index(int t, int slot) { return t + in_const(slot); }
+  // last-stage output element index of register slot (m*RL + q): t + out_const(slot)
+  __device__ static __forceinline__ constexpr int out_const(int slot) {
+    return (slot / RL) * TPL + (slot % RL) * (L / RL);
+  }
+  __device__ static __forceinline__ int out_index(int t, int slot) { return t + out_const(slot); }
+  static constexpr int TBITS = is_pow2(TPL) ? TPL - 1 : -1;  // bits of t (-1: any)
+  // shared-memory slots of the stage-0 inputs / last-stage outputs
+  __device__ static __forceinline__ int in_slot(int t, int slot) {
+    return pidx_split<LAYOUT>(t, in_const(slot), TBITS);
+  }
+  __device__ static __forceinline__ int out_slot(int t, int slot) {
+    return pidx_split<LAYOUT>(t, out_const(slot), TBITS);
+  }
+
+  // k = b mod LC of butterfly b = t + m TPL, as (part of t) + constant of m
+  // where one of TPL and LC divides the other
+  template <int LC>
+  __device__ static __forceinline__ int bfly_k(int t, int m) {
+    if constexpr (LC == 1) return 0;
+    else if constexpr (TPL % LC == 0) return (int)((unsigned)t % (unsigned)LC);
+    else if constexpr (LC % TPL == 0) return t + (m % (LC / TPL)) * TPL;
+    else return (int)((unsigned)(t + m * TPL) % (unsigned)LC);
   }
 
   template <int S>
@@ -366,8 +406,7 @@ struct LineFFT {
 #pragma unroll
     for (int m = 0; m < NB; ++m) {
       if constexpr (LC > 1) {
-        const int b = t + m * TPL;
-        const int k = b % LC;
+        const int k = bfly_k<LC>(t, m);
         constexpr int STR = L / (LC * R);
 #pragma unroll
         for (int p = 1; p < R; ++p) {
@@ -379,7 +418,8 @@ struct LineFFT {
     }
   }
 
-  // write stage-S outputs to shared memory (element e at sm[e*cs])
+  // write stage-S outputs to shared memory (element e at sm[e*cs]): output q
+  // of butterfly b is element (b - k) R + k + q LC
   template <int S>
   __device__ static __forceinline__ void write_out(const C (&v)[E], int t, C* sm, int cs) {
     constexpr int R = plan_radix(L, MAXR, S);
@@ -387,11 +427,25 @@ struct LineFFT {
     constexpr int NB = E / R;
 #pragma unroll
     for (int m = 0; m < NB; ++m) {
-      const int b = t + m * TPL;
-      const int k = b % LC;
-      const int base = (b - k) * R + k;
+      int r, c, rbits;
+      if constexpr (TPL % LC == 0) {
+        const int k = bfly_k<LC>(t, m);
+        r = (t - k) * R + k;
+        c = m * TPL * R;
+        rbits = (is_pow2(TPL) && is_pow2(R)) ? ((LC - 1) | ((TPL - LC) * R)) : -1;
+      } else if constexpr (LC % TPL == 0) {
+        constexpr int QN = LC / TPL;
+        r = t;
+        c = (m / QN) * LC * R + (m % QN) * TPL;
+        rbits = TBITS;
+      } else {
+        const int k = bfly_k<LC>(t, m);
+        r = (t + m * TPL - k) * R + k;
+        c = 0;
+        rbits = -1;
+      }
 #pragma unroll
-      for (int q = 0; q < R; ++q) sm[pidx<LAYOUT>(base + q * LC) * cs] = v[m * R + q];
+      for (int q = 0; q < R; ++q) sm[pidx_split<LAYOUT>(r, c + q * LC, rbits) * cs] = v[m * R + q];
     }
   }
 
@@ -402,9 +456,8 @@ struct LineFFT {
     constexpr int NB = E / R;
 #pragma unroll
     for (int m = 0; m < NB; ++m) {
-      const int b = t + m * TPL;
 #pragma unroll
-      for (int p = 0; p < R; ++p) v[m * R + p] = sm[pidx<LAYOUT>(b + p * (L / R)) * cs];
+      for (int p = 0; p < R; ++p) v[m * R + p] = sm[pidx_split<LAYOUT>(t, m * TPL + p * (L / R), TBITS) * cs];
     }
   }
 

@@ -206,6 +206,27 @@ k_colfft3s(OP op, const cplx<T>* __restrict__ tw, int ncols) {
 //     xform(z, slab, e, col, raw), store_z(z, slab, e, col, v)
 //     (+ kPrefetch: prefetch/store_pre on the same coordinates)
 // ---------------------------------------------------------------------------
+// the tile a persistent CTA works on, (column tile, slab, operand), stepped by
+// the grid size with carries instead of a division per tile
+struct TilePos {
+  int ct, slab, z;
+  __device__ __forceinline__ static TilePos of(int tl, int ntc, int nslab) {
+    TilePos p;
+    p.ct = tl % ntc;
+    const int r = tl / ntc;
+    p.slab = r % nslab;
+    p.z = r / nslab;
+    return p;
+  }
+  // step: the position of tile index gridDim.x
+  __device__ __forceinline__ TilePos next(const TilePos& step, int ntc, int nslab) const {
+    TilePos p{ct + step.ct, slab + step.slab, z + step.z};
+    if (p.ct >= ntc) { p.ct -= ntc; ++p.slab; }
+    if (p.slab >= nslab) { p.slab -= nslab; ++p.z; }
+    return p;
+  }
+};
+
 template <typename T, int L, bool INV, int NCOL, class OP>
 __global__ void __launch_bounds__(NCOL * LineFFT<T, L, INV, MF_COL_MAXR>::TPL,
                                   col_minb(NCOL * LineFFT<T, L, INV, MF_COL_MAXR>::TPL,
@@ -214,19 +235,18 @@ k_colfft_pipe(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nsl
   constexpr int LAY = col_layout<T, NCOL, OP>();
   using F = LineFFT<T, L, INV, MF_COL_MAXR, LAY>;
   using C = cplx<T>;
+  using I = LineIdx<F::TPL>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf0 = reinterpret_cast<C*>(smem_raw);
   C* buf1 = buf0 + L * NCOL;
   const int c = threadIdx.x, t = threadIdx.y;
   const int total = ntc * nslab * nz;
-  auto issue = [&](int tl, C* buf) {
-    const int ct = tl % ntc, r = tl / ntc, slab = r % nslab, z = r / nslab;
-    const int col = ct * NCOL + c;
+  auto issue = [&](const TilePos& p, C* buf) {
+    const int col = p.ct * NCOL + c;
 #pragma unroll
     for (int s = 0; s < F::E; ++s) {
-      const int e = F::in_index(t, s);
-      C* d = buf + pidx<LAY>(e) * NCOL + c;
-      const C* g = (col < ncols) ? op.srcp(z, slab, e, col) : nullptr;
+      C* d = buf + F::in_slot(t, s) * NCOL + c;
+      const C* g = (col < ncols) ? op.srcp(p.z, p.slab, I{t, F::in_const(s)}, col) : nullptr;
       if (g) {
         if constexpr (sizeof(C) == 16) cp_async16(d, g); else cp_async8(d, g);
       } else {
@@ -236,45 +256,44 @@ k_colfft_pipe(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nsl
     cp_async_commit();
   };
   int tl = blockIdx.x;
-  if (tl < total) issue(tl, buf0); else cp_async_commit();
+  const TilePos step = TilePos::of(gridDim.x, ntc, nslab);
+  TilePos nx = TilePos::of(tl, ntc, nslab);
+  if (tl < total) issue(nx, buf0); else cp_async_commit();
   for (int it = 0; tl < total; tl += gridDim.x, ++it) {
     C* cur = (it & 1) ? buf1 : buf0;
     C* nxt = (it & 1) ? buf0 : buf1;
-    const int tn = tl + gridDim.x;
-    if (tn < total) issue(tn, nxt); else cp_async_commit();
+    const TilePos p = nx;
+    nx = p.next(step, ntc, nslab);
+    if (tl + (int)gridDim.x < total) issue(nx, nxt); else cp_async_commit();
     cp_async_wait<1>();
-    const int ct = tl % ntc, r = tl / ntc, slab = r % nslab, z = r / nslab;
-    const int col = ct * NCOL + c;
+    const int col = p.ct * NCOL + c;
     const bool valid = col < ncols;
     C v[F::E];
     if constexpr (has_tile_prep<OP>::value) {
-      const auto tp = op.tile_prep(z, slab, col);
+      const auto tp = op.tile_prep(p.z, p.slab, col);
 #pragma unroll
-      for (int s = 0; s < F::E; ++s) {
-        const int e = F::in_index(t, s);
-        v[s] = valid ? op.xform_tile(tp, e, cur[pidx<LAY>(e) * NCOL + c]) : mkc<T>(T(0), T(0));
-      }
+      for (int s = 0; s < F::E; ++s)
+        v[s] = op.xform_tile(tp, I{t, F::in_const(s)}, cur[F::in_slot(t, s) * NCOL + c]);
     } else {
 #pragma unroll
-      for (int s = 0; s < F::E; ++s) {
-        const int e = F::in_index(t, s);
-        v[s] = valid ? op.xform(z, slab, e, col, cur[pidx<LAY>(e) * NCOL + c]) : mkc<T>(T(0), T(0));
-      }
+      for (int s = 0; s < F::E; ++s)
+        v[s] = op.xform(p.z, p.slab, I{t, F::in_const(s)}, col, cur[F::in_slot(t, s) * NCOL + c]);
     }
     if constexpr (OP::kPrefetch) {
       C pre[F::E];
 #pragma unroll
-      for (int s = 0; s < F::E; ++s) pre[s] = valid ? op.prefetch(slab, F::out_index(t, s), col) : mkc<T>(T(0), T(0));
+      for (int s = 0; s < F::E; ++s)
+        pre[s] = valid ? op.prefetch(p.slab, I{t, F::out_const(s)}, col) : mkc<T>(T(0), T(0));
       F::run(v, t, cur + c, NCOL, tw, SyncBlock{});
       if (valid) {
 #pragma unroll
-        for (int s = 0; s < F::E; ++s) op.store_pre(slab, F::out_index(t, s), col, v[s], pre[s]);
+        for (int s = 0; s < F::E; ++s) op.store_pre(p.slab, I{t, F::out_const(s)}, col, v[s], pre[s]);
       }
     } else {
       F::run(v, t, cur + c, NCOL, tw, SyncBlock{});
       if (valid) {
 #pragma unroll
-        for (int s = 0; s < F::E; ++s) op.store_z(z, slab, F::out_index(t, s), col, v[s]);
+        for (int s = 0; s < F::E; ++s) op.store_z(p.z, p.slab, I{t, F::out_const(s)}, col, v[s]);
       }
     }
     __syncthreads();  // cur is refilled by the next iteration's copies
@@ -395,16 +414,16 @@ k_colfft_trunc(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int ns
   C* buf0 = reinterpret_cast<C*>(smem_raw);
   C* buf1 = buf0 + L * NCOL;
   const int c = threadIdx.x, t = threadIdx.y;
+  using I = LineIdx<FF::TPL>;
   const int total = ntc * nslab;
-  auto issue = [&](int tl, C* buf) {
-    const int ct = tl % ntc, slab = tl / ntc;
-    const int col = ct * NCOL + c;
+  auto issue = [&](const TilePos& p, C* buf) {
+    const int col = p.ct * NCOL + c;
 #pragma unroll
     for (int s = 0; s < FF::E; ++s) {
-      const int e = FF::in_index(t, s);
-      C* d = buf + pidx<LAY>(e) * NCOL + c;
+      C* d = buf + FF::in_slot(t, s) * NCOL + c;
+      const C* g = op.at(p.slab, I{t, FF::in_const(s)}, col);
       if (col < ncols) {
-        if constexpr (sizeof(C) == 16) cp_async16(d, op.at(slab, e, col)); else cp_async8(d, op.at(slab, e, col));
+        if constexpr (sizeof(C) == 16) cp_async16(d, g); else cp_async8(d, g);
       } else {
         *d = mkc<T>(T(0), T(0));
       }
@@ -412,33 +431,33 @@ k_colfft_trunc(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int ns
     cp_async_commit();
   };
   int tl = blockIdx.x;
-  if (tl < total) issue(tl, buf0); else cp_async_commit();
+  const TilePos step = TilePos::of(gridDim.x, ntc, nslab);
+  TilePos nx = TilePos::of(tl, ntc, nslab);
+  if (tl < total) issue(nx, buf0); else cp_async_commit();
   for (int it = 0; tl < total; tl += gridDim.x, ++it) {
     C* cur = (it & 1) ? buf1 : buf0;
     C* nxt = (it & 1) ? buf0 : buf1;
-    const int tn = tl + gridDim.x;
-    if (tn < total) issue(tn, nxt); else cp_async_commit();
+    const TilePos p = nx;
+    nx = p.next(step, ntc, nslab);
+    if (tl + (int)gridDim.x < total) issue(nx, nxt); else cp_async_commit();
     cp_async_wait<1>();
-    const int ct = tl % ntc, slab = tl / ntc;
-    const int col = ct * NCOL + c;
+    const int col = p.ct * NCOL + c;
     const bool valid = col < ncols;
     C v[FF::E];
 #pragma unroll
-    for (int s = 0; s < FF::E; ++s) v[s] = cur[pidx<LAY>(FF::in_index(t, s)) * NCOL + c];
+    for (int s = 0; s < FF::E; ++s) v[s] = cur[FF::in_slot(t, s) * NCOL + c];
     FF::run(v, t, cur + c, NCOL, tw, SyncBlock{});
     __syncthreads();  // the last exchange of the forward transform has been read
 #pragma unroll
-    for (int s = 0; s < FF::E; ++s) {
-      const int e = FF::out_index(t, s);
-      cur[pidx<LAY>(e) * NCOL + c] = op.mask(slab, e, col, v[s]);
-    }
+    for (int s = 0; s < FF::E; ++s)
+      cur[FF::out_slot(t, s) * NCOL + c] = op.mask(p.slab, I{t, FF::out_const(s)}, col, v[s]);
     __syncthreads();
 #pragma unroll
-    for (int s = 0; s < FI::E; ++s) v[s] = cur[pidx<LAY>(FI::in_index(t, s)) * NCOL + c];
+    for (int s = 0; s < FI::E; ++s) v[s] = cur[FI::in_slot(t, s) * NCOL + c];
     FI::run(v, t, cur + c, NCOL, tw, SyncBlock{});
     if (valid) {
 #pragma unroll
-      for (int s = 0; s < FI::E; ++s) *op.at(slab, FI::out_index(t, s), col) = v[s];
+      for (int s = 0; s < FI::E; ++s) *op.at(p.slab, I{t, FI::out_const(s)}, col) = v[s];
     }
     __syncthreads();  // cur is refilled by the next iteration's copies
   }

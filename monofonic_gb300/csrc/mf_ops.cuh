@@ -78,7 +78,24 @@ struct ConvGeom {
   }
   // padded row kept by unpad -> original row, -1 otherwise
   __device__ __forceinline__ int kept_row(int x) const { return src_row(x); }
+  __device__ __forceinline__ long long row_off(int x, long long stride) const { return (long long)src_row(x) * stride; }
 };
+
+// index of an element along a transform: t, from the thread, in [0, TPL), plus
+// c, a constant once the slot loop is unrolled.  Where the whole range
+// [c, c + TPL) falls on one side of a row map's branches, the branch is
+// decided at compile time.
+template <int TPL>
+struct LineIdx {
+  int t, c;
+  __device__ __forceinline__ operator int() const { return t + c; }
+};
+// element offset x * stride with the constant part apart
+__device__ __forceinline__ long long idx_off(int x, long long stride) { return (long long)x * stride; }
+template <int TPL>
+__device__ __forceinline__ long long idx_off(LineIdx<TPL> x, long long stride) {
+  return (long long)x.t * stride + (long long)x.c * stride;
+}
 
 // The same geometry as compile-time constants for a pass of length L over the
 // padded axis (M = L): Orszag 3/2 (N = 2L/3) or the aliased convolver
@@ -95,6 +112,23 @@ struct CGeom {
     return !ORSZAG ? x : (x <= (N >> 1) ? x : (x > N ? x - (N >> 1) : -1));
   }
   __device__ __forceinline__ static constexpr int kept_row(int x) { return src_row(x); }
+  template <int TPL>
+  __device__ __forceinline__ static int src_row(LineIdx<TPL> x) {
+    if (!ORSZAG || x.c + TPL - 1 <= (N >> 1)) return x.t + x.c;
+    if (x.c > N) return x.t + (x.c - (N >> 1));
+    if (x.c > (N >> 1) && x.c + TPL - 1 <= N) return -1;
+    return src_row(x.t + x.c);
+  }
+  template <int TPL>
+  __device__ __forceinline__ static int kept_row(LineIdx<TPL> x) { return src_row(x); }
+  // x * stride, and the kept row of x * stride, the constant part apart
+  template <int TPL>
+  __device__ __forceinline__ static long long row_off(LineIdx<TPL> x, long long stride) {
+    if (!ORSZAG || x.c + TPL - 1 <= (N >> 1)) return idx_off(x, stride);
+    if (x.c > N) return (long long)x.t * stride + (long long)(x.c - (N >> 1)) * stride;
+    return (long long)src_row(x.t + x.c) * stride;
+  }
+  __device__ __forceinline__ static long long row_off(int x, long long stride) { return (long long)src_row(x) * stride; }
 };
 // a run-time geometry matching CGeom<L, ORSZAG>
 template <class G>
@@ -145,13 +179,14 @@ struct ConvXInvOp {
   }
   // pipelined form (k_colfft_pipe): raw source element and on-read transform; z = operand
   static constexpr bool kPipe = true;
-  __device__ __forceinline__ const C* srcp(int z, int j, int x, int kz) const {
-    const int i = g.src_row(x);
-    if (i < 0) return nullptr;
+  template <class I>
+  __device__ __forceinline__ const C* srcp(int z, int j, I x, int kz) const {
+    if (g.src_row(x) < 0) return nullptr;
     const C* f = z == 0 ? opnd[0].f : (z == 1 ? opnd[1].f : opnd[2].f);
-    return f + ((long long)i * g.N + j) * g.Kz + kz;
+    return f + ((long long)j * g.Kz + kz) + g.row_off(x, (long long)g.N * g.Kz);
   }
-  __device__ __forceinline__ C xform(int z, int j, int x, int kz, C v0) const {
+  template <class I>
+  __device__ __forceinline__ C xform(int z, int j, I x, int kz, C v0) const {
     const int i = g.src_row(x);
     const int kind = z == 0 ? opnd[0].kind : (z == 1 ? opnd[1].kind : opnd[2].kind);
     const C v = operand_value<T>(kind, dsel<0>(z), dsel<1>(z), dsel<2>(z), dsel<3>(z), v0, i, j, kz, g.N, kfac);
@@ -193,7 +228,8 @@ struct ConvXInvOp {
     t.c2 *= scale;
     return t;
   }
-  __device__ __forceinline__ C xform_tile(const Tile& t, int x, C v0) const {
+  template <class I>
+  __device__ __forceinline__ C xform_tile(const Tile& t, I x, C v0) const {
     const T gi = gradk<T>(g.src_row(x), g.N, kfac);
     if (t.grad) {
       const T f = t.c1 * gi + t.c0;
@@ -202,9 +238,10 @@ struct ConvXInvOp {
     const T f = (t.c2 * gi + t.c1) * gi + t.c0;
     return mkc<T>(v0.x * f, v0.y * f);
   }
-  __device__ __forceinline__ void store_z(int z, int j, int x, int kz, C v) const {
+  template <class I>
+  __device__ __forceinline__ void store_z(int z, int j, I x, int kz, C v) const {
     C* d = z == 0 ? dst[0] : (z == 1 ? dst[1] : dst[2]);
-    d[((long long)x * g.M + j) * g.Kz + kz] = v;
+    d[((long long)j * g.Kz + kz) + idx_off(x, (long long)g.M * g.Kz)] = v;
   }
 };
 
@@ -239,16 +276,18 @@ struct ConvYInvOp {
     d[((long long)x * g.M + y) * g.Kz + kz] = v;
   }
   static constexpr bool kPipe = true;
-  __device__ __forceinline__ const C* srcp(int z, int x, int y, int kz) const {
-    const int j = g.src_row(y);
-    if (j < 0) return nullptr;
+  template <class I>
+  __device__ __forceinline__ const C* srcp(int z, int x, I y, int kz) const {
+    if (g.src_row(y) < 0) return nullptr;
     const C* s0 = z == 0 ? src[0] : (z == 1 ? src[1] : src[2]);
-    return s0 + ((long long)x * g.M + j) * g.Kz + kz;
+    return s0 + ((long long)x * g.M * g.Kz + kz) + g.row_off(y, g.Kz);
   }
-  __device__ __forceinline__ C xform(int, int, int, int, C v) const { return v; }
-  __device__ __forceinline__ void store_z(int z, int x, int y, int kz, C v) const {
+  template <class I>
+  __device__ __forceinline__ C xform(int, int, I, int, C v) const { return v; }
+  template <class I>
+  __device__ __forceinline__ void store_z(int z, int x, I y, int kz, C v) const {
     C* d = z == 0 ? dst[0] : (z == 1 ? dst[1] : dst[2]);
-    d[((long long)x * g.M + y) * g.Kz + kz] = v;
+    d[((long long)x * g.M * g.Kz + kz) + idx_off(y, g.Kz)] = v;
   }
 };
 
@@ -276,11 +315,16 @@ struct ConvYFwdOp {
     if (j >= 0) dst[((long long)x * g.M + j) * g.Kz + kz] = v;
   }
   static constexpr bool kPipe = true;
-  __device__ __forceinline__ const C* srcp(int, int x, int y, int kz) const {
-    return src + ((long long)x * g.M + y) * g.Kz + kz;
+  template <class I>
+  __device__ __forceinline__ const C* srcp(int, int x, I y, int kz) const {
+    return src + ((long long)x * g.M * g.Kz + kz) + idx_off(y, g.Kz);
   }
-  __device__ __forceinline__ C xform(int, int, int, int, C v) const { return v; }
-  __device__ __forceinline__ void store_z(int, int x, int y, int kz, C v) const { store(x, y, kz, v); }
+  template <class I>
+  __device__ __forceinline__ C xform(int, int, I, int, C v) const { return v; }
+  template <class I>
+  __device__ __forceinline__ void store_z(int, int x, I y, int kz, C v) const {
+    if (g.kept_row(y) >= 0) dst[((long long)x * g.M * g.Kz + kz) + g.row_off(y, g.Kz)] = v;
+  }
 };
 
 // x pass of the product's r2c + unpad + output operator (+ optional inverse
@@ -314,18 +358,19 @@ struct ConvXFwdOp {
   __device__ __forceinline__ C load(int j, int xx, int kz) const {
     return src[((long long)xx * g.M + j) * g.Kz + kz];
   }
-  __device__ __forceinline__ C prefetch(int j, int xx, int kz) const {
-    const int i = g.kept_row(xx);
-    if (i < 0 || out_op == OUT_ASSIGN) return mkc<T>(T(0), T(0));
-    return target[((long long)i * g.N + j) * g.Kz + kz];
+  template <class I>
+  __device__ __forceinline__ C prefetch(int j, I xx, int kz) const {
+    if (g.kept_row(xx) < 0 || out_op == OUT_ASSIGN) return mkc<T>(T(0), T(0));
+    return target[((long long)j * g.Kz + kz) + g.row_off(xx, (long long)g.N * g.Kz)];
   }
-  __device__ __forceinline__ void store_pre(int j, int xx, int kz, C v, C r) const {
+  template <class I>
+  __device__ __forceinline__ void store_pre(int j, I xx, int kz, C v, C r) const {
     const int i = g.kept_row(xx);
     if (i < 0) return;
     const int nh = g.N >> 1;
     v = mkc<T>(v.x * scale, v.y * scale);
     if (g.orszag && (i == nh || j == nh || kz == nh)) v = mkc<T>(T(0), T(0));
-    const long long idx = ((long long)i * g.N + j) * g.Kz + kz;
+    const long long idx = ((long long)j * g.Kz + kz) + g.row_off(xx, (long long)g.N * g.Kz);
     if (out_op == OUT_ASSIGN) r = v;
     else if (out_op == OUT_ADD) r = cadd(r, v);
     else if (out_op == OUT_SUB) r = csub(r, v);
@@ -340,11 +385,16 @@ struct ConvXFwdOp {
   }
   __device__ __forceinline__ void store(int j, int xx, int kz, C v) const { store_pre(j, xx, kz, v, prefetch(j, xx, kz)); }
   static constexpr bool kPipe = true;
-  __device__ __forceinline__ const C* srcp(int, int j, int xx, int kz) const {
-    return src + ((long long)xx * g.M + j) * g.Kz + kz;
+  template <class I>
+  __device__ __forceinline__ const C* srcp(int, int j, I xx, int kz) const {
+    return src + ((long long)j * g.Kz + kz) + idx_off(xx, (long long)g.M * g.Kz);
   }
-  __device__ __forceinline__ C xform(int, int, int, int, C v) const { return v; }
-  __device__ __forceinline__ void store_z(int, int j, int xx, int kz, C v) const { store(j, xx, kz, v); }
+  template <class I>
+  __device__ __forceinline__ C xform(int, int, I, int, C v) const { return v; }
+  template <class I>
+  __device__ __forceinline__ void store_z(int, int j, I xx, int kz, C v) const {
+    store_pre(j, xx, kz, v, prefetch(j, xx, kz));
+  }
 };
 
 // Sub-lattice phase chain: the shift_field calls (grid_fft.hh:832-842) that
@@ -486,8 +536,12 @@ struct ConvXTruncOp {
     o.scale_in = scale_in;
     return o;
   }
-  __device__ __forceinline__ C* at(int j, int x, int kz) const { return buf + ((long long)x * g.M + j) * g.Kz + kz; }
-  __device__ __forceinline__ C mask(int j, int x, int kz, C v) const {
+  template <class I>
+  __device__ __forceinline__ C* at(int j, I x, int kz) const {
+    return buf + ((long long)j * g.Kz + kz) + idx_off(x, (long long)g.M * g.Kz);
+  }
+  template <class I>
+  __device__ __forceinline__ C mask(int j, I x, int kz, C v) const {
     const int i = g.kept_row(x);
     const int nh = g.N >> 1;
     if (i < 0 || (g.orszag && (i == nh || j == nh || kz == nh))) return mkc<T>(T(0), T(0));
@@ -532,11 +586,16 @@ struct PlainStridedOp {
     p[(long long)slab * ss() + (long long)e * es() + col] = mkc<T>(v.x * scale, v.y * scale);
   }
   static constexpr bool kPipe = true;
-  __device__ __forceinline__ const C* srcp(int, int slab, int e, int col) const {
-    return p + (long long)slab * ss() + (long long)e * es() + col;
+  template <class I>
+  __device__ __forceinline__ const C* srcp(int, int slab, I e, int col) const {
+    return p + ((long long)slab * ss() + col) + idx_off(e, es());
   }
-  __device__ __forceinline__ C xform(int, int, int, int, C v) const { return v; }
-  __device__ __forceinline__ void store_z(int, int slab, int e, int col, C v) const { store(slab, e, col, v); }
+  template <class I>
+  __device__ __forceinline__ C xform(int, int, I, int, C v) const { return v; }
+  template <class I>
+  __device__ __forceinline__ void store_z(int, int slab, I e, int col, C v) const {
+    p[((long long)slab * ss() + col) + idx_off(e, es())] = mkc<T>(v.x * scale, v.y * scale);
+  }
 };
 
 // plain z pass on the in-place padded layout: line = i*n + j, row of n+2 reals
