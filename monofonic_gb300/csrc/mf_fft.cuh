@@ -311,26 +311,61 @@ __host__ __device__ constexpr bool is_pow2(int x) { return x > 0 && (x & (x - 1)
 __host__ __device__ constexpr int padded_len(int L, int layout) { return layout == 1 ? L + (L >> 4) + 1 : L; }
 // exchange layout of a contiguous line of length L
 __host__ __device__ constexpr int zlayout(int L) {
-  return (L == 16 || L == 32 || L == 48 || L == 96 || L == 128 || L == 256 || L == 288 || L == 384 || L == 768)
+  return (L == 16 || L == 32 || L == 48 || L == 96 || L == 128 || L == 192 || L == 256 || L == 288 || L == 384 || L == 768)
              ? 13
-             : ((L == 64 || L == 192) ? 12 : 1);
+             : (L == 64 ? 12 : ((L == 24 || L == 72) ? 0 : 1));
 }
 // distance between consecutive lines' exchange buffers (elements): the
 // layout's length, widened where it moves the lines of one half-warp onto
-// different banks
+// different banks.  Counted over a whole transform in FP32 (wavefronts per
+// warp, minimum / this stride): 48: 96/96, 72: 192/240, 96: 96/96,
+// 144: 192/288, 192: 192/192, 288: 192/326, 384: 192/192
 __host__ __device__ constexpr int zline_stride(int L) {
   switch (L) {
     case 16: return 18;
-    case 24: return 27;
+    case 24: return 25;
     case 32: return 36;
     case 48: return 50;
     case 64: return 65;
+    case 72: return 83;
     case 96: return 100;
-    case 144: return 155;
-    case 192: return 193;
-    case 288: return 292;
+    case 144: return 166;
+    case 192: return 200;
+    case 288: return 300;
     default: return padded_len(L, zlayout(L)) | ((zlayout(L) == 1) ? 1 : 0);
   }
+}
+// distance between the staged real lines (L pairs) of the r2c z pass: equal to
+// the threads of a line modulo 16 where that is even, so that a half-warp's
+// reads, 16 / TPL lines of TPL pairs, fall on different banks (lines packed at
+// L pairs, a multiple of 16, all start on the same bank).  Each line is copied
+// on its own then; the stride is even, for 16-byte aligned copies
+__host__ __device__ constexpr int zstage_stride(int L) {
+  switch (L) {
+    case 12: return 14;
+    case 24: return 26;
+    case 48: return 50;
+    case 72: return 78;
+    case 96: return 100;
+    case 144: return 166;
+    case 192: return 200;
+    case 288: return 300;
+    default: return L;
+  }
+}
+// Which line of a batch the g-th line group takes in the z passes that stage
+// lines of N/2+1 elements (1 modulo 16) back to back: a wavefront covers W
+// elements (16 FP32, 8 FP64), i.e. W / TPL groups, and consecutive lines would
+// start one bank apart and overlap; lines TPL apart do not (N=256, TPL = 8: 66
+// instead of 130 wavefronts per warp for the two reads of the c2r)
+template <int TPL, int W>
+__device__ __forceinline__ constexpr int zline_of_group(int g) {
+  constexpr int N = W / TPL;
+  return (g & ~(W - 1)) + (g % W) / N + ((g % W) % N) * TPL;
+}
+template <int TPL, int W>
+__host__ __device__ constexpr bool zline_map_ok(int lpb) {
+  return TPL < W && W % TPL == 0 && lpb % W == 0;
 }
 
 // Line FFT of length L in precision T, direction INV, radices up to MAXR;

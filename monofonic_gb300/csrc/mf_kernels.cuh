@@ -835,11 +835,11 @@ template <typename T, int MODE>
 __host__ __device__ constexpr int zconv_tma_minb() {
   return sizeof(T) != 4 ? 0 : (MODE == 2 ? 4 : 0);
 }
-// the r2c mode exchanges in its staged input lines (kin = H) when the
-// exchange stride of a line fits in one
+// the r2c mode exchanges in its staged input lines (kin = H, zstage_stride
+// apart) when the exchange stride of a line fits in one
 template <int H, int MODE>
 __host__ __device__ constexpr bool zconv_xchg_in_stage() {
-  return MODE == 2 && zline_stride(H) <= H;
+  return MODE == 2 && zline_stride(H) <= zstage_stride(H);
 }
 template <typename T, int H, int MAXR, int LPB, class SYNC, int MODE = 0, int KIN = 0>
 __global__ void __launch_bounds__(LPB * LineFFT<T, H, true, MAXR>::TPL, zconv_tma_minb<T, MODE>())
@@ -855,12 +855,18 @@ k_zconv_tma(ZConvArgs<T> a, const cplx<T>* __restrict__ twH, const cplx<T>* __re
   const int nop = (MODE == 0) ? a.nop : 1;
   const int kin = KIN ? KIN : a.kin;  // line length (compiled in when KIN > 0)
   C* stage = reinterpret_cast<C*>(smem_raw + 128);
-  const int per_op = LPB * kin;
+  constexpr int SP2 = zstage_stride(H);  // staged line stride of the r2c mode
+  constexpr bool PER_LINE = MODE == 2 && SP2 != H;  // its lines are copied one by one
+  const int sline = (MODE == 2) ? SP2 : kin;
+  const int per_op = LPB * sline;
   C* xchg = stage + 2 * nop * per_op;
-  const int t = threadIdx.x % TPL, ly = threadIdx.x / TPL;
-  C* const sm_x = xchg + ly * LS;
+  constexpr int WF = 128 / (int)sizeof(C);  // elements per shared-memory wavefront
+  const int t = threadIdx.x % TPL, lg = threadIdx.x / TPL;
+  int ly = lg;
+  if constexpr (MODE != 2 && zline_map_ok<TPL, WF>(LPB)) ly = zline_of_group<TPL, WF>(lg);
+  C* const sm_x = xchg + lg * LS;
   const int nbatch = a.nlines / LPB;
-  const unsigned bytes_op = (unsigned)(per_op * sizeof(C));
+  const unsigned bytes_op = (unsigned)(LPB * kin * sizeof(C));
   const C* in0 = a.in[0];
   const C* in1 = a.in[1];
   const C* in2 = a.in[2];
@@ -871,20 +877,29 @@ k_zconv_tma(ZConvArgs<T> a, const cplx<T>* __restrict__ twH, const cplx<T>* __re
     fence_mbar_init();
   }
   __syncthreads();
+  // run by the first warp
   auto issue = [&](int b, int st) {
+    const long long off = (long long)b * LPB * kin;
+    if constexpr (PER_LINE) {
+      if (threadIdx.x == 0) mbar_arrive_expect_tx(&bars[st], bytes_op);
+      __syncwarp();
+      for (int l = threadIdx.x; l < LPB; l += 32)
+        tma_load_1d(stage + st * per_op + l * SP2, in0 + off + (long long)l * H, (unsigned)(H * sizeof(C)), &bars[st]);
+      return;
+    }
+    if (threadIdx.x != 0) return;
     mbar_arrive_expect_tx(&bars[st], (unsigned)nop * bytes_op);
-    const long long off = (long long)b * per_op;
     tma_load_1d(stage + (st * nop + 0) * per_op, in0 + off, bytes_op, &bars[st]);
     if (nop > 1) tma_load_1d(stage + (st * nop + 1) * per_op, in1 + off, bytes_op, &bars[st]);
     if (nop > 2) tma_load_1d(stage + (st * nop + 2) * per_op, in2 + off, bytes_op, &bars[st]);
   };
-  if (threadIdx.x == 0 && (int)blockIdx.x < nbatch) issue(blockIdx.x, 0);
+  if (threadIdx.x < 32 && (int)blockIdx.x < nbatch) issue(blockIdx.x, 0);
   int iter = 0;
   bool pending_other = false;
   for (int b = blockIdx.x; b < nbatch; b += gridDim.x, ++iter) {
     const int st = iter & 1;
     const int bn = b + gridDim.x;
-    if (threadIdx.x == 0 && bn < nbatch) {
+    if (threadIdx.x < 32 && bn < nbatch) {
       fence_proxy_async_smem();
       issue(bn, st ^ 1);
     }
@@ -898,9 +913,9 @@ k_zconv_tma(ZConvArgs<T> a, const cplx<T>* __restrict__ twH, const cplx<T>* __re
     C v[E], prod[E];
     // this line's exchange area: its staged input line in the r2c mode (read
     // into registers before the transform's first exchange), else its own
-    C* const sm = zconv_xchg_in_stage<H, MODE>() ? stage + (st * nop) * per_op + ly * kin : sm_x;
+    C* const sm = zconv_xchg_in_stage<H, MODE>() ? stage + (st * nop) * per_op + ly * sline : sm_x;
     if constexpr (MODE == 2) {
-      const C* src = stage + (st * nop) * per_op + ly * kin;
+      const C* src = stage + (st * nop) * per_op + ly * sline;
 #pragma unroll
       for (int s = 0; s < E; ++s) v[s] = src[FF::in_index(t, s)];
     }
@@ -926,10 +941,10 @@ k_zconv_tma(ZConvArgs<T> a, const cplx<T>* __restrict__ twH, const cplx<T>* __re
       if constexpr (MODE == 0) {
         sync();
 #pragma unroll
-        for (int s = 0; s < E; ++s) sm[pidx<LAY>(FI::out_index(t, s))] = prod[s];
+        for (int s = 0; s < E; ++s) sm[FI::out_slot(t, s)] = prod[s];
         sync();
 #pragma unroll
-        for (int s = 0; s < E; ++s) v[s] = sm[pidx<LAY>(FF::in_index(t, s))];
+        for (int s = 0; s < E; ++s) v[s] = sm[FF::in_slot(t, s)];
       }
       FF::run(v, t, sm, 1, twH, sync);
       C* dst = a.out + (long long)(b * LPB + ly) * a.out_stride;

@@ -237,7 +237,11 @@ cudaError_t launch_zconv(const ZConvArgs<T>& a, const cplx<T>* twH, const cplx<T
     // build-time knob: more, smaller CTAs per SM)
     constexpr int LPB0 = tma_lines_per_batch<T, TPL>();
     constexpr int DIV = (MODE == 1) ? MF_ZC2R_LPB_DIV : MF_ZONE_LPB_DIV;
-    constexpr int LPBT = (MODE != 0 && LPB0 >= 2 * DIV) ? LPB0 / DIV : LPB0;
+    constexpr int LPBD = (LPB0 >= 2 * DIV) ? LPB0 / DIV : LPB0;
+    // at least one wavefront's lines where that lets the line groups read
+    // without bank conflicts (zline_of_group)
+    constexpr int WF = 128 / (int)sizeof(cplx<T>);
+    constexpr int LPBT = (MODE != 2 && LPBD < WF && zline_map_ok<TPL, WF>(WF) && WF <= LPB0) ? WF : LPBD;
     // (the r2c mode's lines hold H pairs; its exchanges run in them when they fit)
     const bool tma_ok = MF_ZCONV_TMA && (MODE != 2 || (a.kin == H && a.kout <= 2 * H / 3 + 1)) &&
                         (a.nlines % LPBT == 0) && (a.in_stride == a.kin) &&
@@ -252,7 +256,7 @@ cudaError_t launch_zconv(const ZConvArgs<T>& a, const cplx<T>* twH, const cplx<T
       auto kern = (KIN_CT != 0 && a.kin == KIN_CT) ? k_zconv_tma<T, H, MAXR, LPBT, SYNC, MODE, KIN_CT>
                                                    : k_zconv_tma<T, H, MAXR, LPBT, SYNC, MODE, 0>;
       const size_t smem =
-          128 + ((size_t)2 * a.nop * LPBT * a.kin + (zconv_xchg_in_stage<H, MODE>() ? 0 : (size_t)LPBT * zline_stride(H))) *
+          128 + ((size_t)2 * a.nop * LPBT * (MODE == 2 ? zstage_stride(H) : a.kin) + (zconv_xchg_in_stage<H, MODE>() ? 0 : (size_t)LPBT * zline_stride(H))) *
                     sizeof(cplx<T>);
       cudaError_t e = set_smem(kern, smem);
       if (e != cudaSuccess) return e;
