@@ -3,6 +3,7 @@
 #include <type_traits>
 
 #include "mf_noise.h"
+#include "mf_noise_f32.cuh"
 #include "mf_tma.cuh"
 #include "mf_runtime.h"
 
@@ -49,21 +50,27 @@ __global__ void k_invlap(cplx<T>* d, int n, T kfac) {
 // mf_noise.h, the same bits as the host plugin), written into the padded
 // real layout; pair p = cells 2p, 2p+1 of one z row (n even).  The seed is
 // read from device memory when seed_dev is given (replayable graphs).
+// FP32 grids take the float-pair evaluation (mf_noise_f32.cuh) and, for the
+// draws that it leaves open, the FP64 sequence.
 template <typename T>
-__global__ void k_white_noise(T* d, int n, unsigned long long seed, const unsigned long long* seed_dev) {
+__global__ void __launch_bounds__(kThreads) k_white_noise(T* d, int n, unsigned long long seed,
+                                                          const unsigned long long* seed_dev) {
   using T2 = typename cplx_of<T>::type;
   const unsigned long long sd = seed_dev ? *seed_dev : seed;
   const unsigned hn = (unsigned)n >> 1;
-  const unsigned long long npair = (unsigned long long)n * n * hn;
-  for (unsigned long long p = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; p < npair;
-       p += (unsigned long long)gridDim.x * blockDim.x) {
-    double z0, z1;
-    noise::normal_pair(p, sd, &z0, &z1);
-    const unsigned long long line = p / hn;
-    const unsigned k = 2u * (unsigned)(p - line * hn);
+  const unsigned npair = (unsigned)n * n * hn;  // n <= 1024
+  for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < npair; p += gridDim.x * blockDim.x) {
     T2 v;
-    v.x = (T)z0;
-    v.y = (T)z1;
+    bool done = false;
+    if constexpr (std::is_same<T, float>::value) done = noise::normal_pair_f32(p, sd, &v.x, &v.y);
+    if (!done) {
+      double z0, z1;
+      noise::normal_pair(p, sd, &z0, &z1);
+      v.x = (T)z0;
+      v.y = (T)z1;
+    }
+    const unsigned line = p / hn;
+    const unsigned k = 2u * (p - line * hn);
     *reinterpret_cast<T2*>(d + line * (unsigned long long)(n + 2) + k) = v;
   }
 }
