@@ -11,6 +11,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "mf_fx.cuh"
 #include "mf_runtime.h"
 
 #define MF_VERSION_STR "monofonic_gb300 0.1 (sm_103a)"
@@ -104,6 +105,23 @@ static void twiddle_host(int L, std::vector<double>& re, std::vector<double>& im
   }
 }
 
+// the same as split Q62 values
+void fx_twiddles(int L, longlong2* out) {
+  const long double pi = 3.141592653589793238462643383279502884L;
+  for (int j = 0; j < L; ++j) {
+    // reduced to the first octant, so that the axes are exact and mirrored values match
+    const int q = (int)((8LL * j) / L);           // octant 0..7
+    const long long r = 8LL * j - (long long)q * L;  // position inside it, in L-ths of an octant
+    const long double a = pi / 4.0L * (long double)((q & 1) ? L - r : r) / (long double)L;
+    const long double c = cosl(a), s = sinl(a);
+    // cos and sin of the whole angle from the octant's
+    static const int swap[8] = {0, 1, 1, 0, 0, 1, 1, 0};
+    static const int sc[8] = {1, 1, -1, -1, -1, -1, 1, 1}, ss[8] = {1, 1, 1, 1, -1, -1, -1, -1};
+    const long double re = sc[q] * (swap[q] ? s : c), im = -(ss[q] * (swap[q] ? c : s));
+    out[j] = make_longlong2(fx::split_q62(re), fx::split_q62(im));
+  }
+}
+
 TwiddleCache::~TwiddleCache() { release(); }
 
 void TwiddleCache::release() {
@@ -120,11 +138,13 @@ const double2* TwiddleCache::get64(int L, cudaStream_t s) {
   if (it != t64_.end()) return it->second;
   std::vector<double> re, im;
   twiddle_host(L, re, im);
-  std::vector<double2> h(L);
+  std::vector<double2> h(2 * (size_t)L);  // the table, then the same in fixed point (mf_fx.cuh)
   for (int j = 0; j < L; ++j) h[j] = make_double2(re[j], im[j]);
+  fx_twiddles(L, reinterpret_cast<longlong2*>(h.data() + L));
   double2* d = nullptr;
-  if (cudaMalloc(&d, sizeof(double2) * L) != cudaSuccess) return nullptr;
-  if (cudaMemcpy(d, h.data(), sizeof(double2) * L, cudaMemcpyHostToDevice) != cudaSuccess) { cudaFree(d); return nullptr; }
+  const size_t bytes = sizeof(double2) * h.size();
+  if (cudaMalloc(&d, bytes) != cudaSuccess) return nullptr;
+  if (cudaMemcpy(d, h.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess) { cudaFree(d); return nullptr; }
   t64_[L] = d;
   return d;
 }

@@ -1,0 +1,439 @@
+// FP64 line transforms in 64-bit fixed point.
+//
+// The device issues 1.68 FP64 operations per clock and SM but ~42 64-bit
+// integer additions and ~53 32x32+64 multiply-adds (measured), so a line FFT
+// of FP64 values runs on the integer pipes: the line is converted to
+// q = round(x 2^xs), transformed with exact additions and twiddle products of
+// 62-bit twiddles, and converted back.
+//
+// Scale.  Every value inside an unnormalised DFT is a sum of inputs times
+// phases, so its modulus is at most the line's L1 norm.  xs places an upper
+// bound of that norm at 2^62 (less the growth of a pre- or post-processing
+// step), so nothing overflows and no stage needs a shift.  The error: each
+// conversion and each product is rounded to half a unit of 2^-xs, which over
+// a transform of length L leaves ~0.4 L^(1/2) units; with |x|_1 <= L^(1/2)
+// |x|_2 that is at most ~0.4 L 2^-62 of the output's r.m.s. (0.6 2^-53 at
+// L = 768, less for lines dominated by few values), where FP64 rounding leaves
+// ~1.4 2^-53.
+//
+// Measured (N=256, FP64): z c2r of a padded operand 1734 -> 386 us, y c2r 1000
+// -> 262 us per operand, a 3LPT run 114.0 -> 35.0 ms; a forward transform of
+// white noise is 1.1e-16 (N=256) and 1.7e-16 (N=384) off in relative L2, FP64
+// butterflies were 3.2e-16 and 3.3e-16 off.  What bounds it now is instruction
+// issue: ~100 instructions per element in the butterflies, ~100 in conversions.
+//
+// Lines holding an infinity or a NaN come out NaN.  A line whose norm is
+// outside the float range that the bound is summed in takes its scale from
+// its largest exponent (the bound is then L times that value), and extreme
+// results are scaled by FP64 products.  Subnormal inputs count as zeros.
+#pragma once
+
+#include <cmath>
+#include <type_traits>
+
+#include "mf_fft.cuh"
+
+namespace mf {
+
+template <> struct cplx_of<long long> { using type = longlong2; };
+
+namespace fx {
+
+constexpr int kNan = 1 << 20;  // scale of a line that holds no finite result
+
+// twiddle component w, |w| <= 1, as q = round(w 2^62) split into a signed low
+// word and the matching high word (the form cmul reads)
+__host__ inline long long split_q62(long double w) {
+  long long q = llroundl(w * 4611686018427387904.0L);
+  int lo = (int)(unsigned)(q & 0xffffffffll);
+  if (lo == (int)0x80000000) { ++q; ++lo; }  // so that -lo exists
+  const long long hi = (q - (long long)lo) >> 32;
+  return (long long)(((unsigned long long)hi << 32) | (unsigned)lo);
+}
+
+__device__ __forceinline__ int lo32(long long a) { return (int)(unsigned)(unsigned long long)a; }
+__device__ __forceinline__ int hi32(long long a) { return (int)(a >> 32); }
+__device__ __forceinline__ long long wide(int a, int b) {
+  long long r;
+  asm("mul.wide.s32 %0, %1, %2;" : "=l"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ long long mad(int a, int b, long long c) {  // a b + c
+  long long r;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+  return r;
+}
+// a split into a signed low word and the matching high word
+__device__ __forceinline__ void split(long long a, int& h, int& l) {
+  l = lo32(a);
+  h = hi32(a) + (int)((unsigned)l >> 31);
+}
+// (h 2^64 + m 2^32) / 2^62 for |h 2^2| < 2^63
+__device__ __forceinline__ long long join(long long h, long long m) {
+  const long long u = mad(hi32(m), 1, h);  // h 2^32 + m, its upper 64 bits
+  const unsigned lo = __funnelshift_l((unsigned)lo32(m), (unsigned)lo32(u), 2);
+  const unsigned hi = __funnelshift_l((unsigned)lo32(u), (unsigned)hi32(u), 2);
+  return (long long)(((unsigned long long)hi << 32) | lo);
+}
+// round(a c / 2^62) for a constant c in Q62, |a| < 2^62.5 (the product of the
+// low words, below half a unit, is left out: both are signed)
+__device__ __forceinline__ long long mulc(long long a, int ch, int cl) {
+  int ah, al;
+  split(a, ah, al);
+  return join(wide(ah, ch), mad(ah, cl, mad(al, ch, 1ll << 29)));
+}
+
+// upper bound of |x| as a float: the exponent rebased and the mantissa
+// rounded up; 0 below the float range, infinity or NaN above it
+__device__ __forceinline__ float mag(int hi_abs) {
+  int h = hi_abs - (896 << 20);
+  h = max(h, 0);
+  h = min(h, 0x0ff00000);
+  return __int_as_float((h << 3) + 8);
+}
+__device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
+
+// scale of a line from the bound of its L1 norm and its largest high word;
+// grow: bits of growth of the processing around the transform
+__device__ __forceinline__ int scale(float l1, int maxhi, int len_bits, int grow) {
+  if (l1 > 0x1p-100f && l1 < 0x1p120f) {
+    // l1 (1 + 2^-6) < 2^X covers the rounding of the float sum
+    const int X = (__float_as_int(l1 * 1.015625f) >> 23) - 126;
+    return 62 - grow - X;
+  }
+  const int e = max(maxhi >> 20, 1);
+  if (e == 0x7ff) return kNan;
+  return 62 - grow - (e - 1022 + 1 + len_bits);
+}
+
+// round(x 2^xs) for |x| 2^xs < 2^62, subnormal x as zero
+__device__ __forceinline__ long long from_double(double x, int xs) {
+  const int hi = __double2hiint(x);
+  const unsigned lo = (unsigned)__double2loint(x);
+  // the 53-bit mantissa at bits 10..62, shifted right to twice the value (a
+  // count of 64 or more leaves 0)
+  const unsigned mh = (((unsigned)hi & 0xfffffu) | 0x100000u) << 10 | (lo >> 22);
+  const unsigned long long m = ((unsigned long long)mh << 32) | (lo << 10);
+  const int e = (hi >> 20) & 0x7ff;
+  const unsigned r = e ? (unsigned)(1084 - xs - e) : 64u;
+  unsigned long long q;
+  asm("shr.u64 %0, %1, %2;" : "=l"(q) : "l"(m), "r"(r));
+  const long long s = (long long)(hi >> 31);
+  // (q + 1) / 2 for a positive value, floor(-q / 2) for a negative one: halves away from zero
+  return (((long long)q ^ s) + 1) >> 1;
+}
+
+// q 2^-xs, rounded to the nearest double, for any scale and |q| < 2^63
+static __device__ __noinline__ double to_double_any(long long q, int xs) {
+  if (xs >= kNan) return __longlong_as_double(0x7ff8000000000000ll);
+  double d = (double)q;
+  int k = -xs;
+  while (k > 1000) { d *= 0x1p1000; k -= 1000; }
+  while (k < -1000) { d *= 0x1p-1000; k += 1000; }
+  return d * __hiloint2double((1023 + k) << 20, 0);
+}
+__device__ __forceinline__ double to_double(long long q, int xs) {
+  const int s = hi32(q) >> 31;
+  const unsigned long long a = (unsigned long long)((q ^ (long long)s) - (long long)s);
+  const unsigned ah = (unsigned)(a >> 32), al = (unsigned)a;
+  // |q| < 2^32 (zeros among them) and unusual scales
+  if (ah == 0u || (unsigned)(xs + 900) > 1800u) return q == 0 && xs < kNan ? 0.0 : to_double_any(q, xs);
+  const int lz = __clz((int)ah);  // 1..31
+  // bit 62 set, rounded to 53 bits (or 2^53)
+  const unsigned nh = __funnelshift_l(al, ah, lz - 1), nl = al << (lz - 1);
+  const unsigned long long m = ((((unsigned long long)nh << 32) | nl) + 0x200) >> 10;
+  const unsigned hi = (unsigned)(m >> 32) + ((unsigned)(1085 - xs) << 20) - ((unsigned)lz << 20);
+  return __hiloint2double((int)(hi | ((unsigned)s & 0x80000000u)), (int)(unsigned)m);
+}
+
+__device__ __forceinline__ longlong2 from_c(double2 v, int xs) {
+  return make_longlong2(from_double(v.x, xs), from_double(v.y, xs));
+}
+__device__ __forceinline__ double2 to_c(longlong2 v, int xs) {
+  return make_double2(to_double(v.x, xs), to_double(v.y, xs));
+}
+
+// running bound of a line: sum of the components' magnitudes, largest high word
+struct Norm {
+  float l1 = 0.f;
+  int mx = 0;
+  __device__ __forceinline__ void add(double2 v) {
+    const int a = hi_abs(v.x), b = hi_abs(v.y);
+    l1 += mag(a) + mag(b);
+    mx = max(mx, max(a, b));
+  }
+  __device__ __forceinline__ void add(const Norm& o) {
+    l1 += o.l1;
+    mx = max(mx, o.mx);
+  }
+  __device__ __forceinline__ Norm shfl_xor(int o) const {
+    Norm r;
+    r.l1 = __shfl_xor_sync(0xffffffffu, l1, o);
+    r.mx = __shfl_xor_sync(0xffffffffu, mx, o);
+    return r;
+  }
+};
+
+__host__ __device__ constexpr int ceil_log2(int n) {
+  int b = 0;
+  while ((1 << b) < n) ++b;
+  return b;
+}
+
+}  // namespace fx
+
+// complex products of a fixed-point value with a split Q62 twiddle: four
+// 32x32 products per component are summed in 64 bits before one rounding
+// shift, two more carry the high words
+__device__ __forceinline__ longlong2 fx_cmul(longlong2 a, int wxh, int wxl, int wyh, int wyl) {
+  int axh, axl, ayh, ayl;
+  fx::split(a.x, axh, axl);
+  fx::split(a.y, ayh, ayl);
+  const int nyh = -wyh, nyl = -wyl;
+  const long long half = 1ll << 29;
+  const long long mr = fx::mad(axh, wxl, fx::mad(axl, wxh, fx::mad(ayh, nyl, fx::mad(ayl, nyh, half))));
+  const long long hr = fx::mad(axh, wxh, fx::wide(ayh, nyh));
+  const long long mi = fx::mad(axh, wyl, fx::mad(axl, wyh, fx::mad(ayh, wxl, fx::mad(ayl, wxh, half))));
+  const long long hi = fx::mad(axh, wyh, fx::wide(ayh, wxh));
+  return make_longlong2(fx::join(hr, mr), fx::join(hi, mi));
+}
+template <>
+__device__ __forceinline__ longlong2 cmul<longlong2>(longlong2 a, longlong2 w) {
+  return fx_cmul(a, fx::hi32(w.x), fx::lo32(w.x), fx::hi32(w.y), fx::lo32(w.y));
+}
+// a * conj(w)
+template <>
+__device__ __forceinline__ longlong2 cmulc<longlong2>(longlong2 a, longlong2 w) {
+  return fx_cmul(a, fx::hi32(w.x), fx::lo32(w.x), -fx::hi32(w.y), -fx::lo32(w.y));
+}
+
+// radix-3 and radix-8 butterflies: constants in Q62, halving by a shift that
+// rounds ties to even (a plain shift would leave the same quarter unit in
+// every output)
+namespace fx {
+constexpr int kS32h = 0x376cf5d1, kS32l = -1332128537;  // sqrt(3)/2
+constexpr int kS12h = 0x2d413ccd, kS12l = -25716447;    // 1/sqrt(2)
+__device__ __forceinline__ long long half_even(long long s) { return (s + ((lo32(s) >> 1) & 1)) >> 1; }
+template <bool INV>
+__device__ __forceinline__ void dft3(longlong2* a) {
+  const longlong2 s = cadd(a[1], a[2]), d = csub(a[1], a[2]);
+  const longlong2 m = make_longlong2(a[0].x - half_even(s.x), a[0].y - half_even(s.y));
+  a[0] = cadd(a[0], s);
+  longlong2 r = cmul_mi<INV>(d);
+  r.x = mulc(r.x, kS32h, kS32l);
+  r.y = mulc(r.y, kS32h, kS32l);
+  a[1] = cadd(m, r);
+  a[2] = csub(m, r);
+}
+template <bool INV>
+__device__ __forceinline__ void dft8(longlong2* a) {
+  longlong2 e0 = a[0], e1 = a[2], e2 = a[4], e3 = a[6];
+  longlong2 o0 = a[1], o1 = a[3], o2 = a[5], o3 = a[7];
+  dft4v<long long, INV>(e0, e1, e2, e3);
+  dft4v<long long, INV>(o0, o1, o2, o3);
+  longlong2 w1, w2, w3;
+  if (!INV) {
+    w1 = make_longlong2(mulc(o1.x + o1.y, kS12h, kS12l), mulc(o1.y - o1.x, kS12h, kS12l));
+    w2 = make_longlong2(o2.y, -o2.x);
+    w3 = make_longlong2(mulc(o3.y - o3.x, kS12h, kS12l), mulc(-(o3.x + o3.y), kS12h, kS12l));
+  } else {
+    w1 = make_longlong2(mulc(o1.x - o1.y, kS12h, kS12l), mulc(o1.x + o1.y, kS12h, kS12l));
+    w2 = make_longlong2(-o2.y, o2.x);
+    w3 = make_longlong2(mulc(-(o3.x + o3.y), kS12h, kS12l), mulc(o3.x - o3.y, kS12h, kS12l));
+  }
+  a[0] = cadd(e0, o0); a[4] = csub(e0, o0);
+  a[1] = cadd(e1, w1); a[5] = csub(e1, w1);
+  a[2] = cadd(e2, w2); a[6] = csub(e2, w2);
+  a[3] = cadd(e3, w3); a[7] = csub(e3, w3);
+}
+}  // namespace fx
+template <> __device__ __forceinline__ void dft3<long long, false>(longlong2* a) { fx::dft3<false>(a); }
+template <> __device__ __forceinline__ void dft3<long long, true>(longlong2* a) { fx::dft3<true>(a); }
+template <> __device__ __forceinline__ void dft8<long long, false>(longlong2* a) { fx::dft8<false>(a); }
+template <> __device__ __forceinline__ void dft8<long long, true>(longlong2* a) { fx::dft8<true>(a); }
+
+// ---------------------------------------------------------------------------
+// the transforms of the kernels: FP32 lines as they are, FP64 lines in fixed
+// point.  `tw` of an FP64 transform of length L is followed by its L
+// fixed-point twiddles (TwiddleCache).
+// ---------------------------------------------------------------------------
+template <int L>
+__device__ __forceinline__ const longlong2* fx_table(const double2* tw) {
+  return reinterpret_cast<const longlong2*>(tw + L);
+}
+
+// norm of each column of a strided tile, block (NCOL, TPL), to all its threads
+template <int NCOL, int TPL>
+__device__ __forceinline__ fx::Norm col_norm(fx::Norm n, int t, int c) {
+  constexpr bool WARP = NCOL < 32;  // a warp holds 32 / NCOL elements of a column
+  constexpr int ROWS = WARP ? (NCOL * TPL + 31) / 32 : TPL;
+  __shared__ float l1[ROWS * NCOL];
+  __shared__ int mx[ROWS * NCOL];
+  if constexpr (WARP) {
+#pragma unroll
+    for (int o = NCOL; o < 32; o <<= 1) n.add(n.shfl_xor(o));
+  }
+  const int row = WARP ? (t * NCOL + c) >> 5 : t;
+  l1[row * NCOL + c] = n.l1;  // (a warp's lanes of one column write the same values)
+  mx[row * NCOL + c] = n.mx;
+  __syncthreads();
+  fx::Norm r;
+#pragma unroll 8
+  for (int i = 0; i < ROWS; ++i) {
+    r.l1 += l1[i * NCOL + c];
+    r.mx = max(r.mx, mx[i * NCOL + c]);
+  }
+  return r;
+}
+
+// Transform of the columns of a tile of double2 in fixed point, exchanged in
+// the tile, F the FP64 plan: on entry every thread's own elements (t + i TPL,
+// i < E) hold the inputs, on exit its own elements hold the outputs q, value
+// q 2^-xs with the returned xs.  The conversions run as rolled loops over the
+// tile: unrolled over registers they are ~1000 instructions each, and the
+// kernels then waited on instruction fetch (3.7 of 8 stall cycles per issue).
+template <class F, int NCOL>
+__device__ __forceinline__ int tile_slot(int t, int i) {
+  return pidx<F::kLayout>(t + i * F::TPL) * NCOL;
+}
+template <class F, int NCOL>
+__device__ __forceinline__ void col_fx_run(longlong2* tile, int t, int c, const double2* tw) {
+  using FX = typename F::template with_type<long long>;
+  longlong2 q[F::E];
+#pragma unroll
+  for (int s = 0; s < F::E; ++s) q[s] = tile[F::in_slot(t, s) * NCOL + c];
+  FX::run(q, t, tile + c, NCOL, fx_table<F::LEN>(tw), SyncBlock{});
+  __syncthreads();  // the last exchange has been read
+#pragma unroll
+  for (int s = 0; s < F::E; ++s) tile[F::out_slot(t, s) * NCOL + c] = q[s];
+}
+template <class F, int NCOL>
+__device__ __forceinline__ int col_fx(double2* tile, int t, int c, const double2* tw) {
+  longlong2* tx = reinterpret_cast<longlong2*>(tile);
+  fx::Norm n;
+#pragma unroll 2
+  for (int i = 0; i < F::E; ++i) n.add(tile[tile_slot<F, NCOL>(t, i) + c]);
+  n = col_norm<NCOL, F::TPL>(n, t, c);
+  const int xs = fx::scale(n.l1, n.mx, fx::ceil_log2(F::LEN), 0);
+#pragma unroll 2
+  for (int i = 0; i < F::E; ++i) {
+    const int o = tile_slot<F, NCOL>(t, i) + c;
+    tx[o] = fx::from_c(tile[o], xs);
+  }
+  col_fx_run<F, NCOL>(tx, t, c, tw);
+  return xs;
+}
+
+// norm of each line of a contiguous-line pass, TPL threads per line
+template <int TPL, class SYNC>
+__device__ __forceinline__ fx::Norm line_norm(fx::Norm n, int t, int lg, SYNC sync) {
+  if constexpr (std::is_same<SYNC, SyncWarp>::value) {
+#pragma unroll
+    for (int o = 1; o < TPL; o <<= 1) n.add(n.shfl_xor(o));
+    return n;
+  } else {
+    __shared__ float l1[256];
+    __shared__ int mx[256];
+    sync();
+    if (t == 0) { l1[lg] = 0.f; mx[lg] = 0; }
+    sync();
+    atomicAdd(&l1[lg], n.l1);
+    atomicMax(&mx[lg], n.mx);
+    sync();
+    fx::Norm r;
+    r.l1 = l1[lg];
+    r.mx = mx[lg];
+    return r;
+  }
+}
+
+// a staged half-complex line (kin values, kz >= kin zero) to fixed point in
+// place; returns its scale
+template <int H, int TPL, class SYNC>
+__device__ __forceinline__ int c2r_line_to_fx(double2* src, int kin, int t, int lg, SYNC sync) {
+  fx::Norm n;
+#pragma unroll 2
+  for (int k = t; k < kin; k += TPL) n.add(src[k]);
+  n = line_norm<TPL>(n, t, lg, sync);
+  // inputs of the transform are E + iO: at most twice the moduli of two terms each
+  const int xs = fx::scale(n.l1, n.mx, fx::ceil_log2(H), 2);
+  // the imaginary parts of kz = 0 and kz = H do not count
+#pragma unroll 2
+  for (int k = t; k < kin; k += TPL) {
+    longlong2 q = fx::from_c(src[k], xs);
+    if (k == 0 || k == H) q.y = 0;
+    reinterpret_cast<longlong2*>(src)[k] = q;
+  }
+  sync();
+  return xs;
+}
+
+// a staged line of H real pairs in layout LIN to fixed point in place;
+// returns its scale (the post-processing doubles the values)
+template <int H, int TPL, int LIN, class SYNC>
+__device__ __forceinline__ int r2c_line_to_fx(double2* src, int t, int lg, SYNC sync) {
+  fx::Norm n;
+#pragma unroll 2
+  for (int k = t; k < H; k += TPL) n.add(src[pidx<LIN>(k)]);
+  n = line_norm<TPL>(n, t, lg, sync);
+  const int xs = fx::scale(n.l1, n.mx, fx::ceil_log2(H), 1);
+#pragma unroll 2
+  for (int k = t; k < H; k += TPL)
+    reinterpret_cast<longlong2*>(src)[pidx<LIN>(k)] = fx::from_c(src[pidx<LIN>(k)], xs);
+  return xs;
+}
+
+// one c2r pre-processed input of the half-length transform
+template <int H>
+__device__ __forceinline__ longlong2 c2r_pre_fx(const longlong2* src, int k, int kin,
+                                                const longlong2* __restrict__ twM) {
+  const longlong2 A = (k < kin) ? src[k] : make_longlong2(0, 0);
+  const longlong2 B = (H - k < kin) ? cconj(src[H - k]) : make_longlong2(0, 0);
+  const longlong2 Ev = cadd(A, B);
+  const longlong2 Ov = cmulc(csub(A, B), twM[k]);
+  return make_longlong2(Ev.x - Ov.y, Ev.y + Ov.x);
+}
+// r2c post-processing: twice E + w O from Z[k] and Z[H-k]
+__device__ __forceinline__ longlong2 r2c_post_fx(longlong2 zk, longlong2 zh, longlong2 w) {
+  const longlong2 zc = cconj(zh);
+  const longlong2 d = csub(zk, zc);
+  return cadd(cadd(zk, zc), cmul(make_longlong2(d.y, -d.x), w));
+}
+
+// c2r of a staged line in fixed point (c2r_line_to_fx) into the line area xl:
+// on exit every thread's own elements (t + i TPL) hold the outputs.  xl may be
+// src itself (it is read before the first exchange).
+template <class F, int H, class SYNC>
+__device__ __forceinline__ void c2r_line_fx(const longlong2* src, int kin, longlong2* xl, int t, const double2* twH,
+                                            const double2* twM, SYNC sync) {
+  using FX = typename F::template with_type<long long>;
+  longlong2 q[F::E];
+#pragma unroll
+  for (int s = 0; s < F::E; ++s) q[s] = c2r_pre_fx<H>(src, F::in_index(t, s), kin, fx_table<2 * H>(twM));
+  FX::run(q, t, xl, 1, fx_table<H>(twH), sync);
+  sync();
+#pragma unroll
+  for (int s = 0; s < F::E; ++s) xl[F::out_slot(t, s)] = q[s];
+}
+// forward transform of a staged line of H pairs in fixed point, src (layout
+// LIN) into xl, which may be src; the outputs are visible to the line on exit
+template <class F, int H, int LIN, class SYNC>
+__device__ __forceinline__ void r2c_line_fx(const longlong2* src, longlong2* xl, int t, const double2* twH, SYNC sync) {
+  using FX = typename F::template with_type<long long>;
+  longlong2 q[F::E];
+#pragma unroll
+  for (int s = 0; s < F::E; ++s) q[s] = src[pidx_split<LIN>(t, F::in_const(s), F::TBITS)];
+  FX::run(q, t, xl, 1, fx_table<H>(twH), sync);
+  sync();
+#pragma unroll
+  for (int s = 0; s < F::E; ++s) xl[F::out_slot(t, s)] = q[s];
+  sync();
+}
+// output k of the r2c of a transformed line
+template <int H, int LAY>
+__device__ __forceinline__ double2 r2c_line_out(const longlong2* xl, int k, int xs, const double2* twM) {
+  const longlong2 zk = xl[pidx<LAY>(k == H ? 0 : k)], zh = xl[pidx<LAY>(k == 0 || k == H ? 0 : H - k)];
+  return fx::to_c(r2c_post_fx(zk, zh, fx_table<2 * H>(twM)[k]), xs + 1);
+}
+
+}  // namespace mf

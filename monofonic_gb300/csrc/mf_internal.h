@@ -31,7 +31,11 @@ bool length_supported(int L);
 // grid sizes N the pipeline supports (N, 3N/2, N/2, 3N/4 all compiled)
 bool grid_size_supported(int n);
 
-// per-context twiddle tables w_L^j = exp(-2 pi i j / L), j in [0, L)
+// fixed-point twiddles of length L (mf_fx.cuh)
+void fx_twiddles(int L, longlong2* out);
+
+// per-context twiddle tables w_L^j = exp(-2 pi i j / L), j in [0, L); an FP64
+// table is followed by its L fixed-point twiddles
 class TwiddleCache {
  public:
   ~TwiddleCache();

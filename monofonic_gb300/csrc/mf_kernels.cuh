@@ -16,6 +16,7 @@
 #include <type_traits>
 
 #include "mf_fft.cuh"
+#include "mf_fx.cuh"
 #include "mf_tma.cuh"
 
 // largest radix of the pipelined strided passes' plans (a build-time knob)
@@ -48,6 +49,7 @@ namespace mf {
 __host__ __device__ constexpr int col_minb(int threads, int e, int scalar_bytes) {
   if (!MF_COL_REG_SIZED) return threads <= MF_COL_MINB_LIMIT ? 2 : 1;
   int need = 4 * e * (scalar_bytes / 4) + 32;
+  if (scalar_bytes == 8 && need > 168) need = 168;  // fixed-point FP64 columns: three 128-thread CTAs
   need = need < 64 ? 64 : (need > 255 ? 255 : need);
   const int b = 65536 / (threads * need);
   return b < 1 ? 1 : (b > 4 ? 4 : b);
@@ -91,6 +93,18 @@ k_colfft(OP op, const cplx<T>* __restrict__ tw, int ncols) {
   const int col = blockIdx.x * NCOL + c;
   const int slab = blockIdx.y;
   const bool valid = col < ncols;
+  if constexpr (sizeof(T) == 8) {
+#pragma unroll 1
+    for (int i = 0; i < F::E; ++i)
+      sm[tile_slot<F, NCOL>(t, i) + c] = valid ? op.load(slab, t + i * F::TPL, col) : mkc<T>(T(0), T(0));
+    const int xs = col_fx<F, NCOL>(sm, t, c, tw);
+    if (!valid) return;
+#pragma unroll 2
+    for (int i = 0; i < F::E; ++i)
+      op.store(slab, t + i * F::TPL, col,
+               fx::to_c(reinterpret_cast<const longlong2*>(sm)[tile_slot<F, NCOL>(t, i) + c], xs));
+    return;
+  }
   C v[F::E];
 #pragma unroll
   for (int s = 0; s < F::E; ++s) {
@@ -167,6 +181,29 @@ k_colfft3s(OP op, const cplx<T>* __restrict__ tw, int ncols) {
   const int col = blockIdx.x * NCOL + c;
   const int slab = blockIdx.y;
   const bool valid = col < ncols;
+  if constexpr (sizeof(T) == 8) {
+#pragma unroll 1
+    for (int i = 0; i < F::E; ++i) {
+      C w[3] = {mkc<T>(T(0), T(0)), mkc<T>(T(0), T(0)), mkc<T>(T(0), T(0))};
+      if (valid) op.load3(slab, t + i * F::TPL, col, w);
+      const int o = tile_slot<F, NCOL>(t, i) + c;
+      xchg[o] = w[0];
+      tile1[o] = w[1];
+      tile2[o] = w[2];
+    }
+#pragma unroll 1
+    for (int d = 0; d < 3; ++d) {
+      C* tl = xchg + d * L * NCOL;
+      const int xs = col_fx<F, NCOL>(tl, t, c, tw);
+      if (valid) {
+#pragma unroll 2
+        for (int i = 0; i < F::E; ++i)
+          op.store(d, slab, t + i * F::TPL, col,
+                   fx::to_c(reinterpret_cast<const longlong2*>(tl)[tile_slot<F, NCOL>(t, i) + c], xs));
+      }
+    }
+    return;
+  }
   C v[F::E];
 #pragma unroll
   for (int s = 0; s < F::E; ++s) {
@@ -238,7 +275,7 @@ k_colfft_pipe(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nsl
   using I = LineIdx<F::TPL>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf0 = reinterpret_cast<C*>(smem_raw);
-  C* buf1 = buf0 + L * NCOL;
+  [[maybe_unused]] C* buf1 = buf0 + L * NCOL;
   const int c = threadIdx.x, t = threadIdx.y;
   const int total = ntc * nslab * nz;
   auto issue = [&](const TilePos& p, C* buf) {
@@ -255,6 +292,34 @@ k_colfft_pipe(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nsl
     }
     cp_async_commit();
   };
+  if constexpr (sizeof(T) == 8) {
+    // FP64 columns in fixed point: bound by the integer pipes, so one buffer
+    // per CTA and more CTAs per SM instead of a second buffer
+    const TilePos step = TilePos::of(gridDim.x, ntc, nslab);
+    TilePos p = TilePos::of(blockIdx.x, ntc, nslab);
+    for (int tl = blockIdx.x; tl < total; tl += gridDim.x, p = p.next(step, ntc, nslab)) {
+      issue(p, buf0);
+      cp_async_wait<0>();
+      const int col = p.ct * NCOL + c;
+      if constexpr (has_tile_prep<OP>::value) {
+        const auto tp = op.tile_prep(p.z, p.slab, col);
+#pragma unroll 2
+        for (int i = 0; i < F::E; ++i) {
+          const int o = tile_slot<F, NCOL>(t, i) + c;
+          buf0[o] = op.xform_tile(tp, t + i * F::TPL, buf0[o]);
+        }
+      }
+      const int xs = col_fx<F, NCOL>(buf0, t, c, tw);
+      if (col < ncols) {
+#pragma unroll 2
+        for (int i = 0; i < F::E; ++i)
+          op.store_z(p.z, p.slab, t + i * F::TPL, col,
+                     fx::to_c(reinterpret_cast<const longlong2*>(buf0)[tile_slot<F, NCOL>(t, i) + c], xs));
+      }
+      // (a thread's next copies overwrite only elements that it read itself)
+    }
+    return;
+  }
   int tl = blockIdx.x;
   const TilePos step = TilePos::of(gridDim.x, ntc, nslab);
   TilePos nx = TilePos::of(tl, ntc, nslab);
@@ -302,101 +367,6 @@ k_colfft_pipe(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nsl
 }
 
 // ---------------------------------------------------------------------------
-// The same pass with one column per line group inside a warp (a build-time
-// variant, MF_COL_WPC): the tile is staged column-major ([column][row], column
-// stride LSC = 4 mod 16 elements, so the row-major staging copies and the
-// copy-out reads take the minimum number of wavefronts), each column's
-// transform exchanges through its own column under warp barriers (the XOR
-// layout of the contiguous-line passes), and the results go back to global
-// memory in 64-byte row runs from a column-major copy-out.  Ops with a
-// prefetched read-modify-write target are not eligible.
-// ---------------------------------------------------------------------------
-template <typename T, int L, bool INV>
-__host__ __device__ constexpr int wpc_lsc() {
-  constexpr int base = padded_len(L, zlayout(L));
-  return base + ((4 - base % 16) % 16 + 16) % 16;
-}
-template <typename T, int L, bool INV, class OP>
-__host__ __device__ constexpr bool wpc_ok() {
-  using F = LineFFT<T, L, INV, MF_COL_MAXR>;
-  return !OP::kPrefetch && F::TPL <= 32 && 32 % F::TPL == 0;
-}
-template <typename T, int L, bool INV, int NCOL, class OP>
-__global__ void __launch_bounds__(NCOL * LineFFT<T, L, INV, MF_COL_MAXR>::TPL,
-                                  col_minb(NCOL * LineFFT<T, L, INV, MF_COL_MAXR>::TPL,
-                                           LineFFT<T, L, INV, MF_COL_MAXR>::E, (int)sizeof(T)))
-k_colfft_wpc(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nslab, int nz) {
-  using F = LineFFT<T, L, INV, MF_COL_MAXR, zlayout(L)>;
-  using C = cplx<T>;
-  constexpr int LSC = wpc_lsc<T, L, INV>();
-  constexpr int NT = NCOL * F::TPL;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* buf0 = reinterpret_cast<C*>(smem_raw);
-  C* buf1 = buf0 + NCOL * LSC;
-  const int tid = threadIdx.x;
-  const int cl = tid / F::TPL, t = tid % F::TPL;  // this thread's column in the tile and its line slot
-  const int total = ntc * nslab * nz;
-  auto issue = [&](int tl, C* buf) {
-    const int ct = tl % ntc, r = tl / ntc, slab = r % nslab, z = r / nslab;
-#pragma unroll 4
-    for (int u = tid; u < L * NCOL; u += NT) {
-      const int e = u / NCOL, c = u % NCOL;
-      const int col = ct * NCOL + c;
-      C* d = buf + c * LSC + e;
-      const C* g = (col < ncols) ? op.srcp(z, slab, e, col) : nullptr;
-      if (g) {
-        if constexpr (sizeof(C) == 16) cp_async16(d, g); else cp_async8(d, g);
-      } else {
-        *d = mkc<T>(T(0), T(0));
-      }
-    }
-    cp_async_commit();
-  };
-  int tl = blockIdx.x;
-  if (tl < total) issue(tl, buf0); else cp_async_commit();
-  for (int it = 0; tl < total; tl += gridDim.x, ++it) {
-    C* cur = (it & 1) ? buf1 : buf0;
-    C* nxt = (it & 1) ? buf0 : buf1;
-    const int tn = tl + gridDim.x;
-    if (tn < total) issue(tn, nxt); else cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();  // every thread's copies of this tile have landed
-    const int ct = tl % ntc, r = tl / ntc, slab = r % nslab, z = r / nslab;
-    const int col = ct * NCOL + cl;
-    const bool valid = col < ncols;
-    C* cb = cur + cl * LSC;
-    C v[F::E];
-    if constexpr (has_tile_prep<OP>::value) {
-      const auto tp = op.tile_prep(z, slab, col);
-#pragma unroll
-      for (int s = 0; s < F::E; ++s) {
-        const int e = F::in_index(t, s);
-        v[s] = valid ? op.xform_tile(tp, e, cb[e]) : mkc<T>(T(0), T(0));
-      }
-    } else {
-#pragma unroll
-      for (int s = 0; s < F::E; ++s) {
-        const int e = F::in_index(t, s);
-        v[s] = valid ? op.xform(z, slab, e, col, cb[e]) : mkc<T>(T(0), T(0));
-      }
-    }
-    F::run(v, t, cb, 1, tw, SyncWarp{});
-    __syncwarp();  // the column's last exchange has been read
-#pragma unroll
-    for (int s = 0; s < F::E; ++s) cb[F::out_index(t, s)] = v[s];
-    __syncthreads();  // every column of the tile is transformed
-#pragma unroll 4
-    for (int u = tid; u < L * NCOL; u += NT) {
-      const int e = u / NCOL, c = u % NCOL;
-      const int cc = ct * NCOL + c;
-      if (cc < ncols) op.store_z(z, slab, e, cc, cur[c * LSC + e]);
-    }
-    __syncthreads();  // cur is refilled by the next iteration's copies
-  }
-  cp_async_wait<0>();
-}
-
-// ---------------------------------------------------------------------------
 // strided forward transform, truncation and inverse transform of one column in
 // one pass (ConvXTruncOp), persistent and double-buffered as k_colfft_pipe
 // ---------------------------------------------------------------------------
@@ -412,7 +382,7 @@ k_colfft_trunc(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int ns
   using C = cplx<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf0 = reinterpret_cast<C*>(smem_raw);
-  C* buf1 = buf0 + L * NCOL;
+  [[maybe_unused]] C* buf1 = buf0 + L * NCOL;
   const int c = threadIdx.x, t = threadIdx.y;
   using I = LineIdx<FF::TPL>;
   const int total = ntc * nslab;
@@ -430,6 +400,29 @@ k_colfft_trunc(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int ns
     }
     cp_async_commit();
   };
+  if constexpr (sizeof(T) == 8) {  // one buffer, as in k_colfft_pipe
+    const TilePos step = TilePos::of(gridDim.x, ntc, nslab);
+    TilePos p = TilePos::of(blockIdx.x, ntc, nslab);
+    for (int tl = blockIdx.x; tl < total; tl += gridDim.x, p = p.next(step, ntc, nslab)) {
+      issue(p, buf0);
+      cp_async_wait<0>();
+      const int col = p.ct * NCOL + c;
+      int xs = col_fx<FF, NCOL>(buf0, t, c, tw);
+#pragma unroll 2
+      for (int i = 0; i < FF::E; ++i) {
+        const int o = tile_slot<FF, NCOL>(t, i) + c;
+        buf0[o] = op.mask(p.slab, t + i * FF::TPL, col, fx::to_c(reinterpret_cast<const longlong2*>(buf0)[o], xs));
+      }
+      xs = col_fx<FI, NCOL>(buf0, t, c, tw);
+      if (col < ncols) {
+#pragma unroll 2
+        for (int i = 0; i < FF::E; ++i)
+          *op.at(p.slab, t + i * FF::TPL, col) =
+              fx::to_c(reinterpret_cast<const longlong2*>(buf0)[tile_slot<FF, NCOL>(t, i) + c], xs);
+      }
+    }
+    return;
+  }
   int tl = blockIdx.x;
   const TilePos step = TilePos::of(gridDim.x, ntc, nslab);
   TilePos nx = TilePos::of(tl, ntc, nslab);
@@ -481,6 +474,19 @@ __global__ void __launch_bounds__(NT) k_zr2c(OP op, const cplx<T>* __restrict__ 
   const int line = blockIdx.x * blockDim.y + ly;
   const bool valid = line < nlines;
   C* sm = reinterpret_cast<C*>(smem_raw) + ly * (H + 1);
+  if constexpr (sizeof(T) == 8) {
+#pragma unroll 4
+    for (int i = 0; i < F::E; ++i)
+      sm[t + i * F::TPL] = valid ? op.load_pair(line, t + i * F::TPL) : mkc<T>(T(0), T(0));
+    const int xs = r2c_line_to_fx<H, F::TPL, 0>(sm, t, ly, SYNC{});
+    longlong2* sx = reinterpret_cast<longlong2*>(sm);
+    r2c_line_fx<F, H, 0>(sx, sx, t, twH, SYNC{});
+    if (valid) {
+#pragma unroll 2
+      for (int k = t; k < kout; k += F::TPL) op.store(line, k, r2c_line_out<H, 0>(sx, k, xs, twM));
+    }
+    return;
+  }
   C v[F::E];
 #pragma unroll
   for (int s = 0; s < F::E; ++s) v[s] = valid ? op.load_pair(line, F::in_index(t, s)) : mkc<T>(T(0), T(0));
@@ -530,6 +536,16 @@ __global__ void __launch_bounds__(NT) k_zc2r(OP op, const cplx<T>* __restrict__ 
   const bool valid = line < nlines;
   C* sm = reinterpret_cast<C*>(smem_raw) + ly * (H + 1);
   for (int k = t; k <= H; k += F::TPL) sm[k] = (valid && k < kin) ? op.load(line, k) : mkc<T>(T(0), T(0));
+  if constexpr (sizeof(T) == 8) {
+    const int xs = c2r_line_to_fx<H, F::TPL>(sm, H + 1, t, ly, SYNC{});
+    longlong2* sx = reinterpret_cast<longlong2*>(sm);
+    c2r_line_fx<F, H>(sx, H + 1, sx, t, twH, twM, SYNC{});
+    if (valid) {
+#pragma unroll 2
+      for (int i = 0; i < F::E; ++i) op.store_pair(line, t + i * F::TPL, fx::to_c(sx[t + i * F::TPL], xs));
+    }
+    return;
+  }
   SYNC{}();
   C v[F::E];
 #pragma unroll
@@ -683,12 +699,28 @@ __global__ void __launch_bounds__(LPB * LineFFT<T, H, true>::TPL, (LineFFT<T, H,
 #pragma unroll
     for (int d = 0; d < 3; ++d) sm[d] = cur + d * LPB * Kz + ly * Kz;
     C v[3][F::E];
+    if constexpr (sizeof(T) == 8) {
+      int xs[3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d)
+      for (int d = 0; d < 3; ++d) xs[d] = c2r_line_to_fx<H, F::TPL>(sm[d], Kz, t, ly, SYNC{});
+#pragma unroll 1
+      for (int d = 0; d < 3; ++d) {
+        longlong2* sx = reinterpret_cast<longlong2*>(cur + d * LPB * Kz + ly * Kz);
+        c2r_line_fx<F, H>(sx, Kz, sx, t, twH, twM, SYNC{});
+      }
 #pragma unroll
-      for (int s = 0; s < F::E; ++s) v[d][s] = c2r_pre<T, H>(sm[d], F::in_index(t, s), twM);
+      for (int d = 0; d < 3; ++d)
 #pragma unroll
-    for (int d = 0; d < 3; ++d) F::run(v[d], t, sm[d], 1, twH, SYNC{});
+        for (int s = 0; s < F::E; ++s)
+          v[d][s] = fx::to_c(reinterpret_cast<const longlong2*>(sm[d])[F::out_slot(t, s)], xs[d]);
+    } else {
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int s = 0; s < F::E; ++s) v[d][s] = c2r_pre<T, H>(sm[d], F::in_index(t, s), twM);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) F::run(v[d], t, sm[d], 1, twH, SYNC{});
+    }
     if (valid) lattice_line_out<T, H, P>(a, line, t, v);
     __syncthreads();  // cur is refilled by the next iteration's copies
   }
@@ -831,9 +863,11 @@ __host__ __device__ constexpr int zslot_of(int a) {
 // CTAs per SM the FP32 r2c z pass (MODE 2) is compiled for: it exchanges in
 // its staged input lines, so four fit by shared memory at 128 registers
 // (0 elsewhere: no minimum, the compiler's register choice)
+// FP64 (fixed point): 168 registers, 12 warps
 template <typename T, int MODE>
-__host__ __device__ constexpr int zconv_tma_minb() {
-  return sizeof(T) != 4 ? 0 : (MODE == 2 ? 4 : 0);
+__host__ __device__ constexpr int zconv_tma_minb(int threads) {
+  if (sizeof(T) != 4) return 65536 / (168 * threads) > 16 ? 16 : (65536 / (168 * threads) > 0 ? 65536 / (168 * threads) : 1);
+  return MODE == 2 ? 4 : 0;
 }
 // the r2c mode exchanges in its staged input lines (kin = H, zstage_stride
 // apart) when the exchange stride of a line fits in one
@@ -841,8 +875,15 @@ template <int H, int MODE>
 __host__ __device__ constexpr bool zconv_xchg_in_stage() {
   return MODE == 2 && zline_stride(H) <= zstage_stride(H);
 }
+// FP64 lines are staged one by one, zfx_stride elements apart, and transformed
+// in place in fixed point
+template <int H>
+__host__ __device__ constexpr int zfx_stride(int kin) {
+  return zline_stride(H) > kin ? zline_stride(H) : kin;
+}
 template <typename T, int H, int MAXR, int LPB, class SYNC, int MODE = 0, int KIN = 0>
-__global__ void __launch_bounds__(LPB * LineFFT<T, H, true, MAXR>::TPL, zconv_tma_minb<T, MODE>())
+__global__ void __launch_bounds__(LPB * LineFFT<T, H, true, MAXR>::TPL,
+                                  zconv_tma_minb<T, MODE>(LPB * LineFFT<T, H, true, MAXR>::TPL))
 k_zconv_tma(ZConvArgs<T> a, const cplx<T>* __restrict__ twH, const cplx<T>* __restrict__ twM) {
   constexpr int LAY = zlayout(H);
   using FI = LineFFT<T, H, true, MAXR, LAY, true>;
@@ -877,6 +918,63 @@ k_zconv_tma(ZConvArgs<T> a, const cplx<T>* __restrict__ twH, const cplx<T>* __re
     fence_mbar_init();
   }
   __syncthreads();
+  if constexpr (sizeof(T) == 8) {
+    // One buffer per CTA: the pass is bound by the integer pipes, and smaller
+    // CTAs fill the SM better than a second buffer.  The conversions are
+    // rolled loops over the staged line (mf_fx.cuh).
+    const int sl = zfx_stride<H>(kin);
+    const int kx = (MODE == 2) ? H : kin;
+    int it = 0;
+    for (int b = blockIdx.x; b < nbatch; b += gridDim.x, ++it) {
+      if (threadIdx.x < 32) {
+        fence_proxy_async_smem();
+        if (threadIdx.x == 0) mbar_arrive_expect_tx(&bars[0], (unsigned)(nop * LPB * kx * (int)sizeof(C)));
+        __syncwarp();
+        for (int l = threadIdx.x; l < nop * LPB; l += 32) {
+          const int op = l / LPB, ln = l - op * LPB;
+          const C* in = (op == 0) ? in0 : ((op == 1) ? in1 : in2);
+          tma_load_1d(stage + l * sl, in + ((long long)b * LPB + ln) * kx, (unsigned)(kx * sizeof(C)), &bars[0]);
+        }
+      }
+      const bool ok = mbar_wait_bounded(&bars[0], it & 1, a.err, 1);
+      if (!__syncthreads_and(ok)) return;
+      C* dst = a.out + (long long)(b * LPB + lg) * a.out_stride;
+      C* const l0 = stage + lg * sl;
+      if constexpr (MODE != 2) {
+        const int nops = (MODE == 0) ? nop : 1;
+#pragma unroll 1
+        for (int op = 0; op < nops; ++op) {
+          C* src = stage + (op * LPB + lg) * sl;
+          longlong2* xl = reinterpret_cast<longlong2*>(src);
+          const int xs = c2r_line_to_fx<H, TPL>(src, kin, t, lg, sync);
+          c2r_line_fx<FI, H>(xl, kin, xl, t, twH, twM, sync);
+          // (a thread reads back the elements that it wrote)
+          if (MODE == 0) sync();  // the product goes into the first line in another order
+#pragma unroll 2
+          for (int i = 0; i < E; ++i) {
+            const int m = t + i * TPL;
+            const C r = fx::to_c(xl[pidx<LAY>(m)], xs);
+            if (MODE == 1) dst[m] = r;
+            else l0[pidx<LAY>(m)] = (op == 0) ? r : mkc<T>(l0[pidx<LAY>(m)].x * r.x, l0[pidx<LAY>(m)].y * r.y);
+          }
+        }
+      }
+      if constexpr (MODE != 1) {
+        constexpr int LIN = (MODE == 0) ? LAY : 0;  // layout of the real-space line
+        longlong2* xl = reinterpret_cast<longlong2*>(l0);
+        const int xs = r2c_line_to_fx<H, TPL, LIN>(l0, t, lg, sync);
+        r2c_line_fx<FF, H, LIN>(xl, xl, t, twH, sync);
+        const bool unit = a.out_scale == T(1);
+#pragma unroll 2
+        for (int k = t; k < a.kout; k += TPL) {
+          const C r = r2c_line_out<H, LAY>(xl, k, xs, twM);
+          dst[k] = unit ? r : cscale(r, a.out_scale);
+        }
+      }
+      __syncthreads();  // the stage is read: the next batch may land in it
+    }
+    return;
+  }
   // run by the first warp
   auto issue = [&](int b, int st) {
     const long long off = (long long)b * LPB * kin;

@@ -61,7 +61,8 @@ constexpr int z_lpb() {
 
 template <typename K>
 inline cudaError_t set_smem(K kern, size_t smem) {
-  if (smem > 48 * 1024) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // (a kernel's static arrays, a few KB, count toward the 48 KB that need no opt-in)
+  if (smem > 40 * 1024) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   return cudaSuccess;
 }
 
@@ -80,37 +81,12 @@ constexpr int pipe_ncol() {
   return nc;
 }
 
-// 1: the pipelined strided passes with one column per warp where eligible
-// (k_colfft_wpc; a build-time knob)
-#ifndef MF_COL_WPC
-#define MF_COL_WPC 0
-#endif
-
 template <typename T, int L, bool INV, class OP>
 cudaError_t launch_col(OP op, int nslab, int ncols, int nz, const cplx<T>* tw, cudaStream_t s, int kind) {
-  if constexpr (OP::kPipe && MF_COL_PIPE && MF_COL_WPC && wpc_ok<T, L, INV, OP>()) {
+  if constexpr (OP::kPipe && MF_COL_PIPE) {
     constexpr int NC = pipe_ncol<T, L>();
     constexpr int TPL = LineFFT<T, L, INV, MF_COL_MAXR>::TPL;
-    const size_t smem = (size_t)2 * NC * wpc_lsc<T, L, INV>() * sizeof(cplx<T>);
-    auto kern = k_colfft_wpc<T, L, INV, NC, OP>;
-    cudaError_t e = set_smem(kern, smem);
-    if (e != cudaSuccess) return e;
-    int per_sm = 0, nsm = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NC * TPL, smem);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) per_sm = 1;
-    const int ntc = (ncols + NC - 1) / NC;
-    const int total = ntc * nslab * nz;
-    int grid = nsm * per_sm;
-    if (grid > total) grid = total;
-    kern<<<grid, NC * TPL, smem, s>>>(op, tw, ncols, ntc, nslab, nz);
-    return cudaGetLastError();
-  } else if constexpr (OP::kPipe && MF_COL_PIPE) {
-    constexpr int NC = pipe_ncol<T, L>();
-    constexpr int TPL = LineFFT<T, L, INV, MF_COL_MAXR>::TPL;
-    const size_t smem = (size_t)2 * L * NC * sizeof(cplx<T>);
+    const size_t smem = (size_t)(sizeof(T) == 8 ? 1 : 2) * L * NC * sizeof(cplx<T>);
     auto kern = k_colfft_pipe<T, L, INV, NC, OP>;
     cudaError_t e = set_smem(kern, smem);
     if (e != cudaSuccess) return e;
@@ -255,8 +231,9 @@ cudaError_t launch_zconv(const ZConvArgs<T>& a, const cplx<T>* twH, const cplx<T
       constexpr int KIN_CT = (MODE == 1 && H % 3 == 0) ? 2 * H / 3 + 1 : 0;
       auto kern = (KIN_CT != 0 && a.kin == KIN_CT) ? k_zconv_tma<T, H, MAXR, LPBT, SYNC, MODE, KIN_CT>
                                                    : k_zconv_tma<T, H, MAXR, LPBT, SYNC, MODE, 0>;
-      const size_t smem =
-          128 + ((size_t)2 * a.nop * LPBT * (MODE == 2 ? zstage_stride(H) : a.kin) + (zconv_xchg_in_stage<H, MODE>() ? 0 : (size_t)LPBT * zline_stride(H))) *
+      const size_t smem = sizeof(T) == 8
+          ? 128 + (size_t)a.nop * LPBT * zfx_stride<H>(a.kin) * sizeof(cplx<T>)
+          : 128 + ((size_t)2 * a.nop * LPBT * (MODE == 2 ? zstage_stride(H) : a.kin) + (zconv_xchg_in_stage<H, MODE>() ? 0 : (size_t)LPBT * zline_stride(H))) *
                     sizeof(cplx<T>);
       cudaError_t e = set_smem(kern, smem);
       if (e != cudaSuccess) return e;
@@ -387,6 +364,9 @@ cudaError_t Launch<T>::assemble3_xinv(int L, Assemble3XInvOp<T> op, int nslab, i
 template <typename T, int H>
 cudaError_t launch_zc2r3_lattice(const Lattice3Args& a, bool p64, const cplx<T>* twH, const cplx<T>* twM,
                                  cudaStream_t s) {
+  if constexpr (LineFFT<T, H, true>::E > 8) {
+    return cudaErrorInvalidValue;  // per-component passes there (assemble3_supported)
+  } else {
   // lines per batch: at most 256 threads, two batch buffers within ~100 KB so
   // that two CTAs share an SM
   constexpr int TPL = LineFFT<T, H, true>::TPL;
@@ -412,6 +392,7 @@ cudaError_t launch_zc2r3_lattice(const Lattice3Args& a, bool p64, const cplx<T>*
     return cudaGetLastError();
   };
   return p64 ? go(k_zc2r3_lattice<T, H, LPB, double>) : go(k_zc2r3_lattice<T, H, LPB, float>);
+  }
 }
 template <typename T>
 cudaError_t Launch<T>::z_c2r3_lattice(int H, const Lattice3Args& a, bool p64, const cplx<T>* twH,
@@ -452,7 +433,7 @@ template <typename T, int L, class OP>
 cudaError_t launch_xtrunc(OP op, int nslab, int ncols, const cplx<T>* tw, cudaStream_t s) {
   constexpr int NC = pipe_ncol<T, L>();
   constexpr int TPL = LineFFT<T, L, false, MF_COL_MAXR>::TPL;
-  const size_t smem = (size_t)2 * L * NC * sizeof(cplx<T>);
+  const size_t smem = (size_t)(sizeof(T) == 8 ? 1 : 2) * L * NC * sizeof(cplx<T>);
   auto kern = k_colfft_trunc<T, L, NC, OP>;
   cudaError_t e = set_smem(kern, smem);
   if (e != cudaSuccess) return e;

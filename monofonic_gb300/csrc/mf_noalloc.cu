@@ -38,7 +38,7 @@ constexpr int kNumTw = sizeof(kTwLens) / sizeof(kTwLens[0]);
 constexpr int kTwTotal = 12 + 24 + 48 + 72 + 96 + 144 + 192;
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
-static __device__ __align__(256) double2 g_tw64[kTwTotal];
+static __device__ __align__(256) double2 g_tw64[2 * kTwTotal];  // each table followed by its fixed-point twiddles
 static __device__ __align__(256) float2 g_tw32[kTwTotal];
 static __device__ int g_err;
 
@@ -78,7 +78,7 @@ int setup_device(int dev, DeviceState* out, std::string* why) {
     *why = std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e);
     return MF_ERR_CUDA;
   }
-  std::vector<double2> h64(kTwTotal);
+  std::vector<double2> h64(2 * kTwTotal);
   std::vector<float2> h32(kTwTotal);
   const long double pi = 3.141592653589793238462643383279502884L;
   int off = 0;
@@ -92,12 +92,13 @@ int setup_device(int dev, DeviceState* out, std::string* why) {
         re = c[q];
         im = s[q];
       }
-      h64[off + j] = make_double2(re, im);
+      h64[2 * off + j] = make_double2(re, im);
       h32[off + j] = make_float2((float)re, (float)im);
     }
+    fx_twiddles(L, reinterpret_cast<longlong2*>(h64.data() + 2 * off + L));
     off += L;
   }
-  e = cudaMemcpyToSymbol(g_tw64, h64.data(), sizeof(double2) * kTwTotal);
+  e = cudaMemcpyToSymbol(g_tw64, h64.data(), 2 * sizeof(double2) * kTwTotal);
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_tw32, h32.data(), sizeof(float2) * kTwTotal);
   if (e != cudaSuccess) {
     *why = std::string("twiddle upload: ") + cudaGetErrorString(e);
@@ -111,7 +112,7 @@ int setup_device(int dev, DeviceState* out, std::string* why) {
 template <typename T>
 const cplx<T>* tw_table(const DeviceState& st, int L);
 template <>
-const cplx<double>* tw_table<double>(const DeviceState& st, int L) { return st.tw64 + tw_offset(L); }
+const cplx<double>* tw_table<double>(const DeviceState& st, int L) { return st.tw64 + 2 * tw_offset(L); }
 template <>
 const cplx<float>* tw_table<float>(const DeviceState& st, int L) { return st.tw32 + tw_offset(L); }
 
