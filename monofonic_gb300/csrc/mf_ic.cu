@@ -134,42 +134,59 @@ __global__ void k_masses(P* mass, const T* delta, int n, int ishift, double pmea
   }
 }
 
-// amplitude table amp(k2) = k^{n_s/2} T(k) sqrt(pnorm), k = sqrt(k2)*kfac
-// (get_amplitude, include/cosmology_calculator.hh:405-408), FP64
-__global__ void k_amp_table(double* amp, int nk2, double kfac, const ICDyn* __restrict__ dyn, const double* tk) {
-  const double half_ns = dyn->half_ns, sqrtpnorm = dyn->sqrtpnorm;
-  for (int k2 = blockIdx.x * blockDim.x + threadIdx.x; k2 < nk2; k2 += gridDim.x * blockDim.x) {
-    const double k = sqrt((double)k2) * kfac;
-    const double t = tk ? tk[k2] : eh_eval(dyn->eh, k);
-    amp[k2] = pow(k, half_ns) * t * sqrtpnorm;
+// k-space indices of element idx of an n-grid (n <= 1024: the index and the
+// divisions fit 32 bits)
+struct KIndex {
+  int i, j, kz, ii, jj;
+  __device__ __forceinline__ KIndex(unsigned idx, int n) {
+    const unsigned Kz = (unsigned)n / 2 + 1;
+    const unsigned line = idx / Kz;
+    kz = (int)(idx - line * Kz);
+    i = (int)(line / (unsigned)n);
+    j = (int)(line - (unsigned)i * (unsigned)n);
+    ii = i - (i > n / 2 ? n : 0);
+    jj = j - (j > n / 2 ? n : 0);
   }
+  __device__ __forceinline__ int k2() const { return ii * ii + jj * jj + kz * kz; }
+};
+
+// phi(1) per noise mode, -amp(k) / k^2 with amp(k) = k^{n_s/2} T(k) sqrt(pnorm)
+// and k = sqrt(k2)*kfac (get_amplitude, include/cosmology_calculator.hh:405-408),
+// evaluated in FP64 and rounded once to the grid precision; zero at k2 = 0.
+// A few hundred FP64 operations per entry: one warp per block spreads the
+// table over all SMs (256-thread blocks put the 3073 entries of N=64 on 13:
+// 46 us)
+template <typename T>
+__global__ void __launch_bounds__(32) k_phi_table(T* out, int nk2, double kfac, const ICDyn* __restrict__ dyn,
+                                                  const double* tk) {
+  const double half_ns = dyn->half_ns, sqrtpnorm = dyn->sqrtpnorm;
+  const int k2 = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k2 >= nk2) return;
+  const double k = sqrt((double)k2) * kfac;
+  const double t = tk ? tk[k2] : eh_eval(dyn->eh, k);
+  const double amp = pow(k, half_ns) * t * sqrtpnorm;
+  out[k2] = k2 ? T(-amp / ((double)k2 * kfac * kfac)) : T(0);
 }
 
 // noise normalisation (ic_generator.cc:341-346) in place, then
-// phi = -wn amp(k) / k^2 with zero DC (ic_generator.cc:449-457)
+// phi = -wn amp(k) / k^2 with zero DC (ic_generator.cc:449-457) from the table:
+// a streaming pass (the square root and two divisions per mode that it
+// replaces bounded the FP64 form: 585 us at N=256)
 template <typename T>
-__global__ void k_phi1(cplx<T>* wn, cplx<T>* phi, int n, double kfac, const double* amp, double sign_over_volfac,
+__global__ void k_phi1(cplx<T>* wn, cplx<T>* phi, int n, const T* __restrict__ tab, double sign_over_volfac,
                        int fixing) {
-  const int Kz = n / 2 + 1;
-  const size_t tot = (size_t)n * n * Kz;
-  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < tot; idx += (size_t)gridDim.x * blockDim.x) {
-    const int kz = (int)(idx % Kz);
-    const int j = (int)((idx / Kz) % n);
-    const int i = (int)(idx / ((size_t)Kz * n));
-    const int ii = i - (i > n / 2 ? n : 0), jj = j - (j > n / 2 ? n : 0);
+  const unsigned tot = (unsigned)n * n * (n / 2 + 1);
+  const T sv = T(sign_over_volfac);
+  for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < tot; idx += gridDim.x * blockDim.x) {
+    const T a = tab[KIndex(idx, n).k2()];
     cplx<T> w = wn[idx];
     if (fixing) {
-      const T a = sqrt(w.x * w.x + w.y * w.y);
-      if (a != T(0)) w = mkc<T>(w.x / a, w.y / a);
+      const T m = sqrt(w.x * w.x + w.y * w.y);
+      if (m != T(0)) w = mkc<T>(w.x / m, w.y / m);
     }
-    w = mkc<T>(w.x * T(sign_over_volfac), w.y * T(sign_over_volfac));
+    w = mkc<T>(w.x * sv, w.y * sv);
     wn[idx] = w;
-    const T kx = T(ii) * T(kfac), ky = T(jj) * T(kfac), kk = T(kz) * T(kfac);
-    const T kmod = sqrt(kx * kx + ky * ky + kk * kk);
-    const int k2 = ii * ii + jj * jj + kz * kz;
-    const T a = T(amp[k2]);
-    const T den = kmod * kmod;
-    phi[idx] = (idx == 0) ? mkc<T>(T(0), T(0)) : mkc<T>(-(w.x * a) / den, -(w.y * a) / den);
+    phi[idx] = mkc<T>(w.x * a, w.y * a);
   }
 }
 
@@ -345,7 +362,7 @@ struct mf_ic {
   double* stage = nullptr;  // n^3 doubles: host noise upload of an FP32 pipeline
   int plt_ng = 0;
   mf_conv* conv = nullptr;
-  double* amp = nullptr;
+  double* amp = nullptr;  // phi(1) per noise mode and k2 (grid precision); from nk2 on a tabulated T(k)
   int nk2 = 0;
   void* dpos = nullptr;
   void* dvel = nullptr;
@@ -762,14 +779,14 @@ int enqueue_impl(mf_ic* ic) {
   ic->wn->space = MF_SPACE_K;
   {
     LaunchScope ls0(c, KK_POINTWISE);
-    k_amp_table<<<(ic->nk2 + 255) / 256, 256, 0, s>>>(ic->amp, ic->nk2, kfac, ic->dyn_d,
-                                                       ic->has_tk ? ic->amp + ic->nk2 : nullptr);
+    T* tab = reinterpret_cast<T*>(ic->amp);
+    k_phi_table<T><<<(ic->nk2 + 31) / 32, 32, 0, s>>>(tab, ic->nk2, kfac, ic->dyn_d,
+                                                      ic->has_tk ? ic->amp + ic->nk2 : nullptr);
     CK(cudaGetLastError());
     const double volfac = std::pow(L / n / 2.0 / M_PI, 1.5);
     const double sgn = (p.inversion ? -1.0 : 1.0) / volfac;
     LaunchScope ls1(c, KK_POINTWISE);
-    k_phi1<T><<<blocks_for(nk), kThreads, 0, s>>>((cplx<T>*)ic->wn->d, (cplx<T>*)ic->f[0]->d, n, kfac, ic->amp, sgn,
-                                                   p.fixing);
+    k_phi1<T><<<blocks_for(nk), kThreads, 0, s>>>((cplx<T>*)ic->wn->d, (cplx<T>*)ic->f[0]->d, n, tab, sgn, p.fixing);
     CK(cudaGetLastError());
     ic->f[0]->space = MF_SPACE_K;
   }

@@ -33,12 +33,13 @@ __global__ void k_zero_dc(T* d) {
 // apply_InverseLaplacian (grid_fft.hh:440-449): -x/k^2, then zero_DC_mode
 template <typename T>
 __global__ void k_invlap(cplx<T>* d, int n, T kfac) {
-  const int Kz = n / 2 + 1;
-  const size_t tot = (size_t)n * n * Kz;
-  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < tot; idx += (size_t)gridDim.x * blockDim.x) {
-    const int kz = (int)(idx % Kz);
-    const int j = (int)((idx / Kz) % n);
-    const int i = (int)(idx / ((size_t)Kz * n));
+  const unsigned Kz = n / 2 + 1;
+  const unsigned tot = (unsigned)n * n * Kz;  // n <= 1024
+  for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < tot; idx += gridDim.x * blockDim.x) {
+    const unsigned line = idx / Kz;
+    const int kz = (int)(idx - line * Kz);
+    const int i = (int)(line / (unsigned)n);
+    const int j = (int)(line - (unsigned)i * (unsigned)n);
     const T kx = kcomp<T>(i, n, kfac), ky = kcomp<T>(j, n, kfac), kk = kcomp<T>(kz, n, kfac);
     const T k2 = kx * kx + ky * ky + kk * kk;
     cplx<T> v = d[idx];
@@ -93,11 +94,16 @@ __global__ void k_shift(cplx<T>* d, int n, T kfac, T dx, T s0, T s1, T s2) {
 
 template <typename T>
 __global__ void k_fill_from_f64(T* d, const double* src, int n) {
-  const size_t tot = (size_t)n * n * n;
-  for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < tot; c += (size_t)gridDim.x * blockDim.x) {
-    const size_t line = c / n;
-    const int k = (int)(c % n);
-    d[line * (n + 2) + k] = T(src[c]);
+  // two cells of a row per thread (n even)
+  using T2 = typename cplx_of<T>::type;
+  const unsigned hn = (unsigned)n >> 1;
+  const unsigned tot = (unsigned)n * n * hn;
+  for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < tot; c += gridDim.x * blockDim.x) {
+    const unsigned line = c / hn;
+    const unsigned k = c - line * hn;
+    // (the caller's array is only 8-byte aligned)
+    const double v0 = src[2 * (size_t)c], v1 = src[2 * (size_t)c + 1];
+    reinterpret_cast<T2*>(d + (size_t)line * (n + 2))[k] = mkc<T>(T(v0), T(v1));
   }
 }
 
@@ -148,7 +154,8 @@ cudaError_t pw_zero_dc(T* d, cudaStream_t s) {
 }
 template <typename T>
 cudaError_t pw_invlap(cplx<T>* d, int n, double kfac, cudaStream_t s) {
-  k_invlap<T><<<grid_for((size_t)n * n * (n / 2 + 1), 4), kThreads, 0, s>>>(d, n, T(kfac));
+  // one mode per thread while that fits the grid: small fields wait on latency
+  k_invlap<T><<<grid_for((size_t)n * n * (n / 2 + 1)), kThreads, 0, s>>>(d, n, T(kfac));
   return cudaGetLastError();
 }
 template <typename T>
