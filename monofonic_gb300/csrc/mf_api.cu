@@ -195,6 +195,29 @@ cudaError_t fft3d_r2c(mf_ctx* c, T* data, int n) {
   return Launch<T>::colfft_plain(n, false, PlainStridedOp<T>{z, (long long)n * Kz, Kz, norm}, n, Kz, twN, s);
 }
 
+cudaError_t fft3d_r2c_butterfly(mf_ctx* c, double* data, int n) {
+  cudaStream_t s = c->stream;
+  const int H = n / 2, Kz = H + 1;
+  const double2* twH = c->tw.get<double>(H, s);
+  const double2* twN = c->tw.get<double>(n, s);
+  if (!twH || !twN) return cudaErrorMemoryAllocation;
+  const double norm = 1.0 / std::sqrt((double)n * (double)n * (double)n);
+  cudaError_t e;
+  {
+    LaunchScope ls(c, KK_FFT_Z);
+    e = Launch<double>::z_r2c_butterfly(H, PlainZButterflyOp{{data, n, 1.0}}, n * n, Kz, twH, twN, s);
+  }
+  if (e != cudaSuccess) return e;
+  double2* z = reinterpret_cast<double2*>(data);
+  {
+    LaunchScope ls(c, KK_FFT_COL);
+    e = Launch<double>::colfft_butterfly(n, PlainStridedButterflyOp{{z, Kz, (long long)n * Kz, 1.0}}, n, Kz, twN, s);
+  }
+  if (e != cudaSuccess) return e;
+  LaunchScope ls(c, KK_FFT_COL);
+  return Launch<double>::colfft_butterfly(n, PlainStridedButterflyOp{{z, (long long)n * Kz, Kz, norm}}, n, Kz, twN, s);
+}
+
 template <typename T>
 cudaError_t fft3d_c2r(mf_ctx* c, T* data, int n) {
   cudaStream_t s = c->stream;

@@ -80,6 +80,11 @@ struct Launch {
   // z passes
   static cudaError_t z_r2c_plain(int H, PlainZOp<T> op, int nlines, int kout, const cplx<T>* twH,
                                  const cplx<T>* twM, cudaStream_t s);
+  // forward passes with FP64 butterflies (double only)
+  static cudaError_t colfft_butterfly(int L, PlainStridedButterflyOp op, int nslab, int ncols, const double2* tw,
+                                      cudaStream_t s);
+  static cudaError_t z_r2c_butterfly(int H, PlainZButterflyOp op, int nlines, int kout, const double2* twH,
+                                     const double2* twM, cudaStream_t s);
   static cudaError_t z_c2r_plain(int H, PlainZOp<T> op, int nlines, int kin, const cplx<T>* twH,
                                  const cplx<T>* twM, cudaStream_t s);
   static cudaError_t z_conv(int H, const ZConvArgs<T>& a, const cplx<T>* twH, const cplx<T>* twM,
@@ -92,5 +97,11 @@ struct Launch {
   static cudaError_t z_r2c_tma(int H, const ZConvArgs<T>& a, const cplx<T>* twH, const cplx<T>* twM,
                                cudaStream_t s);
 };
+
+template <>
+cudaError_t Launch<double>::colfft_butterfly(int, PlainStridedButterflyOp, int, int, const double2*, cudaStream_t);
+template <>
+cudaError_t Launch<double>::z_r2c_butterfly(int, PlainZButterflyOp, int, int, const double2*, const double2*,
+                                            cudaStream_t);
 
 }  // namespace mf

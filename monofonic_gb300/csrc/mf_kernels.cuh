@@ -71,6 +71,17 @@ __host__ __device__ constexpr int col_layout() {
   return (col_swizzle<OP>::value && NCOL * (int)sizeof(cplx<T>) == 64) ? 2 : 0;
 }
 
+// whether a pass transforms its lines in fixed point: FP64, unless the op asks
+// for FP64 butterflies
+template <class OP, class = void>
+struct butterfly_op : std::false_type {};
+template <class OP>
+struct butterfly_op<OP, std::void_t<decltype(OP::kButterflies)>> : std::true_type {};
+template <typename T, class OP>
+__host__ __device__ constexpr bool fixed_point_lines() {
+  return sizeof(T) == 8 && !butterfly_op<OP>::value;
+}
+
 // ops with a per-tile prologue (tile_prep / xform_tile) in the pipelined pass
 template <class OP, class = void>
 struct has_tile_prep : std::false_type {};
@@ -292,7 +303,7 @@ k_colfft_pipe(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nsl
     }
     cp_async_commit();
   };
-  if constexpr (sizeof(T) == 8) {
+  if constexpr (fixed_point_lines<T, OP>()) {
     // FP64 columns in fixed point: bound by the integer pipes, so one buffer
     // per CTA and more CTAs per SM instead of a second buffer
     const TilePos step = TilePos::of(gridDim.x, ntc, nslab);
@@ -474,7 +485,7 @@ __global__ void __launch_bounds__(NT) k_zr2c(OP op, const cplx<T>* __restrict__ 
   const int line = blockIdx.x * blockDim.y + ly;
   const bool valid = line < nlines;
   C* sm = reinterpret_cast<C*>(smem_raw) + ly * (H + 1);
-  if constexpr (sizeof(T) == 8) {
+  if constexpr (fixed_point_lines<T, OP>()) {
 #pragma unroll 4
     for (int i = 0; i < F::E; ++i)
       sm[t + i * F::TPL] = valid ? op.load_pair(line, t + i * F::TPL) : mkc<T>(T(0), T(0));

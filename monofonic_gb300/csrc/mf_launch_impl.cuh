@@ -86,7 +86,7 @@ cudaError_t launch_col(OP op, int nslab, int ncols, int nz, const cplx<T>* tw, c
   if constexpr (OP::kPipe && MF_COL_PIPE) {
     constexpr int NC = pipe_ncol<T, L>();
     constexpr int TPL = LineFFT<T, L, INV, MF_COL_MAXR>::TPL;
-    const size_t smem = (size_t)(sizeof(T) == 8 ? 1 : 2) * L * NC * sizeof(cplx<T>);
+    const size_t smem = (size_t)(fixed_point_lines<T, OP>() ? 1 : 2) * L * NC * sizeof(cplx<T>);
     auto kern = k_colfft_pipe<T, L, INV, NC, OP>;
     cudaError_t e = set_smem(kern, smem);
     if (e != cudaSuccess) return e;
@@ -408,6 +408,23 @@ template cudaError_t Launch<MF_T>::colfft_plain(int, bool, PlainStridedOp<MF_T>,
 template cudaError_t Launch<MF_T>::assemble_xinv(int, AssembleXInvOp<MF_T>, int, int, const cplx<MF_T>*, cudaStream_t);
 template cudaError_t Launch<MF_T>::z_r2c_plain(int, PlainZOp<MF_T>, int, int, const cplx<MF_T>*, const cplx<MF_T>*, cudaStream_t);
 template cudaError_t Launch<MF_T>::z_c2r_plain(int, PlainZOp<MF_T>, int, int, const cplx<MF_T>*, const cplx<MF_T>*, cudaStream_t);
+#endif
+
+#if defined(MF_PART_BUTTERFLY)
+template <>
+cudaError_t Launch<double>::colfft_butterfly(int L, PlainStridedButterflyOp op, int nslab, int ncols,
+                                             const double2* tw, cudaStream_t s) {
+#define CASE(LL) case LL: return launch_col<double, LL, false>(op, nslab, ncols, 1, tw, s, KK_FFT_COL);
+  switch (L) { MF_LEN_N(CASE) default: return cudaErrorInvalidValue; }
+#undef CASE
+}
+template <>
+cudaError_t Launch<double>::z_r2c_butterfly(int H, PlainZButterflyOp op, int nlines, int kout, const double2* twH,
+                                            const double2* twM, cudaStream_t s) {
+#define CASE(HH) case HH: return launch_zr2c<double, HH>(op, nlines, kout, twH, twM, s);
+  switch (H) { MF_LEN_NH(CASE) default: return cudaErrorInvalidValue; }
+#undef CASE
+}
 #endif
 
 #if defined(MF_PART_CONVX)

@@ -598,6 +598,11 @@ struct PlainStridedOp {
   }
 };
 
+// the same with FP64 butterflies instead of fixed point (the PLT tables)
+struct PlainStridedButterflyOp : PlainStridedOp<double> {
+  static constexpr bool kButterflies = true;
+};
+
 // plain z pass on the in-place padded layout: line = i*n + j, row of n+2 reals
 template <typename T>
 struct PlainZOp {
@@ -617,6 +622,10 @@ struct PlainZOp {
   __device__ __forceinline__ void store_pair(int line, int m, C v) const {
     reinterpret_cast<C*>(p + (long long)line * (n + 2))[m] = mkc<T>(v.x * scale, v.y * scale);
   }
+};
+
+struct PlainZButterflyOp : PlainZOp<double> {
+  static constexpr bool kButterflies = true;
 };
 
 // Shared-source form of the Orszag convolutions: every padded operand field

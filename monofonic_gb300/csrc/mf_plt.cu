@@ -393,7 +393,7 @@ int plt_build_tables(mf_ctx* c, int lattice, int ng, PLTTables* out) {
       CK(cudaGetLastError());
     }
     // forward transforms (unitary), real parts read by the eigen pass
-    for (int m = 0; m < 6; ++m) CK(fft3d_r2c<double>(c, grids + m * greals, nl));
+    for (int m = 0; m < 6; ++m) CK(fft3d_r2c_butterfly(c, grids + m * greals, nl));
     EigenArgs ga{};
     ga.L = LT;
     ga.nl = nl;

@@ -90,6 +90,10 @@ inline size_t prec_size(int prec) { return prec == MF_PREC_F32 ? 4 : 8; }
 // 3D transforms on an n-grid in the padded in-place layout (unitary)
 template <typename T> cudaError_t fft3d_r2c(mf_ctx* c, T* data, int n);
 template <typename T> cudaError_t fft3d_c2r(mf_ctx* c, T* data, int n);
+// the FP64 forward transform with FP64 butterflies.  The PLT tables take it:
+// the eigenvectors of a degenerate mode are fixed by the rounding of the
+// dynamical matrix alone, so another rounding is another (equally valid) table
+cudaError_t fft3d_r2c_butterfly(mf_ctx* c, double* data, int n);
 
 // convolution on k-space N-grids
 template <typename T>
