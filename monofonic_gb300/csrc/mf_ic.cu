@@ -231,49 +231,6 @@ __global__ void k_phitot(cplx<T>* out, const cplx<T>* p1, const cplx<T>* p2, con
   }
 }
 
-// lattice readout of the three components of one sub-lattice
-// (set_positions / set_velocities, particle_generator.hh:499-639): particle
-// ip = ishift*n^3 + cell, AoS [ip][3]; positions q + Psi in FP64 with
-// q_d = (idx_d + s_d)/n * lunit (get_unit_r_shifted, grid_fft.hh:242-252)
-template <typename T, typename P>
-__global__ void k_lattice3(const T* psi0, const T* psi1, const T* psi2, int n, P* dst, int ishift,
-                           const double* __restrict__ q, int with_q, int fields_mode,
-                           const float2* __restrict__ qf = nullptr) {
-  const size_t n3 = (size_t)n * n * n;
-  for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n3; c += (size_t)gridDim.x * blockDim.x) {
-    const size_t line = c / n;
-    const int k = (int)(c % n);
-    const size_t off = line * (n + 2) + k;
-    if constexpr (std::is_same<P, float>::value && std::is_same<T, float>::value) {
-      if (with_q && !fields_mode) {  // FP32 positions: q as a float pair (ff_add_q)
-        const int j = (int)(line % n), i = (int)(line / n);
-        P* o = dst + 3 * ((size_t)ishift * n3 + c);
-        o[0] = ff_add_q(qf[i], psi0[off]);
-        o[1] = ff_add_q(qf[n + j], psi1[off]);
-        o[2] = ff_add_q(qf[2 * n + k], psi2[off]);
-        continue;
-      }
-    }
-    double v0 = (double)psi0[off], v1 = (double)psi1[off], v2 = (double)psi2[off];
-    if (fields_mode) {
-      dst[c] = (P)v0;
-      dst[n3 + c] = (P)v1;
-      dst[2 * n3 + c] = (P)v2;
-      continue;
-    }
-    if (with_q) {  // q_d = (idx_d + s_d) / n * lunit, tabulated on the host
-      const int j = (int)(line % n), i = (int)(line / n);
-      v0 = q[i] + v0;
-      v1 = q[n + j] + v1;
-      v2 = q[2 * n + k] + v2;
-    }
-    P* o = dst + 3 * ((size_t)ishift * n3 + c);
-    o[0] = (P)v0;
-    o[1] = (P)v1;
-    o[2] = (P)v2;
-  }
-}
-
 // PLT gradient and growth-rate correction of every N-grid mode, tabulated
 // once per pipeline (they depend on the lattice, N and the PLT mesh only):
 // out[4 idx + {0,1,2,3}] = g_x, g_y, g_z, vfac_corr
@@ -914,9 +871,8 @@ int enqueue_impl(mf_ic* ic) {
     void* dst = sp ? (vel ? ic->bvel : ic->bpos) : (vel ? ic->dvel : ic->dpos);
     const double* qbase = sp ? ic->bqtab : ic->qtab;
     const float2* qfbase = reinterpret_cast<const float2*>(qbase + (size_t)overload * 3 * n);
-    const bool three = Launch<T>::assemble3_supported(n);
     for (int ish = 0; ish < overload; ++ish) {
-      if (three) {  // x pass of the three components in one launch
+      {  // x pass of the three components in one launch
         Assemble3XInvOp<T> op{};
         op.phitot = (const cplx<T>*)wsum;
         for (int d = 0; d < 3; ++d) {
@@ -936,84 +892,26 @@ int enqueue_impl(mf_ic* ic) {
         CK(Launch<T>::assemble3_xinv(n, op, n, Kz, twN, s));
       }
       for (int d = 0; d < 3; ++d) {
-        T* tmpr = (T*)ic->tmp[d]->d;
-        cplx<T>* tk = (cplx<T>*)tmpr;
-        AssembleXInvOp<T> op{};
-        op.phitot = (const cplx<T>*)wsum;
-        op.A3p = p.lpt_order > 2 ? (const cplx<T>*)ic->f[3 + (d + 1) % 3]->d : nullptr;
-        op.A3pp = p.lpt_order > 2 ? (const cplx<T>*)ic->f[3 + (d + 2) % 3]->d : nullptr;
-        op.dst = tk;
-        op.n = n;
-        op.Kz = Kz;
-        op.d = d;
-        op.ch = lattice_chain<T>(ic->phase, p.lattice, sp == 1, ish);
-        op.kfac = T(kfac);
-        op.wA = &ic->dyn_d->w[pass][3];
-        op.unit = T((vel ? p.vunit : p.lunit) / L);
-        op.plt = p.plt;
-        op.vel = vel ? 1 : 0;
-        if (p.plt) {
-          const size_t nkt = (size_t)ic->plt_ng * ic->plt_ng * (ic->plt_ng / 2 + 1);
-          const T* base = (const T*)ic->plt;
-          op.P.Dr = base;
-          op.P.Dth = base + nkt;
-          op.P.Dph = base + 2 * nkt;
-          op.P.Dvf = base + 3 * nkt;
-          op.P.ng = ic->plt_ng;
-          op.P.mapratio = T((double)ic->plt_ng / (double)n);
-          op.P.inv_mr_L = T(1.0 / ((double)ic->plt_ng / (double)n) / L);
-          op.pg = (const T*)ic->pltg;
-        }
-        if (!three) {
-          LaunchScope ls(c, KK_FFT_COL);
-          CK(Launch<T>::assemble_xinv(n, op, n, Kz, twN, s));
-        }
-        {
-          LaunchScope ls(c, KK_FFT_COL);
-          CK(Launch<T>::colfft_plain(n, true, PlainStridedOp<T>{tk, Kz, (long long)n * Kz, T(1)}, n, Kz, twN, s));
-        }
-        if (!three) {
-          LaunchScope ls(c, KK_FFT_Z);
-          const T norm = T(1.0 / std::sqrt((double)n * (double)n * (double)n));
-          CK(Launch<T>::z_c2r_plain(n / 2, PlainZOp<T>{tmpr, n, norm}, n * n, Kz, twH, twN, s));
-        }
+        cplx<T>* tk = (cplx<T>*)ic->tmp[d]->d;
+        LaunchScope ls(c, KK_FFT_COL);
+        CK(Launch<T>::colfft_plain(n, true, PlainStridedOp<T>{tk, Kz, (long long)n * Kz, T(1)}, n, Kz, twN, s));
       }
-      const double* qt = qbase + (size_t)ish * 3 * n;
-      if (three) {  // the three components' z passes with the lattice readout fused
-        Lattice3Args la{};
-        for (int d = 0; d < 3; ++d) la.comp[d] = ic->tmp[d]->d;
-        la.dst = dst;
-        la.q = qt;
-        la.qf = qfbase + (size_t)ish * 3 * n;
-        la.n = n;
-        la.nlines = n * n;
-        la.ishift = fields ? 0 : ish;
-        la.with_q = (!fields && !vel) ? 1 : 0;
-        la.fields_mode = fields ? 1 : 0;
-        la.norm = 1.0 / std::sqrt((double)n * (double)n * (double)n);
-        {
-          LaunchScope ls(c, KK_FFT_Z);
-          CK(Launch<T>::z_c2r3_lattice(n / 2, la, fields || p.pos64, twH, twN, s));
-        }
-        if (ic->early && !fields && MF_STREAM_HANDOFF) {
-          const size_t slice = (vel ? ic->vel_bytes : ic->pos_bytes) / overload;
-          CK(early_copy((char*)(vel ? ic->early->vel : ic->early->pos) + ish * slice, (const char*)dst + ish * slice,
-                        slice));
-        }
-        continue;
+      // the three components' z passes with the lattice readout fused
+      Lattice3Args la{};
+      for (int d = 0; d < 3; ++d) la.comp[d] = ic->tmp[d]->d;
+      la.dst = dst;
+      la.q = qbase + (size_t)ish * 3 * n;
+      la.qf = qfbase + (size_t)ish * 3 * n;
+      la.n = n;
+      la.nlines = n * n;
+      la.ishift = fields ? 0 : ish;
+      la.with_q = (!fields && !vel) ? 1 : 0;
+      la.fields_mode = fields ? 1 : 0;
+      la.norm = 1.0 / std::sqrt((double)n * (double)n * (double)n);
+      {
+        LaunchScope ls(c, KK_FFT_Z);
+        CK(Launch<T>::z_c2r3_lattice(n / 2, la, fields || p.pos64, twH, twN, s));
       }
-      const T* q0 = (const T*)ic->tmp[0]->d;
-      const T* q1 = (const T*)ic->tmp[1]->d;
-      const T* q2 = (const T*)ic->tmp[2]->d;
-      LaunchScope ls(c, KK_POINTWISE);
-      if (fields)
-        k_lattice3<T, double><<<blocks_for(n3), kThreads, 0, s>>>(q0, q1, q2, n, (double*)dst, 0, qt, 0, 1);
-      else if (p.pos64)
-        k_lattice3<T, double><<<blocks_for(n3), kThreads, 0, s>>>(q0, q1, q2, n, (double*)dst, ish, qt, vel ? 0 : 1, 0);
-      else
-        k_lattice3<T, float><<<blocks_for(n3), kThreads, 0, s>>>(q0, q1, q2, n, (float*)dst, ish, qt, vel ? 0 : 1, 0,
-                                                                 qfbase + (size_t)ish * 3 * n);
-      CK(cudaGetLastError());
       if (ic->early && !fields && MF_STREAM_HANDOFF) {
         const size_t slice = (vel ? ic->vel_bytes : ic->pos_bytes) / overload;
         CK(early_copy((char*)(vel ? ic->early->vel : ic->early->pos) + ish * slice, (const char*)dst + ish * slice,

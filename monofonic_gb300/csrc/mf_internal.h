@@ -56,10 +56,7 @@ struct Launch {
   // strided pass kinds
   static cudaError_t colfft_plain(int L, bool inv, PlainStridedOp<T> op, int nslab, int ncols,
                                   const cplx<T>* tw, cudaStream_t s);
-  static cudaError_t assemble_xinv(int L, AssembleXInvOp<T> op, int nslab, int ncols, const cplx<T>* tw,
-                                   cudaStream_t s);
-  // all three components in one launch (lengths whose plan keeps E <= 8)
-  static bool assemble3_supported(int L);
+  // x pass of the three displacement / velocity components in one launch
   static cudaError_t assemble3_xinv(int L, Assemble3XInvOp<T> op, int nslab, int ncols, const cplx<T>* tw,
                                     cudaStream_t s);
   // z c2r of the three components with the lattice readout fused (H = n/2);

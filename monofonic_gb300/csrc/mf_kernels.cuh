@@ -89,91 +89,9 @@ template <class OP>
 struct has_tile_prep<OP, std::void_t<decltype(&OP::tile_prep)>> : std::true_type {};
 
 // ---------------------------------------------------------------------------
-// strided column pass
-// ---------------------------------------------------------------------------
-// OP: __device__ C load(int slab, int e, int col) const;
-//     __device__ void store(int slab, int e, int col, C v) const;
-template <typename T, int L, bool INV, int NCOL, class OP>
-__global__ void __launch_bounds__(NCOL * LineFFT<T, L, INV>::TPL)
-k_colfft(OP op, const cplx<T>* __restrict__ tw, int ncols) {
-  using F = LineFFT<T, L, INV>;
-  using C = cplx<T>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* sm = reinterpret_cast<C*>(smem_raw);
-  const int c = threadIdx.x, t = threadIdx.y;
-  const int col = blockIdx.x * NCOL + c;
-  const int slab = blockIdx.y;
-  const bool valid = col < ncols;
-  if constexpr (sizeof(T) == 8) {
-#pragma unroll 1
-    for (int i = 0; i < F::E; ++i)
-      sm[tile_slot<F, NCOL>(t, i) + c] = valid ? op.load(slab, t + i * F::TPL, col) : mkc<T>(T(0), T(0));
-    const int xs = col_fx<F, NCOL>(sm, t, c, tw);
-    if (!valid) return;
-#pragma unroll 2
-    for (int i = 0; i < F::E; ++i)
-      op.store(slab, t + i * F::TPL, col,
-               fx::to_c(reinterpret_cast<const longlong2*>(sm)[tile_slot<F, NCOL>(t, i) + c], xs));
-    return;
-  }
-  C v[F::E];
-#pragma unroll
-  for (int s = 0; s < F::E; ++s) {
-    const int e = F::in_index(t, s);
-    v[s] = valid ? op.load(slab, e, col) : mkc<T>(T(0), T(0));
-  }
-  if constexpr (OP::kPrefetch) {
-    C pre[F::E];
-#pragma unroll
-    for (int s = 0; s < F::E; ++s) pre[s] = valid ? op.prefetch(slab, F::out_index(t, s), col) : mkc<T>(T(0), T(0));
-    F::run(v, t, sm + c, NCOL, tw, SyncBlock{});
-    if (valid) {
-#pragma unroll
-      for (int s = 0; s < F::E; ++s) op.store_pre(slab, F::out_index(t, s), col, v[s], pre[s]);
-    }
-  } else {
-    F::run(v, t, sm + c, NCOL, tw, SyncBlock{});
-    if (valid) {
-#pragma unroll
-      for (int s = 0; s < F::E; ++s) op.store(slab, F::out_index(t, s), col, v[s]);
-    }
-  }
-}
-
 // strided pass producing three transforms per column (three-component
-// assembly): the loader yields the three inputs of each element at once, the
-// three line FFTs run one after the other through the same shared tile
-template <typename T, int L, bool INV, int NCOL, class OP>
-__global__ void __launch_bounds__(NCOL * LineFFT<T, L, INV>::TPL)
-k_colfft3(OP op, const cplx<T>* __restrict__ tw, int ncols) {
-  using F = LineFFT<T, L, INV>;
-  using C = cplx<T>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* sm = reinterpret_cast<C*>(smem_raw);
-  const int c = threadIdx.x, t = threadIdx.y;
-  const int col = blockIdx.x * NCOL + c;
-  const int slab = blockIdx.y;
-  const bool valid = col < ncols;
-  C v[3][F::E];
-#pragma unroll
-  for (int s = 0; s < F::E; ++s) {
-    C w[3] = {mkc<T>(T(0), T(0)), mkc<T>(T(0), T(0)), mkc<T>(T(0), T(0))};
-    if (valid) op.load3(slab, F::in_index(t, s), col, w);
-    v[0][s] = w[0];
-    v[1][s] = w[1];
-    v[2][s] = w[2];
-  }
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    F::run(v[d], t, sm + c, NCOL, tw, SyncBlock{});
-    if (valid) {
-#pragma unroll
-      for (int s = 0; s < F::E; ++s) op.store(d, slab, F::out_index(t, s), col, v[d][s]);
-    }
-  }
-}
-
-// The same staged through shared memory: the first component stays in
+// assembly): the loader yields the three inputs of each element at once.
+// FP32: the first component stays in
 // registers, the other two go to their own tiles as they are loaded, and each
 // later component's transform runs from (and exchanges through) its tile, so
 // registers hold one component and two CTAs share an SM (one's loads overlap
@@ -250,7 +168,7 @@ k_colfft3s(OP op, const cplx<T>* __restrict__ tw, int ncols) {
 // copied into the other shared-memory buffer with cp.async.  Every thread
 // copies exactly the elements it reads for its first FFT stage, so a
 // per-thread wait_group suffices before the read.
-// OP: kPipe, srcp(z, slab, e, col) -> const C* (nullptr = zero),
+// OP: srcp(z, slab, e, col) -> const C* (nullptr = zero),
 //     xform(z, slab, e, col, raw), store_z(z, slab, e, col, v)
 //     (+ kPrefetch: prefetch/store_pre on the same coordinates)
 // ---------------------------------------------------------------------------
@@ -576,109 +494,104 @@ __global__ void __launch_bounds__(NT) k_zc2r(OP op, const cplx<T>* __restrict__ 
 // grids of doubles.  Inputs: the three component grids after their x and y
 // passes, [line][n/2+1] complex.
 // ---------------------------------------------------------------------------
-// the lattice readout of one transformed line (particle ip = ishift*n^3 + cell)
-template <typename T, int H, typename P>
-__device__ __forceinline__ void lattice_line_out(Lattice3Args a, int line, int t,
-                                                 const cplx<T> (&v)[3][LineFFT<T, H, true>::E]) {
-  using F = LineFFT<T, H, true>;
+// the lattice readout of cells 2m, 2m+1 of a transformed line (particle
+// ip = ishift*n^3 + cell), v the unnormalised component values
+template <typename T, typename P>
+__device__ __forceinline__ void lattice_out(const Lattice3Args& a, int line, int m, const cplx<T> (&v)[3]) {
   const int n = a.n;
   const long long n3 = (long long)n * n * n;
   const int i = line / n, j = line % n;
   if constexpr (std::is_same<P, float>::value && std::is_same<T, float>::value) {
     if (!a.fields_mode) {
-      // FP32 particles: the two particles 2m, 2m+1 of a slot are 24 contiguous
-      // bytes (8-byte aligned for even n), stored as three float2
+      // FP32 particles: the two particles are 24 contiguous bytes (8-byte
+      // aligned for even n), stored as three float2; positions q + Psi with q
+      // as a float pair: the correctly rounded sum on the FP32 pipes (ff_add_q)
+      float w[6];
 #pragma unroll
-      for (int s = 0; s < F::E; ++s) {
-        const int m = F::out_index(t, s);
-        float w[6];
+      for (int h = 0; h < 2; ++h) {
+        const int k = 2 * m + h;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int k = 2 * m + h;
-#pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            const float x = (h ? v[d][s].y : v[d][s].x) * T(a.norm);
-            const int qi = (d == 0) ? i : ((d == 1) ? n + j : 2 * n + k);
-            w[3 * h + d] = a.with_q ? ff_add_q(a.qf[qi], x) : x;
-          }
+        for (int d = 0; d < 3; ++d) {
+          const float x = (h ? v[d].y : v[d].x) * T(a.norm);
+          const int qi = (d == 0) ? i : ((d == 1) ? n + j : 2 * n + k);
+          w[3 * h + d] = a.with_q ? ff_add_q(a.qf[qi], x) : x;
         }
-        float2* o = reinterpret_cast<float2*>(reinterpret_cast<float*>(a.dst) +
-                                              3 * ((long long)a.ishift * n3 + (long long)line * n + 2 * m));
-        o[0] = make_float2(w[0], w[1]);
-        o[1] = make_float2(w[2], w[3]);
-        o[2] = make_float2(w[4], w[5]);
       }
+      float2* o = reinterpret_cast<float2*>(reinterpret_cast<float*>(a.dst) +
+                                            3 * ((long long)a.ishift * n3 + (long long)line * n + 2 * m));
+      o[0] = make_float2(w[0], w[1]);
+      o[1] = make_float2(w[2], w[3]);
+      o[2] = make_float2(w[4], w[5]);
       return;
     }
   }
 #pragma unroll
-  for (int s = 0; s < F::E; ++s) {
-    const int m = F::out_index(t, s);
+  for (int h = 0; h < 2; ++h) {
+    const int k = 2 * m + h;
+    const long long c = (long long)line * n + k;
+    if (std::is_same<P, T>::value && !a.with_q && !a.fields_mode) {
+      // velocities (no lattice coordinate) in the grid precision: no FP64 step
+      P* o = reinterpret_cast<P*>(a.dst) + 3 * ((long long)a.ishift * n3 + c);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int k = 2 * m + h;
-      const long long c = (long long)line * n + k;
-      if (std::is_same<P, T>::value && !a.with_q && !a.fields_mode) {
-        // velocities (no lattice coordinate) in the grid precision: no FP64 step
-        P* o = reinterpret_cast<P*>(a.dst) + 3 * ((long long)a.ishift * n3 + c);
+      for (int d = 0; d < 3; ++d) o[d] = (P)((h ? v[d].y : v[d].x) * T(a.norm));
+      continue;
+    }
+    double val[3];
+    // normalised in the grid precision, as the component grids of the per-component path
 #pragma unroll
-        for (int d = 0; d < 3; ++d) o[d] = (P)((h ? v[d][s].y : v[d][s].x) * T(a.norm));
-        continue;
+    for (int d = 0; d < 3; ++d) val[d] = (double)((h ? v[d].y : v[d].x) * T(a.norm));
+    if (a.fields_mode) {
+      double* o = reinterpret_cast<double*>(a.dst);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) o[d * n3 + c] = val[d];
+    } else {
+      if (a.with_q) {
+        val[0] += a.q[i];
+        val[1] += a.q[n + j];
+        val[2] += a.q[2 * n + k];
       }
-      if constexpr (std::is_same<P, float>::value && std::is_same<T, float>::value) {
-        if (a.with_q && !a.fields_mode) {
-          // FP32 positions q + Psi with q as a float pair: the correctly
-          // rounded sum on the FP32 pipes (ff_add_q)
-          P* o = reinterpret_cast<P*>(a.dst) + 3 * ((long long)a.ishift * n3 + c);
-          const int qi[3] = {i, n + j, 2 * n + k};
+      P* o = reinterpret_cast<P*>(a.dst) + 3 * ((long long)a.ishift * n3 + c);
 #pragma unroll
-          for (int d = 0; d < 3; ++d) o[d] = ff_add_q(a.qf[qi[d]], (h ? v[d][s].y : v[d][s].x) * T(a.norm));
-          continue;
-        }
-      }
-      double val[3];
-      // normalised in the grid precision, as the component grids of the per-component path
-#pragma unroll
-      for (int d = 0; d < 3; ++d) val[d] = (double)((h ? v[d][s].y : v[d][s].x) * T(a.norm));
-      if (a.fields_mode) {
-        double* o = reinterpret_cast<double*>(a.dst);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) o[d * n3 + c] = val[d];
-      } else {
-        if (a.with_q) {
-          val[0] += a.q[i];
-          val[1] += a.q[n + j];
-          val[2] += a.q[2 * n + k];
-        }
-        P* o = reinterpret_cast<P*>(a.dst) + 3 * ((long long)a.ishift * n3 + c);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) o[d] = (P)val[d];
-      }
+      for (int d = 0; d < 3; ++d) o[d] = (P)val[d];
     }
   }
 }
 
-
+// Whether the lattice z pass goes component by component through the staged
+// lines (one register set) instead of holding three: FP64, and lengths of more
+// than eight values per thread.  One staging buffer then, for the warps that
+// fit an SM by shared memory.
+template <typename T, int H>
+__host__ __device__ constexpr bool lattice_staged() {
+  return sizeof(T) == 8 || LineFFT<T, H, true>::E > 8;
+}
 template <typename T, int H, int LPB, typename P>
 __global__ void __launch_bounds__(LPB * LineFFT<T, H, true>::TPL, (LineFFT<T, H, true>::E <= 8) ? 2 : 1)
     k_zc2r3_lattice(Lattice3Args a, const cplx<T>* __restrict__ twH, const cplx<T>* __restrict__ twM) {
   // each line's exchanges run in its own staged region (XOR layout of the
   // contiguous-line passes), under warp barriers when a line's threads sit
-  // inside one warp
-  // (the identity layout where three components of E > 8 values already fill the registers)
-  using F = LineFFT<T, H, true, 8, (LineFFT<T, H, true>::E <= 8) ? zlayout(H) : 0>;
+  // inside one warp; the staged lines of a component are H+1 elements apart,
+  // so the line groups take lines TPL apart (zline_of_group).  The layout may
+  // not need more than H+1 elements.
+  constexpr int LAY = padded_len(H, zlayout(H)) <= H + 1 ? zlayout(H) : 0;
+  using F = LineFFT<T, H, true, 8, LAY>;
   using SYNC = typename std::conditional<(F::TPL <= 32 && 32 % F::TPL == 0 && (LPB * F::TPL) % 32 == 0), SyncWarp,
                                          SyncBlock>::type;
   using C = cplx<T>;
+  constexpr bool STAGED = lattice_staged<T, H>();
   constexpr int SL = 3 * (H + 1);  // complex values of one line's three components
-  // persistent CTAs over batches of LPB lines; the next batch is copied into
-  // the other shared-memory buffer (cp.async) while this one is transformed
+  // persistent CTAs over batches of LPB lines; in the unstaged form the next
+  // batch is copied into the other shared-memory buffer (cp.async) while this
+  // one is transformed
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf0 = reinterpret_cast<C*>(smem_raw);
-  C* buf1 = buf0 + LPB * SL;
-  const int t = threadIdx.x, ly = threadIdx.y;
-  const int tid = ly * F::TPL + t;
-  const int n = a.n, Kz = H + 1;
+  [[maybe_unused]] C* buf1 = buf0 + LPB * SL;
+  const int t = threadIdx.x, lg = threadIdx.y;
+  constexpr int WF = 128 / (int)sizeof(C);
+  int ly = lg;
+  if constexpr (zline_map_ok<F::TPL, WF>(LPB)) ly = zline_of_group<F::TPL, WF>(lg);
+  const int tid = lg * F::TPL + t;
+  const int Kz = H + 1;
   const int nb = (a.nlines + LPB - 1) / LPB;
   // a batch of one component is LPB consecutive lines, contiguous in global
   // memory: staged as [d][l][k] with 16-byte copies (an even LPB keeps both
@@ -695,47 +608,78 @@ __global__ void __launch_bounds__(LPB * LineFFT<T, H, true>::TPL, (LineFFT<T, H,
     }
     cp_async_commit();
   };
-  int bt = blockIdx.x;
-  if (bt < nb) issue(bt, buf0); else cp_async_commit();
-  for (int it = 0; bt < nb; bt += gridDim.x, ++it) {
-    C* cur = (it & 1) ? buf1 : buf0;
-    C* nxt = (it & 1) ? buf0 : buf1;
-    const int bn = bt + gridDim.x;
-    if (bn < nb) issue(bn, nxt); else cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();  // every thread's copies of this batch have landed
-    const int line = bt * LPB + ly;
-    const bool valid = line < a.nlines;
-    C* sm[3];
+  if constexpr (STAGED) {
+    for (int bt = blockIdx.x; bt < nb; bt += gridDim.x) {
+      issue(bt, buf0);
+      cp_async_wait<0>();
+      __syncthreads();  // every thread's copies of this batch have landed
+      [[maybe_unused]] int xs[3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) sm[d] = cur + d * LPB * Kz + ly * Kz;
-    C v[3][F::E];
-    if constexpr (sizeof(T) == 8) {
-      int xs[3];
-#pragma unroll
-      for (int d = 0; d < 3; ++d) xs[d] = c2r_line_to_fx<H, F::TPL>(sm[d], Kz, t, ly, SYNC{});
+      for (int d = 0; d < 3; ++d) {
+        C* sm = buf0 + d * LPB * Kz + ly * Kz;
+        if constexpr (sizeof(T) == 8) xs[d] = c2r_line_to_fx<H, F::TPL>(sm, Kz, t, lg, SYNC{});
+      }
 #pragma unroll 1
       for (int d = 0; d < 3; ++d) {
-        longlong2* sx = reinterpret_cast<longlong2*>(cur + d * LPB * Kz + ly * Kz);
-        c2r_line_fx<F, H>(sx, Kz, sx, t, twH, twM, SYNC{});
+        C* sm = buf0 + d * LPB * Kz + ly * Kz;
+        if constexpr (sizeof(T) == 8) {
+          longlong2* sx = reinterpret_cast<longlong2*>(sm);
+          c2r_line_fx<F, H>(sx, Kz, sx, t, twH, twM, SYNC{});
+        } else {
+          C v[F::E];
+#pragma unroll
+          for (int s = 0; s < F::E; ++s) v[s] = c2r_pre<T, H>(sm, F::in_index(t, s), twM);
+          F::run(v, t, sm, 1, twH, SYNC{});
+          SYNC{}();
+#pragma unroll
+          for (int s = 0; s < F::E; ++s) sm[F::out_slot(t, s)] = v[s];
+        }
       }
+      // every thread reads back the elements that it wrote
+#pragma unroll 2
+      for (int q = 0; q < F::E; ++q) {
+        const int m = t + q * F::TPL;
+        C v[3];
 #pragma unroll
-      for (int d = 0; d < 3; ++d)
+        for (int d = 0; d < 3; ++d) {
+          const C r = buf0[d * LPB * Kz + ly * Kz + pidx<LAY>(m)];
+          if constexpr (sizeof(T) == 8) v[d] = fx::to_c(reinterpret_cast<const longlong2&>(r), xs[d]);
+          else v[d] = r;
+        }
+        lattice_out<T, P>(a, bt * LPB + ly, m, v);
+      }
+      __syncthreads();  // the buffer is refilled by the next iteration's copies
+    }
+    return;
+  } else {
+    int bt = blockIdx.x;
+    if (bt < nb) issue(bt, buf0); else cp_async_commit();
+    for (int it = 0; bt < nb; bt += gridDim.x, ++it) {
+      C* cur = (it & 1) ? buf1 : buf0;
+      C* nxt = (it & 1) ? buf0 : buf1;
+      const int bn = bt + gridDim.x;
+      if (bn < nb) issue(bn, nxt); else cp_async_commit();
+      cp_async_wait<1>();
+      __syncthreads();  // every thread's copies of this batch have landed
+      C* sm[3];
 #pragma unroll
-        for (int s = 0; s < F::E; ++s)
-          v[d][s] = fx::to_c(reinterpret_cast<const longlong2*>(sm[d])[F::out_slot(t, s)], xs[d]);
-    } else {
+      for (int d = 0; d < 3; ++d) sm[d] = cur + d * LPB * Kz + ly * Kz;
+      C v[3][F::E];
 #pragma unroll
       for (int d = 0; d < 3; ++d)
 #pragma unroll
         for (int s = 0; s < F::E; ++s) v[d][s] = c2r_pre<T, H>(sm[d], F::in_index(t, s), twM);
 #pragma unroll
       for (int d = 0; d < 3; ++d) F::run(v[d], t, sm[d], 1, twH, SYNC{});
+#pragma unroll
+      for (int s = 0; s < F::E; ++s) {
+        const C w[3] = {v[0][s], v[1][s], v[2][s]};
+        lattice_out<T, P>(a, bt * LPB + ly, F::out_index(t, s), w);
+      }
+      __syncthreads();  // cur is refilled by the next iteration's copies
     }
-    if (valid) lattice_line_out<T, H, P>(a, line, t, v);
-    __syncthreads();  // cur is refilled by the next iteration's copies
+    cp_async_wait<0>();
   }
-  cp_async_wait<0>();
 }
 
 // ---------------------------------------------------------------------------

@@ -10,10 +10,6 @@
 #ifndef MF_ZCONV_MINB_F32
 #define MF_ZCONV_MINB_F32 2
 #endif
-// 1: persistent double-buffered (cp.async) strided passes (a build-time knob)
-#ifndef MF_COL_PIPE
-#define MF_COL_PIPE 1
-#endif
 // 1: TMA-pipelined fused z pass where the layout allows it (a build-time knob)
 #ifndef MF_ZCONV_TMA
 #define MF_ZCONV_TMA 1
@@ -83,39 +79,27 @@ constexpr int pipe_ncol() {
 
 template <typename T, int L, bool INV, class OP>
 cudaError_t launch_col(OP op, int nslab, int ncols, int nz, const cplx<T>* tw, cudaStream_t s, int kind) {
-  if constexpr (OP::kPipe && MF_COL_PIPE) {
-    constexpr int NC = pipe_ncol<T, L>();
-    constexpr int TPL = LineFFT<T, L, INV, MF_COL_MAXR>::TPL;
-    const size_t smem = (size_t)(fixed_point_lines<T, OP>() ? 1 : 2) * L * NC * sizeof(cplx<T>);
-    auto kern = k_colfft_pipe<T, L, INV, NC, OP>;
-    cudaError_t e = set_smem(kern, smem);
-    if (e != cudaSuccess) return e;
-    int per_sm = 0, nsm = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NC * TPL, smem);
-    if (e != cudaSuccess) return e;
-    const PassSched sc = sched_get(kind, L, (int)sizeof(T));
-    if (sc.occ > 0 && sc.occ < per_sm) per_sm = sc.occ;
-    if (per_sm < 1) per_sm = 1;
-    const int ntc = (ncols + NC - 1) / NC;
-    const int total = ntc * nslab * nz;
-    int grid = nsm * per_sm;
-    if (grid > total) grid = total;
-    dim3 block(NC, TPL);
-    kern<<<grid, block, smem, s>>>(op, tw, ncols, ntc, nslab, nz);
-    return cudaGetLastError();
-  } else {
-    constexpr int NC = col_ncol<T, L>();
-    constexpr int TPL = LineFFT<T, L, INV>::TPL;
-    const size_t smem = (size_t)L * NC * sizeof(cplx<T>);
-    auto kern = k_colfft<T, L, INV, NC, OP>;
-    cudaError_t e = set_smem(kern, smem);
-    if (e != cudaSuccess) return e;
-    dim3 block(NC, TPL), grid((ncols + NC - 1) / NC, nslab, nz);
-    kern<<<grid, block, smem, s>>>(op, tw, ncols);
-    return cudaGetLastError();
-  }
+  constexpr int NC = pipe_ncol<T, L>();
+  constexpr int TPL = LineFFT<T, L, INV, MF_COL_MAXR>::TPL;
+  const size_t smem = (size_t)(fixed_point_lines<T, OP>() ? 1 : 2) * L * NC * sizeof(cplx<T>);
+  auto kern = k_colfft_pipe<T, L, INV, NC, OP>;
+  cudaError_t e = set_smem(kern, smem);
+  if (e != cudaSuccess) return e;
+  int per_sm = 0, nsm = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NC * TPL, smem);
+  if (e != cudaSuccess) return e;
+  const PassSched sc = sched_get(kind, L, (int)sizeof(T));
+  if (sc.occ > 0 && sc.occ < per_sm) per_sm = sc.occ;
+  if (per_sm < 1) per_sm = 1;
+  const int ntc = (ncols + NC - 1) / NC;
+  const int total = ntc * nslab * nz;
+  int grid = nsm * per_sm;
+  if (grid > total) grid = total;
+  dim3 block(NC, TPL);
+  kern<<<grid, block, smem, s>>>(op, tw, ncols, ntc, nslab, nz);
+  return cudaGetLastError();
 }
 
 // N-grid lengths, and the convolution pass lengths that have a compile-time
@@ -312,47 +296,33 @@ cudaError_t Launch<T>::z_c2r_plain(int H, PlainZOp<T> op, int nlines, int kin, c
   switch (H) { MF_LEN_NH(CASE) default: return cudaErrorInvalidValue; }
 #undef CASE
 }
-template <typename T>
-cudaError_t Launch<T>::assemble_xinv(int L, AssembleXInvOp<T> op, int nslab, int ncols, const cplx<T>* tw,
-                                     cudaStream_t s) {
-#define CASE(LL) case LL: return launch_col<T, LL, true>(op, nslab, ncols, 1, tw, s, KK_FFT_COL);
-  switch (L) { MF_LEN_N(CASE) default: return cudaErrorInvalidValue; }
-#undef CASE
+// columns per CTA of the three-component assembly: at most 512 threads, and
+// where a thread holds more than eight values, three tiles of at most ~75 KB
+// (several CTAs per SM)
+template <typename T, int L>
+constexpr int col3_ncol() {
+  constexpr int tpl = LineFFT<T, L, true>::TPL;
+  int nc = col_ncol<T, L>();
+  while (nc > 1 && nc * tpl > 512) nc /= 2;
+  if (LineFFT<T, L, true>::E > 8)
+    while (nc > 32 / (int)(2 * sizeof(T)) && 3 * L * nc * (int)sizeof(cplx<T>) > 75 * 1024) nc /= 2;
+  return nc;
 }
 template <typename T, int L>
 cudaError_t launch_col3(Assemble3XInvOp<T> op, int nslab, int ncols, const cplx<T>* tw, cudaStream_t s) {
-  if constexpr (LineFFT<T, L, true>::E > 8) {
-    return cudaErrorInvalidValue;  // three register sets of E > 8 elements: per-component passes instead
-  } else {
-    // at most 512 threads, so that the three register sets fit without spilling
-    constexpr int TPL = LineFFT<T, L, true>::TPL;
-    constexpr int NC0 = col_ncol<T, L>();
-    constexpr int NC = (NC0 * TPL > 512) ? ((512 / TPL) > 0 ? 512 / TPL : 1) : NC0;
-    dim3 block(NC, TPL), grid((ncols + NC - 1) / NC, nslab, 1);
-    if (op.n == L && op.Kz == L / 2 + 1) {
-      // the grid as compile-time constants, components staged through shared
-      // memory (two CTAs per SM where three tiles fit twice)
-      const size_t smem = (size_t)3 * L * NC * sizeof(cplx<T>);
-      constexpr int MINB = (2 * 3 * L * NC * (int)sizeof(cplx<T>) <= 200 * 1024 && NC * TPL <= 512) ? 2 : 1;
-      auto kern = k_colfft3s<T, L, true, NC, Assemble3XInvOp<T, L>, MINB>;
-      cudaError_t e = set_smem(kern, smem);
-      if (e != cudaSuccess) return e;
-      kern<<<grid, block, smem, s>>>(op.template with_n<L>(), tw, ncols);
-      return cudaGetLastError();
-    }
-    const size_t smem = (size_t)L * NC * sizeof(cplx<T>);
-    auto kern = k_colfft3<T, L, true, NC, Assemble3XInvOp<T>>;
-    cudaError_t e = set_smem(kern, smem);
-    if (e != cudaSuccess) return e;
-    kern<<<grid, block, smem, s>>>(op, tw, ncols);
-    return cudaGetLastError();
-  }
-}
-template <typename T>
-bool Launch<T>::assemble3_supported(int L) {
-#define CASE(LL) case LL: return LineFFT<T, LL, true>::E <= 8;
-  switch (L) { MF_LEN_N(CASE) default: return false; }
-#undef CASE
+  if (op.n != L || op.Kz != L / 2 + 1) return cudaErrorInvalidValue;
+  // the grid as compile-time constants, components staged through shared
+  // memory (two CTAs per SM where three tiles fit twice)
+  constexpr int TPL = LineFFT<T, L, true>::TPL;
+  constexpr int NC = col3_ncol<T, L>();
+  const size_t smem = (size_t)3 * L * NC * sizeof(cplx<T>);
+  constexpr int MINB = (2 * 3 * L * NC * (int)sizeof(cplx<T>) <= 200 * 1024 && NC * TPL <= 512) ? 2 : 1;
+  auto kern = k_colfft3s<T, L, true, NC, Assemble3XInvOp<T, L>, MINB>;
+  cudaError_t e = set_smem(kern, smem);
+  if (e != cudaSuccess) return e;
+  dim3 block(NC, TPL), grid((ncols + NC - 1) / NC, nslab, 1);
+  kern<<<grid, block, smem, s>>>(op.template with_n<L>(), tw, ncols);
+  return cudaGetLastError();
 }
 template <typename T>
 cudaError_t Launch<T>::assemble3_xinv(int L, Assemble3XInvOp<T> op, int nslab, int ncols, const cplx<T>* tw,
@@ -364,20 +334,17 @@ cudaError_t Launch<T>::assemble3_xinv(int L, Assemble3XInvOp<T> op, int nslab, i
 template <typename T, int H>
 cudaError_t launch_zc2r3_lattice(const Lattice3Args& a, bool p64, const cplx<T>* twH, const cplx<T>* twM,
                                  cudaStream_t s) {
-  if constexpr (LineFFT<T, H, true>::E > 8) {
-    return cudaErrorInvalidValue;  // per-component passes there (assemble3_supported)
-  } else {
-  // lines per batch: at most 256 threads, two batch buffers within ~100 KB so
-  // that two CTAs share an SM
+  // lines per batch: at most 256 threads; unstaged, two batch buffers within
+  // ~100 KB so that two CTAs share an SM; staged, one buffer of at most ~76 KB
   constexpr int TPL = LineFFT<T, H, true>::TPL;
+  constexpr int NBUF = lattice_staged<T, H>() ? 1 : 2;
   constexpr int LPB = [] {
-    int l = 256 / TPL;
-    if (l < 1) l = 1;
-    while (l > 1 && 2 * (size_t)l * 3 * (H + 1) * sizeof(cplx<T>) > 100 * 1024) l /= 2;
+    int l = 2;
+    while (2 * l * TPL <= 256 && (size_t)NBUF * 2 * l * 3 * (H + 1) * sizeof(cplx<T>) <= (NBUF == 2 ? 100u : 76u) * 1024u) l *= 2;
     return l;
   }();
-  const size_t smem = (size_t)2 * LPB * 3 * (H + 1) * sizeof(cplx<T>);
-  if (a.nlines % LPB) return cudaErrorInvalidValue;  // whole batches (n^2 lines, n even)
+  const size_t smem = (size_t)NBUF * LPB * 3 * (H + 1) * sizeof(cplx<T>);
+  if (a.nlines % LPB) return cudaErrorInvalidValue;  // whole batches (n^2 lines, n a multiple of 16)
   const int nb = a.nlines / LPB;
   auto go = [&](auto kern) -> cudaError_t {
     cudaError_t e = set_smem(kern, smem);
@@ -392,7 +359,6 @@ cudaError_t launch_zc2r3_lattice(const Lattice3Args& a, bool p64, const cplx<T>*
     return cudaGetLastError();
   };
   return p64 ? go(k_zc2r3_lattice<T, H, LPB, double>) : go(k_zc2r3_lattice<T, H, LPB, float>);
-  }
 }
 template <typename T>
 cudaError_t Launch<T>::z_c2r3_lattice(int H, const Lattice3Args& a, bool p64, const cplx<T>* twH,
@@ -402,10 +368,8 @@ cudaError_t Launch<T>::z_c2r3_lattice(int H, const Lattice3Args& a, bool p64, co
 #undef CASE
 }
 template cudaError_t Launch<MF_T>::z_c2r3_lattice(int, const Lattice3Args&, bool, const cplx<MF_T>*, const cplx<MF_T>*, cudaStream_t);
-template bool Launch<MF_T>::assemble3_supported(int);
 template cudaError_t Launch<MF_T>::assemble3_xinv(int, Assemble3XInvOp<MF_T>, int, int, const cplx<MF_T>*, cudaStream_t);
 template cudaError_t Launch<MF_T>::colfft_plain(int, bool, PlainStridedOp<MF_T>, int, int, const cplx<MF_T>*, cudaStream_t);
-template cudaError_t Launch<MF_T>::assemble_xinv(int, AssembleXInvOp<MF_T>, int, int, const cplx<MF_T>*, cudaStream_t);
 template cudaError_t Launch<MF_T>::z_r2c_plain(int, PlainZOp<MF_T>, int, int, const cplx<MF_T>*, const cplx<MF_T>*, cudaStream_t);
 template cudaError_t Launch<MF_T>::z_c2r_plain(int, PlainZOp<MF_T>, int, int, const cplx<MF_T>*, const cplx<MF_T>*, cudaStream_t);
 #endif

@@ -46,24 +46,6 @@ struct Operand {
 
 __device__ __forceinline__ int sel3(int d, int i, int j, int k) { return d == 0 ? i : (d == 1 ? j : k); }
 
-// apply the operand's k-space factor to f at (i, j, kz)
-template <typename T>
-__device__ __forceinline__ cplx<T> operand_value(int kind, int d0, int d1, int d2, int d3, cplx<T> f, int i, int j,
-                                                int kz, int n, T kfac) {
-  if (kind == OPND_PLAIN) return f;
-  if (kind == OPND_GRAD) {
-    const T g = gradk<T>(sel3(d0, i, j, kz), n, kfac);
-    return mkc<T>(-g * f.y, g * f.x);
-  }
-  const T h1 = -(gradk<T>(sel3(d0, i, j, kz), n, kfac) * gradk<T>(sel3(d1, i, j, kz), n, kfac));
-  T h = h1;
-  if (kind != OPND_HESS) {
-    const T h2 = -(gradk<T>(sel3(d2, i, j, kz), n, kfac) * gradk<T>(sel3(d3, i, j, kz), n, kfac));
-    h = (kind == OPND_SUM) ? (h1 + h2) : (h1 - h2);
-  }
-  return mkc<T>(h * f.x, h * f.y);
-}
-
 struct ConvGeom {
   int N;       // unpadded size
   int M;       // padded size (3N/2, or N for the aliased convolver)
@@ -162,35 +144,12 @@ struct ConvXInvOp {
   __device__ __forceinline__ int dsel(int z) const {
     return z == 0 ? opnd[0].d[F] : (z == 1 ? opnd[1].d[F] : opnd[2].d[F]);
   }
-  __device__ __forceinline__ C load(int j, int x, int kz) const {
-    const int i = g.src_row(x);
-    if (i < 0) return mkc<T>(T(0), T(0));
-    const int z = blockIdx.z;
-    const C* f = z == 0 ? opnd[0].f : (z == 1 ? opnd[1].f : opnd[2].f);
-    const int kind = z == 0 ? opnd[0].kind : (z == 1 ? opnd[1].kind : opnd[2].kind);
-    const C v0 = f[((long long)i * g.N + j) * g.Kz + kz];
-    const C v = operand_value<T>(kind, dsel<0>(z), dsel<1>(z), dsel<2>(z), dsel<3>(z), v0, i, j, kz, g.N, kfac);
-    return mkc<T>(v.x * scale, v.y * scale);
-  }
-  __device__ __forceinline__ void store(int j, int x, int kz, C v) const {
-    const int z = blockIdx.z;
-    C* d = z == 0 ? dst[0] : (z == 1 ? dst[1] : dst[2]);
-    d[((long long)x * g.M + j) * g.Kz + kz] = v;
-  }
-  // pipelined form (k_colfft_pipe): raw source element and on-read transform; z = operand
-  static constexpr bool kPipe = true;
+  // raw source element and on-read transform; z = operand
   template <class I>
   __device__ __forceinline__ const C* srcp(int z, int j, I x, int kz) const {
     if (g.src_row(x) < 0) return nullptr;
     const C* f = z == 0 ? opnd[0].f : (z == 1 ? opnd[1].f : opnd[2].f);
     return f + ((long long)j * g.Kz + kz) + g.row_off(x, (long long)g.N * g.Kz);
-  }
-  template <class I>
-  __device__ __forceinline__ C xform(int z, int j, I x, int kz, C v0) const {
-    const int i = g.src_row(x);
-    const int kind = z == 0 ? opnd[0].kind : (z == 1 ? opnd[1].kind : opnd[2].kind);
-    const C v = operand_value<T>(kind, dsel<0>(z), dsel<1>(z), dsel<2>(z), dsel<3>(z), v0, i, j, kz, g.N, kfac);
-    return mkc<T>(v.x * scale, v.y * scale);
   }
   // per-tile form: along x only g_i varies, so the operand factor (times the
   // scale) is the polynomial c0 + c1 g_i + c2 g_i^2 with coefficients fixed
@@ -263,19 +222,6 @@ struct ConvYInvOp {
     return o;
   }
   static constexpr bool kColSwizzle = true;  // bank-conflict-free exchange rows (registers to spare)
-  __device__ __forceinline__ C load(int x, int y, int kz) const {
-    const int j = g.src_row(y);
-    if (j < 0) return mkc<T>(T(0), T(0));
-    const int z = blockIdx.z;
-    const C* s = z == 0 ? src[0] : (z == 1 ? src[1] : src[2]);
-    return s[((long long)x * g.M + j) * g.Kz + kz];
-  }
-  __device__ __forceinline__ void store(int x, int y, int kz, C v) const {
-    const int z = blockIdx.z;
-    C* d = z == 0 ? dst[0] : (z == 1 ? dst[1] : dst[2]);
-    d[((long long)x * g.M + y) * g.Kz + kz] = v;
-  }
-  static constexpr bool kPipe = true;
   template <class I>
   __device__ __forceinline__ const C* srcp(int z, int x, I y, int kz) const {
     if (g.src_row(y) < 0) return nullptr;
@@ -307,14 +253,6 @@ struct ConvYFwdOp {
     return o;
   }
   static constexpr bool kColSwizzle = true;  // bank-conflict-free exchange rows (registers to spare)
-  __device__ __forceinline__ C load(int x, int y, int kz) const {
-    return src[((long long)x * g.M + y) * g.Kz + kz];
-  }
-  __device__ __forceinline__ void store(int x, int y, int kz, C v) const {
-    const int j = g.kept_row(y);
-    if (j >= 0) dst[((long long)x * g.M + j) * g.Kz + kz] = v;
-  }
-  static constexpr bool kPipe = true;
   template <class I>
   __device__ __forceinline__ const C* srcp(int, int x, I y, int kz) const {
     return src + ((long long)x * g.M * g.Kz + kz) + idx_off(y, g.Kz);
@@ -355,9 +293,6 @@ struct ConvXFwdOp {
   // the read-modify-write target is fetched before the transform so its
   // latency overlaps the FFT
   static constexpr bool kPrefetch = true;
-  __device__ __forceinline__ C load(int j, int xx, int kz) const {
-    return src[((long long)xx * g.M + j) * g.Kz + kz];
-  }
   template <class I>
   __device__ __forceinline__ C prefetch(int j, I xx, int kz) const {
     if (g.kept_row(xx) < 0 || out_op == OUT_ASSIGN) return mkc<T>(T(0), T(0));
@@ -383,8 +318,6 @@ struct ConvXFwdOp {
     }
     target[idx] = r;
   }
-  __device__ __forceinline__ void store(int j, int xx, int kz, C v) const { store_pre(j, xx, kz, v, prefetch(j, xx, kz)); }
-  static constexpr bool kPipe = true;
   template <class I>
   __device__ __forceinline__ const C* srcp(int, int j, I xx, int kz) const {
     return src + ((long long)j * g.Kz + kz) + idx_off(xx, (long long)g.M * g.Kz);
@@ -442,79 +375,6 @@ struct ShiftChain {
       for (int d = 0; d < K; ++d) v[d] = cmul(v[d], ph);
     }
   }
-};
-
-// x pass of the c2r of one displacement / velocity component, with the
-// k-space assembly of ic_generator.cc:829-858 / :884-931 fused into the load:
-//   i g_d phitot + w_A (i g_d' A3[d''] - i g_d'' A3[d']), times unit/L, zero DC,
-// times the sub-lattice phase chain (ShiftChain).
-// slab = j, e = i, col = kz; in place on the destination grid.
-template <typename T>
-struct AssembleXInvOp {
-  using C = cplx<T>;
-  const C* phitot;  // growth-weighted order sum (FP64 sum stored in T)
-  const C* A3p;     // A3[d'] (nullptr below 3LPT)
-  const C* A3pp;    // A3[d'']
-  C* dst;
-  int n, Kz, d;
-  ShiftChain<T> ch;
-  T kfac, unit;
-  const double* wA;  // device scalar: weight of the A3 term (growth factor of this pass)
-  int plt;          // PLT corrected gradient (lattice_gradient, particle_plt.hh:551-573)
-  int vel;          // velocities: times the PLT growth-rate correction vfac_corr (:575-585)
-  PLTDev<T> P;
-  const T* pg;  // tabulated PLT gradient and vfac_corr [idx][4] (nullptr: evaluate from P)
-  static constexpr bool kPrefetch = false;
-  static constexpr bool kPipe = false;
-
-  // k-space combination at (i, j, kz) before any sub-lattice phase
-  __device__ __forceinline__ C assemble(int i, int j, int kz) const {
-    const long long idx = ((long long)i * n + j) * Kz + kz;
-    if (idx == 0) return mkc<T>(T(0), T(0));
-    const int dp = (d + 1) % 3, dpp = (d + 2) % 3;
-    T gd, gp, gpp, vc = T(1);
-    if (plt) {
-      T g[3];
-      if (pg) {
-        const T* q = pg + 4 * idx;
-        g[0] = q[0];
-        g[1] = q[1];
-        g[2] = q[2];
-        if (vel) vc = q[3];
-      } else {
-        plt_gradient<T>(P, i, j, kz, g, vel ? &vc : nullptr);
-      }
-      gd = (d == 0) ? g[0] : ((d == 1) ? g[1] : g[2]);
-      gp = (dp == 0) ? g[0] : ((dp == 1) ? g[1] : g[2]);
-      gpp = (dpp == 0) ? g[0] : ((dpp == 1) ? g[1] : g[2]);
-    } else {
-      gd = gradk<T>(sel3(d, i, j, kz), n, kfac);
-      gp = gradk<T>(sel3(dp, i, j, kz), n, kfac);
-      gpp = gradk<T>(sel3(dpp, i, j, kz), n, kfac);
-    }
-    const C P1 = phitot[idx];
-    T rr = -gd * P1.y, ri = gd * P1.x;
-    if (A3p) {
-      const C X1 = A3pp[idx], X2 = A3p[idx];
-      const T w = T(__ldg(wA));
-      rr += w * (-(gp * X1.y) + gpp * X2.y);
-      ri += w * (gp * X1.x - gpp * X2.x);
-    }
-    if (plt && vel) {
-      rr *= vc;
-      ri *= vc;
-    }
-    return mkc<T>(rr * unit, ri * unit);
-  }
-  __device__ __forceinline__ C load(int j, int i, int kz) const {
-    C v[1] = {assemble(i, j, kz)};
-    if (ch.nstep == 0) return v[0];
-    C vm[1] = {mkc<T>(T(0), T(0))};
-    if (kz == 0 || kz == (n >> 1)) vm[0] = assemble((n - i) % n, (n - j) % n, kz);
-    ch.template apply<1>(n, i, j, kz, v, vm);
-    return v[0];
-  }
-  __device__ __forceinline__ void store(int j, int i, int kz, C v) const { dst[((long long)i * n + j) * Kz + kz] = v; }
 };
 
 // convolve3's intermediate truncation on a work buffer, in place: the x pass
@@ -579,13 +439,6 @@ struct PlainStridedOp {
   PlainStridedOp<T, L2, AX2> with_axis() const {
     return PlainStridedOp<T, L2, AX2>{p, e_str, slab_str, scale};
   }
-  __device__ __forceinline__ C load(int slab, int e, int col) const {
-    return p[(long long)slab * ss() + (long long)e * es() + col];
-  }
-  __device__ __forceinline__ void store(int slab, int e, int col, C v) const {
-    p[(long long)slab * ss() + (long long)e * es() + col] = mkc<T>(v.x * scale, v.y * scale);
-  }
-  static constexpr bool kPipe = true;
   template <class I>
   __device__ __forceinline__ const C* srcp(int, int slab, I e, int col) const {
     return p + ((long long)slab * ss() + col) + idx_off(e, es());
@@ -632,10 +485,13 @@ struct PlainZButterflyOp : PlainZOp<double> {
 // is transformed to real space once and kept in HBM as lines of M reals,
 // stored as H = M/2 packed pairs [line][H], line = x*M + y.
 
-// the x pass of all three displacement / velocity components of one
-// sub-lattice in one launch: the same k-space combination and sub-lattice
-// phase chain as AssembleXInvOp, with the order sum, the three A3 fields and
-// the gradient read once per mode for the three components
+// x pass of the c2r of the three displacement / velocity components of one
+// sub-lattice, with the k-space assembly of ic_generator.cc:829-858 / :884-931
+// fused into the load: per component d
+//   i g_d phitot + w_A (i g_d' A3[d''] - i g_d'' A3[d']), times unit/L, zero DC,
+// times the sub-lattice phase chain (ShiftChain); the order sum, the three A3
+// fields and the gradient are read once per mode for the three components.
+// slab = j, e = i, col = kz
 template <typename T, int NN = 0>
 struct Assemble3XInvOp {
   using C = cplx<T>;
