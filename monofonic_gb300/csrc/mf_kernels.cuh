@@ -391,10 +391,17 @@ k_colfft_trunc(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int ns
 // OP: __device__ C load_pair(int line, int m) const;   // (x[2m], x[2m+1])
 //     __device__ void store(int line, int k, C v) const;  // k in [0, kout)
 // ---------------------------------------------------------------------------
+// distance between the lines' areas of the plain z passes: the exchange stride
+// of the XOR layouts, at least the H+1 values of a half-complex line
+template <int H>
+__host__ __device__ constexpr int zplain_stride() {
+  return zline_stride(H) > H + 1 ? zline_stride(H) : H + 1;
+}
 template <typename T, int H, int NT, class OP>
 __global__ void __launch_bounds__(NT) k_zr2c(OP op, const cplx<T>* __restrict__ twH,
                                                const cplx<T>* __restrict__ twM, int nlines, int kout) {
-  using F = LineFFT<T, H, false>;
+  constexpr int LAY = zlayout(H);
+  using F = LineFFT<T, H, false, 8, LAY>;
   using C = cplx<T>;
   // a line's shared-memory area is its own: warp barriers when its threads sit inside one warp
   using SYNC = typename std::conditional<(F::TPL <= 32 && 32 % F::TPL == 0 && NT % 32 == 0), SyncWarp, SyncBlock>::type;
@@ -402,7 +409,7 @@ __global__ void __launch_bounds__(NT) k_zr2c(OP op, const cplx<T>* __restrict__ 
   const int t = threadIdx.x, ly = threadIdx.y;
   const int line = blockIdx.x * blockDim.y + ly;
   const bool valid = line < nlines;
-  C* sm = reinterpret_cast<C*>(smem_raw) + ly * (H + 1);
+  C* sm = reinterpret_cast<C*>(smem_raw) + ly * zplain_stride<H>();
   if constexpr (fixed_point_lines<T, OP>()) {
 #pragma unroll 4
     for (int i = 0; i < F::E; ++i)
@@ -412,7 +419,7 @@ __global__ void __launch_bounds__(NT) k_zr2c(OP op, const cplx<T>* __restrict__ 
     r2c_line_fx<F, H, 0>(sx, sx, t, twH, SYNC{});
     if (valid) {
 #pragma unroll 2
-      for (int k = t; k < kout; k += F::TPL) op.store(line, k, r2c_line_out<H, 0>(sx, k, xs, twM));
+      for (int k = t; k < kout; k += F::TPL) op.store(line, k, r2c_line_out<H, LAY>(sx, k, xs, twM));
     }
     return;
   }
@@ -422,12 +429,12 @@ __global__ void __launch_bounds__(NT) k_zr2c(OP op, const cplx<T>* __restrict__ 
   F::run(v, t, sm, 1, twH, SYNC{});
   SYNC{}();
 #pragma unroll
-  for (int s = 0; s < F::E; ++s) sm[F::out_index(t, s)] = v[s];
+  for (int s = 0; s < F::E; ++s) sm[F::out_slot(t, s)] = v[s];
   SYNC{}();
   if (valid) {
     for (int k = t; k < kout; k += F::TPL) {
-      const C zk = sm[k % H];
-      const C zc = cconj(sm[(H - k) % H]);
+      const C zk = sm[pidx<LAY>(k == H ? 0 : k)];
+      const C zc = cconj(sm[pidx<LAY>(k == 0 || k == H ? 0 : H - k)]);
       const C E = mkc<T>(T(0.5) * (zk.x + zc.x), T(0.5) * (zk.y + zc.y));
       // O = (zk - zc) / (2i)
       const C O = mkc<T>(T(0.5) * (zk.y - zc.y), -T(0.5) * (zk.x - zc.x));
@@ -455,7 +462,7 @@ __device__ __forceinline__ cplx<T> c2r_pre(const cplx<T>* sm, int k, const cplx<
 template <typename T, int H, int NT, class OP>
 __global__ void __launch_bounds__(NT) k_zc2r(OP op, const cplx<T>* __restrict__ twH,
                                                const cplx<T>* __restrict__ twM, int nlines, int kin) {
-  using F = LineFFT<T, H, true>;
+  using F = LineFFT<T, H, true, 8, zlayout(H)>;
   using C = cplx<T>;
   // a line's shared-memory area is its own: warp barriers when its threads sit inside one warp
   using SYNC = typename std::conditional<(F::TPL <= 32 && 32 % F::TPL == 0 && NT % 32 == 0), SyncWarp, SyncBlock>::type;
@@ -463,7 +470,7 @@ __global__ void __launch_bounds__(NT) k_zc2r(OP op, const cplx<T>* __restrict__ 
   const int t = threadIdx.x, ly = threadIdx.y;
   const int line = blockIdx.x * blockDim.y + ly;
   const bool valid = line < nlines;
-  C* sm = reinterpret_cast<C*>(smem_raw) + ly * (H + 1);
+  C* sm = reinterpret_cast<C*>(smem_raw) + ly * zplain_stride<H>();
   for (int k = t; k <= H; k += F::TPL) sm[k] = (valid && k < kin) ? op.load(line, k) : mkc<T>(T(0), T(0));
   if constexpr (sizeof(T) == 8) {
     const int xs = c2r_line_to_fx<H, F::TPL>(sm, H + 1, t, ly, SYNC{});
@@ -471,7 +478,7 @@ __global__ void __launch_bounds__(NT) k_zc2r(OP op, const cplx<T>* __restrict__ 
     c2r_line_fx<F, H>(sx, H + 1, sx, t, twH, twM, SYNC{});
     if (valid) {
 #pragma unroll 2
-      for (int i = 0; i < F::E; ++i) op.store_pair(line, t + i * F::TPL, fx::to_c(sx[t + i * F::TPL], xs));
+      for (int i = 0; i < F::E; ++i) op.store_pair(line, t + i * F::TPL, fx::to_c(sx[pidx<F::kLayout>(t + i * F::TPL)], xs));
     }
     return;
   }

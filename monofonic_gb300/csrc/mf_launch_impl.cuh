@@ -142,9 +142,9 @@ cudaError_t with_plain_axis(const PlainStridedOp<T>& op, LAUNCH&& go) {
 
 template <typename T, int H, class OP>
 cudaError_t launch_zr2c(OP op, int nlines, int kout, const cplx<T>* twH, const cplx<T>* twM, cudaStream_t s) {
-  constexpr int LPB = z_lpb<T, H, H + 1>();
+  constexpr int LPB = z_lpb<T, H, zplain_stride<H>()>();
   constexpr int TPL = LineFFT<T, H, false>::TPL;
-  const size_t smem = (size_t)LPB * (H + 1) * sizeof(cplx<T>);
+  const size_t smem = (size_t)LPB * zplain_stride<H>() * sizeof(cplx<T>);
   auto kern = k_zr2c<T, H, TPL * LPB, OP>;
   cudaError_t e = set_smem(kern, smem);
   if (e != cudaSuccess) return e;
@@ -155,9 +155,9 @@ cudaError_t launch_zr2c(OP op, int nlines, int kout, const cplx<T>* twH, const c
 
 template <typename T, int H, class OP>
 cudaError_t launch_zc2r(OP op, int nlines, int kin, const cplx<T>* twH, const cplx<T>* twM, cudaStream_t s) {
-  constexpr int LPB = z_lpb<T, H, H + 1>();
+  constexpr int LPB = z_lpb<T, H, zplain_stride<H>()>();
   constexpr int TPL = LineFFT<T, H, true>::TPL;
-  const size_t smem = (size_t)LPB * (H + 1) * sizeof(cplx<T>);
+  const size_t smem = (size_t)LPB * zplain_stride<H>() * sizeof(cplx<T>);
   auto kern = k_zc2r<T, H, TPL * LPB, OP>;
   cudaError_t e = set_smem(kern, smem);
   if (e != cudaSuccess) return e;
