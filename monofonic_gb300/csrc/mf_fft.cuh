@@ -193,6 +193,74 @@ __device__ __forceinline__ void dft_pfa(cplx<T>* a) {
   }
 }
 
+// exp(-2 pi i m / 32) for m in [0, 32), from cos(pi j / 16)
+struct C32 {
+  static constexpr double q[9] = {1.0,
+                                  0.98078528040323044912618223613424,
+                                  0.92387953251128675612818318939679,
+                                  0.83146961230254523707878837761791,
+                                  0.70710678118654752440084436210485,
+                                  0.55557023301960222474283081394853,
+                                  0.38268343236508977172845998403040,
+                                  0.19509032201612826784828486847702,
+                                  0.0};
+  __host__ __device__ static constexpr double cs(int m) {  // cos(2 pi m / 32)
+    m &= 31;
+    if (m > 16) m = 32 - m;
+    return m <= 8 ? q[m] : -q[16 - m];
+  }
+  __host__ __device__ static constexpr double sn(int m) { return cs(m - 8); }
+};
+// a times exp(-+2 pi i M / 32)
+template <typename T, bool INV, int M>
+__device__ __forceinline__ cplx<T> mul_w32(cplx<T> a) {
+  constexpr int m = M & 31;
+  if constexpr (m == 0) return a;
+  else if constexpr (m == 8) return cmul_mi<INV>(a);
+  else if constexpr (m == 16) return mkc<T>(-a.x, -a.y);
+  else if constexpr (m == 24) return cmul_mi<!INV>(a);
+  else if constexpr (m % 8 == 4) {  // odd multiples of an eighth turn
+    constexpr T cx = T(C32::cs(m)), cy = T(INV ? C32::sn(m) : -C32::sn(m));
+    return mkc<T>(a.x * cx - a.y * cy, a.x * cy + a.y * cx);
+  } else {
+    constexpr T cx = T(C32::cs(m)), cy = T(INV ? C32::sn(m) : -C32::sn(m));
+    return cmul(a, mkc<T>(cx, cy));
+  }
+}
+// DFT of size R = R1 R2 in registers with the twiddles exp(-2 pi i n2 k1 / R)
+// as constants (R divides 32): input n = n1 R2 + n2, output k = k1 + R1 k2
+template <typename T, bool INV, int R1, int R2, int N2, int K1>
+__device__ __forceinline__ void dft_ct_tw(cplx<T> (&t)[R1 * R2]) {
+  if constexpr (N2 < R2) {
+    if constexpr (K1 < R1) {
+      t[N2 * R1 + K1] = mul_w32<T, INV, N2 * K1 * (32 / (R1 * R2))>(t[N2 * R1 + K1]);
+      dft_ct_tw<T, INV, R1, R2, N2, K1 + 1>(t);
+    } else {
+      dft_ct_tw<T, INV, R1, R2, N2 + 1, 1>(t);
+    }
+  }
+}
+template <typename T, bool INV, int R1, int R2>
+__device__ __forceinline__ void dft_ct(cplx<T>* a) {
+  cplx<T> t[R1 * R2];  // [n2][n1] -> [n2][k1]
+#pragma unroll
+  for (int n2 = 0; n2 < R2; ++n2) {
+#pragma unroll
+    for (int n1 = 0; n1 < R1; ++n1) t[n2 * R1 + n1] = a[n1 * R2 + n2];
+    dftR<T, INV, R1>(&t[n2 * R1]);
+  }
+  dft_ct_tw<T, INV, R1, R2, 1, 1>(t);
+#pragma unroll
+  for (int k1 = 0; k1 < R1; ++k1) {
+    cplx<T> s[R2];
+#pragma unroll
+    for (int n2 = 0; n2 < R2; ++n2) s[n2] = t[n2 * R1 + k1];
+    dftR<T, INV, R2>(s);
+#pragma unroll
+    for (int k2 = 0; k2 < R2; ++k2) a[k1 + R1 * k2] = s[k2];
+  }
+}
+
 template <typename T, bool INV, int R>
 __device__ __forceinline__ void dftR(cplx<T>* a) {
   if constexpr (R == 2) dft2<T, INV>(a);
@@ -201,6 +269,9 @@ __device__ __forceinline__ void dftR(cplx<T>* a) {
   else if constexpr (R == 8) dft8<T, INV>(a);
   else if constexpr (R == 6) dft_pfa<T, INV, 2, 3>(a);
   else if constexpr (R == 12) dft_pfa<T, INV, 4, 3>(a);
+  else if constexpr (R == 16) dft_ct<T, INV, 4, 4>(a);
+  else if constexpr (R == 24) dft_pfa<T, INV, 8, 3>(a);
+  else if constexpr (R == 32) dft_ct<T, INV, 8, 4>(a);
   else static_assert(R == 2, "unsupported radix");
 }
 
@@ -368,6 +439,13 @@ __host__ __device__ constexpr bool zline_map_ok(int lpb) {
   return TPL < W && W % TPL == 0 && lpb % W == 0;
 }
 
+// whether the z c2r of one operand indexes its exchanges as thread part plus
+// constant: below 192.  From there the slots computed one by one, which the
+// persistent loop keeps in registers, are faster: c2r at H = 384 72.3 against
+// 80.0 us, at 192 23.0 against 25.1 us (at 144 20.3 against 19.8, at 96 10.6
+// against 10.2; 73728, 36864, .. lines)
+__host__ __device__ constexpr bool zinv_split(int H) { return H < 192; }
+
 // Line FFT of length L in precision T, direction INV, radices up to MAXR;
 // LAYOUT selects the shared-memory exchange index (pidx).  HOIST: a stage
 // whose butterflies of one thread all share k = t mod LC (TPL a multiple of
@@ -375,7 +453,8 @@ __host__ __device__ constexpr bool zline_map_ok(int lpb) {
 // loads, but the twiddles stay live across the butterflies, so it is for
 // kernels with registers to spare (the strided passes at 128 registers
 // spill with it).
-template <typename T, int L, bool INV, int MAXR = 8, int LAYOUT = 0, bool HOIST = false>
+// SPLIT: exchange slots as thread part plus constant (pidx_split).
+template <typename T, int L, bool INV, int MAXR = 8, int LAYOUT = 0, bool HOIST = false, bool SPLIT = true>
 struct LineFFT {
   static_assert(plan_ok(L), "FFT length must be 2^a 3^b >= 4");
   using C = cplx<T>;
@@ -403,12 +482,15 @@ struct LineFFT {
   }
   __device__ static __forceinline__ int out_index(int t, int slot) { return t + out_const(slot); }
   static constexpr int TBITS = is_pow2(TPL) ? TPL - 1 : -1;  // bits of t (-1: any)
+  __device__ static __forceinline__ int slot_of(int r, int c, int rbits) {
+    return SPLIT ? pidx_split<LAYOUT>(r, c, rbits) : pidx<LAYOUT>(r + c);
+  }
   // shared-memory slots of the stage-0 inputs / last-stage outputs
   __device__ static __forceinline__ int in_slot(int t, int slot) {
-    return pidx_split<LAYOUT>(t, in_const(slot), TBITS);
+    return slot_of(t, in_const(slot), TBITS);
   }
   __device__ static __forceinline__ int out_slot(int t, int slot) {
-    return pidx_split<LAYOUT>(t, out_const(slot), TBITS);
+    return slot_of(t, out_const(slot), TBITS);
   }
 
   // k = b mod LC of butterfly b = t + m TPL, as (part of t) + constant of m
@@ -484,7 +566,7 @@ struct LineFFT {
         rbits = -1;
       }
 #pragma unroll
-      for (int q = 0; q < R; ++q) sm[pidx_split<LAYOUT>(r, c + q * LC, rbits) * cs] = v[m * R + q];
+      for (int q = 0; q < R; ++q) sm[slot_of(r, c + q * LC, rbits) * cs] = v[m * R + q];
     }
   }
 
@@ -496,7 +578,7 @@ struct LineFFT {
 #pragma unroll
     for (int m = 0; m < NB; ++m) {
 #pragma unroll
-      for (int p = 0; p < R; ++p) v[m * R + p] = sm[pidx_split<LAYOUT>(t, m * TPL + p * (L / R), TBITS) * cs];
+      for (int p = 0; p < R; ++p) v[m * R + p] = sm[slot_of(t, m * TPL + p * (L / R), TBITS) * cs];
     }
   }
 

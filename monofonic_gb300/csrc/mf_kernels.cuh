@@ -296,6 +296,231 @@ k_colfft_pipe(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nsl
 }
 
 // ---------------------------------------------------------------------------
+// Two-stage strided pass (FP32): a column of length L = R1 R2 as one radix-R1
+// and one radix-R2 butterfly with a single exchange between them, where the
+// radix-8 plans take three stages and two exchanges.  At those plans the
+// passes spent ~70% of the shared-memory pipe and half of the issue slots;
+// a stage less takes a quarter of the shared-memory accesses, two of the five
+// CTA barriers per tile and one set of twiddles away.
+//   stage 1: butterfly b in [0, R2) takes rows b + p R2, leaves q at row b R1 + q
+//   stage 2: butterfly k in [0, R1) takes rows k + p R1 (times w_L^(pk)),
+//            outputs row k + q R1
+// Threads are column-fastest, (b or k) = threadIdx.y; the stages use R2 and R1
+// of them (whole warps idle in the smaller one).  In the exchange the low row
+// bit is flipped by the parity of b, so that the two rows of a half-warp fall
+// on different banks.
+// ---------------------------------------------------------------------------
+// (measured per launch, before -> after: y c2r of an operand pair 22.1 -> 17.2
+// us at L = 192, 70.0 -> 52.1 at 288, 142 -> 121 at 384, of three operands 1176
+// -> 979 us at 768; N-grid passes 292 -> 229 us at 512.  L = 256 keeps its
+// radix-8 plan, eight values per thread: 36 us, 16 x 16 took 41.)
+__host__ __device__ constexpr int col2_r1(int L) {
+  switch (L) {
+    case 128: return 8;
+    case 144: return 12;
+    case 192: return 12;
+    case 288: return 12;
+    case 384: return 16;
+    case 512: return 16;
+    case 576: return 24;
+    case 768: return 24;
+    default: return 0;
+  }
+}
+template <int L>
+struct Col2 {
+  static constexpr int R1 = col2_r1(L), R2 = R1 ? L / R1 : 0;
+  static constexpr int TY = R1 > R2 ? R1 : R2;  // threads per column
+  static constexpr int RMAX = TY;
+};
+// resident CTAs per SM, from the registers that the larger butterfly needs
+__host__ __device__ constexpr int col2_minb(int threads, int rmax) {
+  const int need = rmax >= 32 ? 128 : (rmax >= 24 ? 104 : 80);
+  const int b = 65536 / (threads * need);
+  return b < 1 ? 1 : b;
+}
+template <int R1>
+__device__ __forceinline__ int col2_out(int b, int q) {  // row of output q of stage-1 butterfly b
+  const int f = b & 1;
+  return b * R1 + ((q & 1) ? q - f : q + f);
+}
+template <int R1>
+__device__ __forceinline__ int col2_in(int k, int p) {  // row of input p of stage-2 butterfly k
+  return p * R1 + ((p & 1) ? (k ^ 1) : k);
+}
+
+template <typename T, int L, bool INV, int NCOL, class OP>
+__global__ void __launch_bounds__(NCOL * Col2<L>::TY, col2_minb(NCOL * Col2<L>::TY, Col2<L>::RMAX))
+k_col2(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nslab, int nz) {
+  constexpr int R1 = Col2<L>::R1, R2 = Col2<L>::R2;
+  using C = cplx<T>;
+  using I1 = LineIdx<R2>;
+  using I2 = LineIdx<R1>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* buf0 = reinterpret_cast<C*>(smem_raw);
+  C* buf1 = buf0 + L * NCOL;
+  const int c = threadIdx.x, u = threadIdx.y;
+  const int total = ntc * nslab * nz;
+  auto issue = [&](const TilePos& p, C* buf) {
+    const int col = p.ct * NCOL + c;
+    if (R2 == Col2<L>::TY || u < R2) {
+#pragma unroll
+      for (int s = 0; s < R1; ++s) {
+        C* d = buf + (u + s * R2) * NCOL + c;
+        const C* g = (col < ncols) ? op.srcp(p.z, p.slab, I1{u, s * R2}, col) : nullptr;
+        if (g) cp_async8(d, g);
+        else *d = mkc<T>(T(0), T(0));
+      }
+    }
+    cp_async_commit();
+  };
+  int tl = blockIdx.x;
+  const TilePos step = TilePos::of(gridDim.x, ntc, nslab);
+  TilePos nx = TilePos::of(tl, ntc, nslab);
+  if (tl < total) issue(nx, buf0); else cp_async_commit();
+  for (int it = 0; tl < total; tl += gridDim.x, ++it) {
+    C* cur = (it & 1) ? buf1 : buf0;
+    C* nxt = (it & 1) ? buf0 : buf1;
+    const TilePos p = nx;
+    nx = p.next(step, ntc, nslab);
+    if (tl + (int)gridDim.x < total) issue(nx, nxt); else cp_async_commit();
+    cp_async_wait<1>();
+    const int col = p.ct * NCOL + c;
+    const bool act1 = R2 == Col2<L>::TY || u < R2, act2 = (R1 == Col2<L>::TY || u < R1) && col < ncols;
+    C v[R1];
+    if (act1) {
+      if constexpr (has_tile_prep<OP>::value) {
+        const auto tp = op.tile_prep(p.z, p.slab, col);
+#pragma unroll
+        for (int s = 0; s < R1; ++s) v[s] = op.xform_tile(tp, I1{u, s * R2}, cur[(u + s * R2) * NCOL + c]);
+      } else {
+#pragma unroll
+        for (int s = 0; s < R1; ++s) v[s] = op.xform(p.z, p.slab, I1{u, s * R2}, col, cur[(u + s * R2) * NCOL + c]);
+      }
+      dftR<T, INV, R1>(v);
+    }
+    __syncthreads();  // every input of the tile has been read
+    if (act1) {
+#pragma unroll
+      for (int q = 0; q < R1; ++q) cur[col2_out<R1>(u, q) * NCOL + c] = v[q];
+    }
+    __syncthreads();
+    if (act2) {
+      C w[R2];
+#pragma unroll
+      for (int s = 0; s < R2; ++s) w[s] = cur[col2_in<R1>(u, s) * NCOL + c];
+#pragma unroll
+      for (int s = 1; s < R2; ++s) w[s] = INV ? cmulc(w[s], tw[s * u]) : cmul(w[s], tw[s * u]);
+      dftR<T, INV, R2>(w);
+      if constexpr (OP::kPrefetch) {  // a read-modify-write target, eight values in flight
+#pragma unroll
+        for (int h = 0; h < R2; h += 8) {
+          C pre[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            if (h + q < R2) pre[q] = op.prefetch(p.slab, I2{u, (h + q) * R1}, col);
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            if (h + q < R2) op.store_pre(p.slab, I2{u, (h + q) * R1}, col, w[h + q], pre[q]);
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < R2; ++q) op.store_z(p.z, p.slab, I2{u, q * R1}, col, w[q]);
+      }
+    }
+    __syncthreads();  // cur is refilled by the next iteration's copies
+  }
+  cp_async_wait<0>();
+}
+
+// convolve3's truncation (ConvXTruncOp) in the two-stage form: the forward
+// transform's outputs of a thread, rows k + q R1, are the inputs of the
+// radix-R2 butterfly that starts the inverse transform (R2, then R1), so the
+// truncation and the turn happen in registers: two exchanges in all
+template <typename T, int L, int NCOL, class OP>
+__global__ void __launch_bounds__(NCOL * Col2<L>::TY, col2_minb(NCOL * Col2<L>::TY, Col2<L>::RMAX))
+k_col2_trunc(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nslab) {
+  constexpr int R1 = Col2<L>::R1, R2 = Col2<L>::R2, TY = Col2<L>::TY;
+  using C = cplx<T>;
+  using I1 = LineIdx<R2>;
+  using I2 = LineIdx<R1>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* buf0 = reinterpret_cast<C*>(smem_raw);
+  C* buf1 = buf0 + L * NCOL;
+  const int c = threadIdx.x, u = threadIdx.y;
+  const int total = ntc * nslab;
+  auto issue = [&](const TilePos& p, C* buf) {
+    const int col = p.ct * NCOL + c;
+    if (R2 == TY || u < R2) {
+#pragma unroll
+      for (int s = 0; s < R1; ++s) {
+        C* d = buf + (u + s * R2) * NCOL + c;
+        if (col < ncols) cp_async8(d, op.at(p.slab, I1{u, s * R2}, col));
+        else *d = mkc<T>(T(0), T(0));
+      }
+    }
+    cp_async_commit();
+  };
+  int tl = blockIdx.x;
+  const TilePos step = TilePos::of(gridDim.x, ntc, nslab);
+  TilePos nx = TilePos::of(tl, ntc, nslab);
+  if (tl < total) issue(nx, buf0); else cp_async_commit();
+  for (int it = 0; tl < total; tl += gridDim.x, ++it) {
+    C* cur = (it & 1) ? buf1 : buf0;
+    C* nxt = (it & 1) ? buf0 : buf1;
+    const TilePos p = nx;
+    nx = p.next(step, ntc, nslab);
+    if (tl + (int)gridDim.x < total) issue(nx, nxt); else cp_async_commit();
+    cp_async_wait<1>();
+    const int col = p.ct * NCOL + c;
+    const bool act1 = R2 == TY || u < R2, act2 = R1 == TY || u < R1;
+    {
+      C v[R1];
+      if (act1) {
+#pragma unroll
+        for (int s = 0; s < R1; ++s) v[s] = cur[(u + s * R2) * NCOL + c];
+        dftR<T, false, R1>(v);
+      }
+      __syncthreads();
+      if (act1) {
+#pragma unroll
+        for (int q = 0; q < R1; ++q) cur[col2_out<R1>(u, q) * NCOL + c] = v[q];
+      }
+    }
+    __syncthreads();
+    C v[R2];
+    if (act2) {
+#pragma unroll
+      for (int s = 0; s < R2; ++s) v[s] = cur[col2_in<R1>(u, s) * NCOL + c];
+#pragma unroll
+      for (int s = 1; s < R2; ++s) v[s] = cmul(v[s], tw[s * u]);
+      dftR<T, false, R2>(v);
+#pragma unroll
+      for (int q = 0; q < R2; ++q) v[q] = op.mask(p.slab, I2{u, q * R1}, col, v[q]);
+      dftR<T, true, R2>(v);
+    }
+    __syncthreads();  // every input of the second stage has been read
+    if (act2) {
+#pragma unroll
+      for (int q = 0; q < R2; ++q) cur[col2_out<R2>(u, q) * NCOL + c] = v[q];
+    }
+    __syncthreads();
+    if (act1 && col < ncols) {
+      C w[R1];
+#pragma unroll
+      for (int s = 0; s < R1; ++s) w[s] = cur[col2_in<R2>(u, s) * NCOL + c];
+#pragma unroll
+      for (int s = 1; s < R1; ++s) w[s] = cmulc(w[s], tw[s * u]);
+      dftR<T, true, R1>(w);
+#pragma unroll
+      for (int q = 0; q < R1; ++q) *op.at(p.slab, I1{u, q * R2}, col) = w[q];
+    }
+    __syncthreads();  // cur is refilled by the next iteration's copies
+  }
+  cp_async_wait<0>();
+}
+
+// ---------------------------------------------------------------------------
 // strided forward transform, truncation and inverse transform of one column in
 // one pass (ConvXTruncOp), persistent and double-buffered as k_colfft_pipe
 // ---------------------------------------------------------------------------
@@ -848,7 +1073,7 @@ __global__ void __launch_bounds__(LPB * LineFFT<T, H, true, MAXR>::TPL,
                                   zconv_tma_minb<T, MODE>(LPB * LineFFT<T, H, true, MAXR>::TPL))
 k_zconv_tma(ZConvArgs<T> a, const cplx<T>* __restrict__ twH, const cplx<T>* __restrict__ twM) {
   constexpr int LAY = zlayout(H);
-  using FI = LineFFT<T, H, true, MAXR, LAY, true>;
+  using FI = LineFFT<T, H, true, MAXR, LAY, true, sizeof(T) == 8 || MODE != 1 || zinv_split(H)>;
   using FF = LineFFT<T, H, false, MAXR, LAY, true>;
   using C = cplx<T>;
   constexpr int E = FI::E, TPL = FI::TPL;

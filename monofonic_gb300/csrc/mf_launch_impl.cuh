@@ -77,29 +77,44 @@ constexpr int pipe_ncol() {
   return nc;
 }
 
-template <typename T, int L, bool INV, class OP>
-cudaError_t launch_col(OP op, int nslab, int ncols, int nz, const cplx<T>* tw, cudaStream_t s, int kind) {
-  constexpr int NC = pipe_ncol<T, L>();
-  constexpr int TPL = LineFFT<T, L, INV, MF_COL_MAXR>::TPL;
-  const size_t smem = (size_t)(fixed_point_lines<T, OP>() ? 1 : 2) * L * NC * sizeof(cplx<T>);
-  auto kern = k_colfft_pipe<T, L, INV, NC, OP>;
+// whether a strided pass takes the two-stage kernels
+template <typename T, int L>
+constexpr bool two_stage() { return sizeof(T) == 4 && col2_r1(L) > 0; }
+constexpr int kCol2Cols = 8;  // 64-byte rows
+
+// a persistent strided pass: as many CTAs as fit, or the tuned number per SM
+template <class KERN, typename... ARGS>
+cudaError_t launch_tiles(KERN kern, dim3 block, size_t smem, int occ, int total, cudaStream_t s, ARGS... args) {
   cudaError_t e = set_smem(kern, smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0, nsm = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NC * TPL, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)(block.x * block.y), smem);
   if (e != cudaSuccess) return e;
-  const PassSched sc = sched_get(kind, L, (int)sizeof(T));
-  if (sc.occ > 0 && sc.occ < per_sm) per_sm = sc.occ;
+  if (occ > 0 && occ < per_sm) per_sm = occ;
   if (per_sm < 1) per_sm = 1;
-  const int ntc = (ncols + NC - 1) / NC;
-  const int total = ntc * nslab * nz;
   int grid = nsm * per_sm;
   if (grid > total) grid = total;
-  dim3 block(NC, TPL);
-  kern<<<grid, block, smem, s>>>(op, tw, ncols, ntc, nslab, nz);
+  kern<<<grid, block, smem, s>>>(args...);
   return cudaGetLastError();
+}
+
+template <typename T, int L, bool INV, class OP>
+cudaError_t launch_col(OP op, int nslab, int ncols, int nz, const cplx<T>* tw, cudaStream_t s, int kind) {
+  const int occ = sched_get(kind, L, (int)sizeof(T)).occ;
+  if constexpr (two_stage<T, L>()) {
+    constexpr int NC = kCol2Cols;
+    const int ntc = (ncols + NC - 1) / NC;
+    return launch_tiles(k_col2<T, L, INV, NC, OP>, dim3(NC, Col2<L>::TY), (size_t)2 * L * NC * sizeof(cplx<T>), occ,
+                        ntc * nslab * nz, s, op, tw, ncols, ntc, nslab, nz);
+  } else {
+    constexpr int NC = pipe_ncol<T, L>();
+    const int ntc = (ncols + NC - 1) / NC;
+    return launch_tiles(k_colfft_pipe<T, L, INV, NC, OP>, dim3(NC, LineFFT<T, L, INV, MF_COL_MAXR>::TPL),
+                        (size_t)(fixed_point_lines<T, OP>() ? 1 : 2) * L * NC * sizeof(cplx<T>), occ, ntc * nslab * nz, s,
+                        op, tw, ncols, ntc, nslab, nz);
+  }
 }
 
 // N-grid lengths, and the convolution pass lengths that have a compile-time
@@ -412,24 +427,18 @@ cudaError_t Launch<T>::conv_xfwd(int L, ConvXFwdOp<T> op, int nslab, int ncols, 
 }
 template <typename T, int L, class OP>
 cudaError_t launch_xtrunc(OP op, int nslab, int ncols, const cplx<T>* tw, cudaStream_t s) {
-  constexpr int NC = pipe_ncol<T, L>();
-  constexpr int TPL = LineFFT<T, L, false, MF_COL_MAXR>::TPL;
-  const size_t smem = (size_t)(sizeof(T) == 8 ? 1 : 2) * L * NC * sizeof(cplx<T>);
-  auto kern = k_colfft_trunc<T, L, NC, OP>;
-  cudaError_t e = set_smem(kern, smem);
-  if (e != cudaSuccess) return e;
-  int per_sm = 0, nsm = 0, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NC * TPL, smem);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
-  const int ntc = (ncols + NC - 1) / NC;
-  const int total = ntc * nslab;
-  int grid = nsm * per_sm;
-  if (grid > total) grid = total;
-  kern<<<grid, dim3(NC, TPL), smem, s>>>(op, tw, ncols, ntc, nslab);
-  return cudaGetLastError();
+  if constexpr (two_stage<T, L>()) {
+    constexpr int NC = kCol2Cols;
+    const int ntc = (ncols + NC - 1) / NC;
+    return launch_tiles(k_col2_trunc<T, L, NC, OP>, dim3(NC, Col2<L>::TY), (size_t)2 * L * NC * sizeof(cplx<T>), 0,
+                        ntc * nslab, s, op, tw, ncols, ntc, nslab);
+  } else {
+    constexpr int NC = pipe_ncol<T, L>();
+    const int ntc = (ncols + NC - 1) / NC;
+    return launch_tiles(k_colfft_trunc<T, L, NC, OP>, dim3(NC, LineFFT<T, L, false, MF_COL_MAXR>::TPL),
+                        (size_t)(sizeof(T) == 8 ? 1 : 2) * L * NC * sizeof(cplx<T>), 0, ntc * nslab, s, op, tw, ncols, ntc,
+                        nslab);
+  }
 }
 template <typename T>
 cudaError_t Launch<T>::conv_xtrunc(int L, ConvXTruncOp<T> op, int nslab, int ncols, const cplx<T>* tw,
