@@ -168,7 +168,8 @@ k_colfft3s(OP op, const cplx<T>* __restrict__ tw, int ncols) {
 // copied into the other shared-memory buffer with cp.async.  Every thread
 // copies exactly the elements it reads for its first FFT stage, so a
 // per-thread wait_group suffices before the read.
-// OP: srcp(z, slab, e, col) -> const C* (nullptr = zero),
+// OP: src_ok(e) (else the element is zero), gap(e) (zero for every thread,
+//     known at compile time), srcp(z, slab, e, col) -> const C*,
 //     xform(z, slab, e, col, raw), store_z(z, slab, e, col, v)
 //     (+ kPrefetch: prefetch/store_pre on the same coordinates)
 // ---------------------------------------------------------------------------
@@ -212,8 +213,9 @@ k_colfft_pipe(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nsl
 #pragma unroll
     for (int s = 0; s < F::E; ++s) {
       C* d = buf + F::in_slot(t, s) * NCOL + c;
-      const C* g = (col < ncols) ? op.srcp(p.z, p.slab, I{t, F::in_const(s)}, col) : nullptr;
-      if (g) {
+      const I e{t, F::in_const(s)};
+      if (col < ncols && op.src_ok(e)) {
+        const C* g = op.srcp(p.z, p.slab, e, col);
         if constexpr (sizeof(C) == 16) cp_async16(d, g); else cp_async8(d, g);
       } else {
         *d = mkc<T>(T(0), T(0));
@@ -300,7 +302,7 @@ k_colfft_pipe(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nsl
 // and one radix-R2 butterfly with a single exchange between them, where the
 // radix-8 plans take three stages and two exchanges.  At those plans the
 // passes spent ~70% of the shared-memory pipe and half of the issue slots;
-// a stage less takes a quarter of the shared-memory accesses, two of the five
+// a stage less takes a quarter of the shared-memory accesses, three of the five
 // CTA barriers per tile and one set of twiddles away.
 //   stage 1: butterfly b in [0, R2) takes rows b + p R2, leaves q at row b R1 + q
 //   stage 2: butterfly k in [0, R1) takes rows k + p R1 (times w_L^(pk)),
@@ -366,9 +368,10 @@ k_col2(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nslab, int
     if (R2 == Col2<L>::TY || u < R2) {
 #pragma unroll
       for (int s = 0; s < R1; ++s) {
+        const I1 e{u, s * R2};
+        if (op.gap(e)) continue;  // neither staged nor read
         C* d = buf + (u + s * R2) * NCOL + c;
-        const C* g = (col < ncols) ? op.srcp(p.z, p.slab, I1{u, s * R2}, col) : nullptr;
-        if (g) cp_async8(d, g);
+        if (col < ncols && op.src_ok(e)) cp_async8(d, op.srcp(p.z, p.slab, e, col));
         else *d = mkc<T>(T(0), T(0));
       }
     }
@@ -377,7 +380,7 @@ k_col2(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nslab, int
   int tl = blockIdx.x;
   const TilePos step = TilePos::of(gridDim.x, ntc, nslab);
   TilePos nx = TilePos::of(tl, ntc, nslab);
-  if (tl < total) issue(nx, buf0); else cp_async_commit();
+  if (tl < total) issue(nx, buf0);
   for (int it = 0; tl < total; tl += gridDim.x, ++it) {
     C* cur = (it & 1) ? buf1 : buf0;
     C* nxt = (it & 1) ? buf0 : buf1;
@@ -392,10 +395,14 @@ k_col2(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nslab, int
       if constexpr (has_tile_prep<OP>::value) {
         const auto tp = op.tile_prep(p.z, p.slab, col);
 #pragma unroll
-        for (int s = 0; s < R1; ++s) v[s] = op.xform_tile(tp, I1{u, s * R2}, cur[(u + s * R2) * NCOL + c]);
+        for (int s = 0; s < R1; ++s)
+          v[s] = op.gap(I1{u, s * R2}) ? mkc<T>(T(0), T(0))
+                                       : op.xform_tile(tp, I1{u, s * R2}, cur[(u + s * R2) * NCOL + c]);
       } else {
 #pragma unroll
-        for (int s = 0; s < R1; ++s) v[s] = op.xform(p.z, p.slab, I1{u, s * R2}, col, cur[(u + s * R2) * NCOL + c]);
+        for (int s = 0; s < R1; ++s)
+          v[s] = op.gap(I1{u, s * R2}) ? mkc<T>(T(0), T(0))
+                                       : op.xform(p.z, p.slab, I1{u, s * R2}, col, cur[(u + s * R2) * NCOL + c]);
       }
       dftR<T, INV, R1>(v);
     }
@@ -430,7 +437,6 @@ k_col2(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nslab, int
     }
     __syncthreads();  // cur is refilled by the next iteration's copies
   }
-  cp_async_wait<0>();
 }
 
 // convolve3's truncation (ConvXTruncOp) in the two-stage form: the forward
@@ -464,14 +470,13 @@ k_col2_trunc(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nsla
   int tl = blockIdx.x;
   const TilePos step = TilePos::of(gridDim.x, ntc, nslab);
   TilePos nx = TilePos::of(tl, ntc, nslab);
-  if (tl < total) issue(nx, buf0); else cp_async_commit();
+  if (tl < total) issue(nx, buf0);
   for (int it = 0; tl < total; tl += gridDim.x, ++it) {
     C* cur = (it & 1) ? buf1 : buf0;
     C* nxt = (it & 1) ? buf0 : buf1;
     const TilePos p = nx;
     nx = p.next(step, ntc, nslab);
-    if (tl + (int)gridDim.x < total) issue(nx, nxt); else cp_async_commit();
-    cp_async_wait<1>();
+    cp_async_wait<0>();
     const int col = p.ct * NCOL + c;
     const bool act1 = R2 == TY || u < R2, act2 = R1 == TY || u < R1;
     {
@@ -481,7 +486,8 @@ k_col2_trunc(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nsla
         for (int s = 0; s < R1; ++s) v[s] = cur[(u + s * R2) * NCOL + c];
         dftR<T, false, R1>(v);
       }
-      __syncthreads();
+      __syncthreads();  // (as in k_col2)
+      if (tl + (int)gridDim.x < total) issue(nx, nxt);
       if (act1) {
 #pragma unroll
         for (int q = 0; q < R1; ++q) cur[col2_out<R1>(u, q) * NCOL + c] = v[q];
@@ -515,9 +521,7 @@ k_col2_trunc(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nsla
 #pragma unroll
       for (int q = 0; q < R1; ++q) *op.at(p.slab, I1{u, q * R2}, col) = w[q];
     }
-    __syncthreads();  // cur is refilled by the next iteration's copies
   }
-  cp_async_wait<0>();
 }
 
 // ---------------------------------------------------------------------------

@@ -103,6 +103,25 @@ struct CGeom {
   }
   template <int TPL>
   __device__ __forceinline__ static int kept_row(LineIdx<TPL> x) { return src_row(x); }
+  // whether the whole range of x lies in the zero gap (decided at compile time)
+  template <int TPL>
+  __device__ __forceinline__ static bool gap(LineIdx<TPL> x) {
+    return ORSZAG && x.c > (N >> 1) && x.c + TPL - 1 <= N;
+  }
+  // gradient component (over kfac) of the source row of x: x below the gap,
+  // x - M above it, zero on the Nyquist row N/2
+  template <typename T, int TPL>
+  __device__ __forceinline__ static T row_comp(LineIdx<TPL> x) {
+    const T v = T(x.t) + T(x.c - (x.c > (N >> 1) ? M : 0));  // exact
+    if (x.c > (N >> 1) || x.c + TPL - 1 < (N >> 1)) return v;
+    const int i = src_row(x.t + x.c);
+    return T(i == (N >> 1) ? 0 : i - (i > (N >> 1) ? N : 0));
+  }
+  template <typename T>
+  __device__ __forceinline__ static T row_comp(int x) {
+    const int i = src_row(x);
+    return T(i == (N >> 1) ? 0 : i - (i > (N >> 1) ? N : 0));
+  }
   // x * stride, and the kept row of x * stride, the constant part apart
   template <int TPL>
   __device__ __forceinline__ static long long row_off(LineIdx<TPL> x, long long stride) {
@@ -145,9 +164,13 @@ struct ConvXInvOp {
     return z == 0 ? opnd[0].d[F] : (z == 1 ? opnd[1].d[F] : opnd[2].d[F]);
   }
   // raw source element and on-read transform; z = operand
+  // whether element x has a source row; whether it has none for all threads
+  template <class I>
+  __device__ __forceinline__ bool src_ok(I x) const { return g.src_row(x) >= 0; }
+  template <class I>
+  __device__ __forceinline__ bool gap(I x) const { return g.gap(x); }
   template <class I>
   __device__ __forceinline__ const C* srcp(int z, int j, I x, int kz) const {
-    if (g.src_row(x) < 0) return nullptr;
     const C* f = z == 0 ? opnd[0].f : (z == 1 ? opnd[1].f : opnd[2].f);
     return f + ((long long)j * g.Kz + kz) + g.row_off(x, (long long)g.N * g.Kz);
   }
@@ -189,7 +212,7 @@ struct ConvXInvOp {
   }
   template <class I>
   __device__ __forceinline__ C xform_tile(const Tile& t, I x, C v0) const {
-    const T gi = gradk<T>(g.src_row(x), g.N, kfac);
+    const T gi = G::template row_comp<T>(x) * kfac;
     if (t.grad) {
       const T f = t.c1 * gi + t.c0;
       return mkc<T>(-f * v0.y, f * v0.x);
@@ -223,8 +246,11 @@ struct ConvYInvOp {
   }
   static constexpr bool kColSwizzle = true;  // bank-conflict-free exchange rows (registers to spare)
   template <class I>
+  __device__ __forceinline__ bool src_ok(I y) const { return g.src_row(y) >= 0; }
+  template <class I>
+  __device__ __forceinline__ bool gap(I y) const { return g.gap(y); }
+  template <class I>
   __device__ __forceinline__ const C* srcp(int z, int x, I y, int kz) const {
-    if (g.src_row(y) < 0) return nullptr;
     const C* s0 = z == 0 ? src[0] : (z == 1 ? src[1] : src[2]);
     return s0 + ((long long)x * g.M * g.Kz + kz) + g.row_off(y, g.Kz);
   }
@@ -253,6 +279,10 @@ struct ConvYFwdOp {
     return o;
   }
   static constexpr bool kColSwizzle = true;  // bank-conflict-free exchange rows (registers to spare)
+  template <class I>
+  __device__ __forceinline__ bool src_ok(I) const { return true; }
+  template <class I>
+  __device__ __forceinline__ bool gap(I) const { return false; }
   template <class I>
   __device__ __forceinline__ const C* srcp(int, int x, I y, int kz) const {
     return src + ((long long)x * g.M * g.Kz + kz) + idx_off(y, g.Kz);
@@ -318,6 +348,10 @@ struct ConvXFwdOp {
     }
     target[idx] = r;
   }
+  template <class I>
+  __device__ __forceinline__ bool src_ok(I) const { return true; }
+  template <class I>
+  __device__ __forceinline__ bool gap(I) const { return false; }
   template <class I>
   __device__ __forceinline__ const C* srcp(int, int j, I xx, int kz) const {
     return src + ((long long)j * g.Kz + kz) + idx_off(xx, (long long)g.M * g.Kz);
@@ -439,6 +473,10 @@ struct PlainStridedOp {
   PlainStridedOp<T, L2, AX2> with_axis() const {
     return PlainStridedOp<T, L2, AX2>{p, e_str, slab_str, scale};
   }
+  template <class I>
+  __device__ __forceinline__ bool src_ok(I) const { return true; }
+  template <class I>
+  __device__ __forceinline__ bool gap(I) const { return false; }
   template <class I>
   __device__ __forceinline__ const C* srcp(int, int slab, I e, int col) const {
     return p + ((long long)slab * ss() + col) + idx_off(e, es());
