@@ -587,11 +587,13 @@ extern "C" int mf_grid_power_spectrum(mf_grid* g, double* bin_k, double* bin_P, 
   if (nbins_cap < nbins || !bin_k || !bin_P || !bin_eP || !bin_count)
     return set_err(c, MF_ERR_ARG, "mf_grid_power_spectrum: output arrays too small");
   double* acc = nullptr;
-  cudaError_t e = cudaMallocAsync(&acc, sizeof(double) * 4 * nbins, c->stream);
+  const size_t acc_bytes = sizeof(double) * 4 * nbins;  // the sums, then the scratch tables
+  cudaError_t e = cudaMallocAsync(&acc, acc_bytes + pw_power_spectrum_scratch(g->n), c->stream);
+  void* scratch = (char*)acc + acc_bytes;
   if (e == cudaSuccess) e = cudaMemsetAsync(acc, 0, sizeof(double) * 4 * nbins, c->stream);
   if (e == cudaSuccess)
-    e = (g->prec == MF_PREC_F64) ? pw_power_spectrum<double>((cplx<double>*)g->d, g->n, kfac, nbins, acc, c->stream)
-                                 : pw_power_spectrum<float>((cplx<float>*)g->d, g->n, kfac, nbins, acc, c->stream);
+    e = (g->prec == MF_PREC_F64) ? pw_power_spectrum<double>((cplx<double>*)g->d, g->n, kfac, nbins, acc, scratch, c->stream)
+                                 : pw_power_spectrum<float>((cplx<float>*)g->d, g->n, kfac, nbins, acc, scratch, c->stream);
   std::vector<double> h(4 * (size_t)nbins);
   if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), acc, sizeof(double) * 4 * nbins, cudaMemcpyDeviceToHost, c->stream);
   if (acc) cudaFreeAsync(acc, c->stream);

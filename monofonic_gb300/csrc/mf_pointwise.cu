@@ -107,37 +107,77 @@ __global__ void k_fill_from_f64(T* d, const double* src, int n) {
   }
 }
 
-// binned |delta_k|^2 (grid_fft.cc:1133-1181): per-block shared histograms
+// |k| = sqrt(k2) kfac and the P(k) bin of every k2 < nk2 with bins of width kfac
+// (grid_fft.cc:1150-1165).  A k2 that is a perfect square sits on a bin edge,
+// where the bin follows the rounding of the mode's own kx^2 + ky^2 + kz^2:
+// marked -1 and decided per mode.  Every other |k| is at least 1 / (2 sqrt(k2))
+// bins away from an edge, far more than any rounding.  -2: outside the bins.
+__global__ void __launch_bounds__(32) k_pk_table(double* kval, int* bin, int nk2, int n, double kfac) {
+  const int k2 = blockIdx.x * 32 + threadIdx.x;
+  if (k2 >= nk2) return;
+  int r = (int)sqrtf((float)k2);
+  while (r * r > k2) --r;
+  while ((r + 1) * (r + 1) <= k2) ++r;
+  kval[k2] = sqrt((double)k2) * kfac;
+  bin[k2] = (r * r == k2) ? -1 : (k2 > (n / 2) * (n / 2) ? -2 : r);
+}
+
+// binned |delta_k|^2 (grid_fft.cc:1133-1181): per-block shared histograms, one
+// copy per kPkWarps warps.  The bins and |k| come from the table: per mode that
+// leaves ~6 of ~35 FP64 operations (the square root, the division and the
+// conversions bounded the pass: 778 -> 330 us at N=256).
+constexpr int kPkWarps = 2;
 template <typename T>
-__global__ void k_pk(const cplx<T>* d, int n, double kfac, int nbins, double* acc) {
-  extern __shared__ double sh[];  // 4 * nbins
-  for (int b = threadIdx.x; b < 4 * nbins; b += blockDim.x) sh[b] = 0.0;
+__global__ void __launch_bounds__(kThreads) k_pk(const cplx<T>* d, int n, double kfac, int nbins, double* acc,
+                                                 const double* __restrict__ kval, const int* __restrict__ bin) {
+  constexpr int NCOPY = kThreads / (32 * kPkWarps);
+  extern __shared__ double sh[];  // NCOPY x 3 nbins sums, then NCOPY x nbins counts
+  unsigned* cnt0 = reinterpret_cast<unsigned*>(sh + NCOPY * 3 * nbins);
+  for (int b = threadIdx.x; b < NCOPY * 3 * nbins; b += blockDim.x) sh[b] = 0.0;
+  for (int b = threadIdx.x; b < NCOPY * nbins; b += blockDim.x) cnt0[b] = 0u;
   __syncthreads();
-  const int Kz = n / 2 + 1;
-  const size_t tot = (size_t)n * n * Kz;
+  const int copy = threadIdx.x / (32 * kPkWarps);
+  double* h = sh + copy * 3 * nbins;
+  unsigned* cnt = cnt0 + copy * nbins;
+  const unsigned Kz = n / 2 + 1;
+  const unsigned tot = (unsigned)n * n * Kz;  // n <= 1024
   const double kmin = kfac, kmax = kfac * (n / 2), dk = kmin;
-  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < tot; idx += (size_t)gridDim.x * blockDim.x) {
-    const int kz = (int)(idx % Kz);
-    const int j = (int)((idx / Kz) % n);
-    const int i = (int)(idx / ((size_t)Kz * n));
-    const double kx = kcomp<double>(i, n, kfac), ky = kcomp<double>(j, n, kfac), kk = kcomp<double>(kz, n, kfac);
-    // |k| without contraction into FMAs (modes of integer norm sit on bin
-    // edges, so the bin follows the exact rounding of x*x + y*y + z*z)
-    const double k = sqrt(__dadd_rn(__dadd_rn(__dmul_rn(kx, kx), __dmul_rn(ky, ky)), __dmul_rn(kk, kk)));
-    if (k >= kmin && k < kmax) {
-      const int b = (int)(k / dk);
+  for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < tot; idx += gridDim.x * blockDim.x) {
+    const unsigned line = idx / Kz;
+    const int kz = (int)(idx - line * Kz);
+    const int i = (int)(line / (unsigned)n);
+    const int j = (int)(line - (unsigned)i * (unsigned)n);
+    const int ii = i - (i > n / 2 ? n : 0), jj = j - (j > n / 2 ? n : 0);
+    const int k2 = ii * ii + jj * jj + kz * kz;
+    int b = bin[k2];
+    double k = kval[k2];
+    if (b == -1) {
+      const double kx = kcomp<double>(i, n, kfac), ky = kcomp<double>(j, n, kfac), kk = kcomp<double>(kz, n, kfac);
+      // |k| without contraction into FMAs (the bin follows the exact rounding of x*x + y*y + z*z)
+      k = sqrt(__dadd_rn(__dadd_rn(__dmul_rn(kx, kx), __dmul_rn(ky, ky)), __dmul_rn(kk, kk)));
+      b = (k >= kmin && k < kmax) ? (int)(k / dk) : -2;
+    }
+    if (b >= 0 && b < nbins) {
       const cplx<T> z = d[idx];
       const double v = (double)z.x * (double)z.x + (double)z.y * (double)z.y;
-      const double w = (kz == 0) ? 1.0 : 2.0;
-      atomicAdd(&sh[b], w * v);
-      atomicAdd(&sh[nbins + b], w * v * v);
-      atomicAdd(&sh[2 * nbins + b], w * k);
-      atomicAdd(&sh[3 * nbins + b], w);
+      const double wv = (kz == 0) ? v : v + v;
+      atomicAdd(&h[b], wv);
+      atomicAdd(&h[nbins + b], wv * v);
+      atomicAdd(&h[2 * nbins + b], (kz == 0) ? k : k + k);
+      atomicAdd(&cnt[b], (kz == 0) ? 1u : 2u);
     }
   }
   __syncthreads();
-  for (int b = threadIdx.x; b < 4 * nbins; b += blockDim.x)
-    if (sh[b] != 0.0) atomicAdd(&acc[b], sh[b]);
+  for (int b = threadIdx.x; b < 3 * nbins; b += blockDim.x) {
+    double s = 0.0;
+    for (int c = 0; c < NCOPY; ++c) s += sh[c * 3 * nbins + b];
+    if (s != 0.0) atomicAdd(&acc[b], s);
+  }
+  for (int b = threadIdx.x; b < nbins; b += blockDim.x) {
+    unsigned s = 0;
+    for (int c = 0; c < NCOPY; ++c) s += cnt0[c * nbins + b];
+    if (s) atomicAdd(&acc[3 * nbins + b], (double)s);
+  }
 }
 
 }  // namespace
@@ -175,14 +215,27 @@ cudaError_t pw_white_noise(T* d, int n, unsigned long long seed, const unsigned 
   k_white_noise<T><<<grid_for((size_t)n * n * (n / 2), 2), kThreads, 0, s>>>(d, n, seed, seed_dev);
   return cudaGetLastError();
 }
+size_t pw_power_spectrum_scratch(int n) {
+  const size_t nk2 = 3 * (size_t)(n / 2) * (n / 2) + 1;
+  return nk2 * (sizeof(double) + sizeof(int));
+}
 template <typename T>
-cudaError_t pw_power_spectrum(const cplx<T>* d, int n, double kfac, int nbins, double* acc, cudaStream_t s) {
-  const size_t smem = (size_t)4 * nbins * sizeof(double);
+cudaError_t pw_power_spectrum(const cplx<T>* d, int n, double kfac, int nbins, double* acc, void* scratch,
+                              cudaStream_t s) {
+  const int nk2 = 3 * (n / 2) * (n / 2) + 1;
+  double* kval = (double*)scratch;
+  int* bin = (int*)(kval + nk2);
+  k_pk_table<<<(nk2 + 31) / 32, 32, 0, s>>>(kval, bin, nk2, n, kfac);
+  constexpr int NCOPY = kThreads / (32 * kPkWarps);
+  const size_t smem = (size_t)NCOPY * nbins * (3 * sizeof(double) + sizeof(unsigned));
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k_pk<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  k_pk<T><<<grid_for((size_t)n * n * (n / 2 + 1), 8), kThreads, smem, s>>>(d, n, kfac, nbins, acc);
+  // a few blocks per SM: every block adds its histogram to the result
+  unsigned grid = grid_for((size_t)n * n * (n / 2 + 1), 8);
+  if (grid > 152u * 8u) grid = 152u * 8u;
+  k_pk<T><<<grid, kThreads, smem, s>>>(d, n, kfac, nbins, acc, kval, bin);
   return cudaGetLastError();
 }
 
@@ -193,7 +246,7 @@ cudaError_t pw_power_spectrum(const cplx<T>* d, int n, double kfac, int nbins, d
   template cudaError_t pw_shift<T>(cplx<T>*, int, double, double, const double*, cudaStream_t);      \
   template cudaError_t pw_fill_from_f64<T>(T*, const double*, int, cudaStream_t);                    \
   template cudaError_t pw_white_noise<T>(T*, int, unsigned long long, const unsigned long long*, cudaStream_t); \
-  template cudaError_t pw_power_spectrum<T>(const cplx<T>*, int, double, int, double*, cudaStream_t);
+  template cudaError_t pw_power_spectrum<T>(const cplx<T>*, int, double, int, double*, void*, cudaStream_t);
 INST(float)
 INST(double)
 #undef INST

@@ -119,7 +119,10 @@ cudaError_t pw_sources(int set, const T* const* fields, T* const* outs, size_t n
 // seed from *seed_dev when it is not null
 template <typename T>
 cudaError_t pw_white_noise(T* d, int n, unsigned long long seed, const unsigned long long* seed_dev, cudaStream_t s);
+// binned |delta_k|^2; scratch: pw_power_spectrum_scratch(n) bytes
+size_t pw_power_spectrum_scratch(int n);
 template <typename T>
-cudaError_t pw_power_spectrum(const cplx<T>* d, int n, double kfac, int nbins, double* acc /*4*nbins*/, cudaStream_t s);
+cudaError_t pw_power_spectrum(const cplx<T>* d, int n, double kfac, int nbins, double* acc /*4*nbins*/, void* scratch,
+                              cudaStream_t s);
 
 }  // namespace mf
