@@ -71,6 +71,12 @@ __host__ __device__ constexpr int col_layout() {
   return (col_swizzle<OP>::value && NCOL * (int)sizeof(cplx<T>) == 64) ? 2 : 0;
 }
 
+// the plain N-grid passes
+template <class OP>
+struct plain_op : std::false_type {};
+template <typename T, int L, int AXIS>
+struct plain_op<PlainStridedOp<T, L, AXIS>> : std::true_type {};
+
 // whether a pass transforms its lines in fixed point: FP64, unless the op asks
 // for FP64 butterflies
 template <class OP, class = void>
@@ -314,13 +320,14 @@ k_colfft_pipe(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nsl
 // ---------------------------------------------------------------------------
 // (measured per launch, before -> after: y c2r of an operand pair 22.1 -> 17.2
 // us at L = 192, 70.0 -> 52.1 at 288, 142 -> 121 at 384, of three operands 1176
-// -> 979 us at 768; N-grid passes 292 -> 229 us at 512.  L = 256 keeps its
-// radix-8 plan, eight values per thread: 36 us, 16 x 16 took 41.)
+// -> 979 us at 768; N-grid passes 292 -> 229 us at 512; five aliased
+// products at N=256 1430 -> 1309 us with tiles of 16 columns.)
 __host__ __device__ constexpr int col2_r1(int L) {
   switch (L) {
     case 128: return 8;
     case 144: return 12;
     case 192: return 12;
+    case 256: return 16;
     case 288: return 12;
     case 384: return 16;
     case 512: return 16;

@@ -80,7 +80,13 @@ constexpr int pipe_ncol() {
 // whether a strided pass takes the two-stage kernels
 template <typename T, int L>
 constexpr bool two_stage() { return sizeof(T) == 4 && col2_r1(L) > 0; }
-constexpr int kCol2Cols = 8;  // 64-byte rows
+// columns per tile of the two-stage passes: 128-byte rows (16) for length 256 and
+// for the N-grid passes of length 384, where two tiles of a CTA leave room for
+// enough CTAs; else 64-byte rows.  Measured, 16 against 8 columns: five aliased
+// products at N=256 1309 / 1430 us, a 384^3 field 1138 / 1173 us, but padded
+// products at N=256 (length 384) 2158 / 2098 us, at N=128 (192) 388 / 370 us.
+template <int L, class OP>
+constexpr int col2_cols() { return (L == 256 || (L == 384 && plain_op<OP>::value)) ? 16 : 8; }
 
 // a persistent strided pass: as many CTAs as fit, or the tuned number per SM
 template <class KERN, typename... ARGS>
@@ -104,7 +110,7 @@ template <typename T, int L, bool INV, class OP>
 cudaError_t launch_col(OP op, int nslab, int ncols, int nz, const cplx<T>* tw, cudaStream_t s, int kind) {
   const int occ = sched_get(kind, L, (int)sizeof(T)).occ;
   if constexpr (two_stage<T, L>()) {
-    constexpr int NC = kCol2Cols;
+    constexpr int NC = col2_cols<L, OP>();
     const int ntc = (ncols + NC - 1) / NC;
     return launch_tiles(k_col2<T, L, INV, NC, OP>, dim3(NC, Col2<L>::TY), (size_t)2 * L * NC * sizeof(cplx<T>), occ,
                         ntc * nslab * nz, s, op, tw, ncols, ntc, nslab, nz);
@@ -428,7 +434,7 @@ cudaError_t Launch<T>::conv_xfwd(int L, ConvXFwdOp<T> op, int nslab, int ncols, 
 template <typename T, int L, class OP>
 cudaError_t launch_xtrunc(OP op, int nslab, int ncols, const cplx<T>* tw, cudaStream_t s) {
   if constexpr (two_stage<T, L>()) {
-    constexpr int NC = kCol2Cols;
+    constexpr int NC = col2_cols<L, OP>();
     const int ntc = (ncols + NC - 1) / NC;
     return launch_tiles(k_col2_trunc<T, L, NC, OP>, dim3(NC, Col2<L>::TY), (size_t)2 * L * NC * sizeof(cplx<T>), 0,
                         ntc * nslab, s, op, tw, ncols, ntc, nslab);
