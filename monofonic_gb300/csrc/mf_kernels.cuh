@@ -243,7 +243,7 @@ k_colfft_pipe(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nsl
 #pragma unroll 2
         for (int i = 0; i < F::E; ++i) {
           const int o = tile_slot<F, NCOL>(t, i) + c;
-          buf0[o] = op.xform_tile(tp, t + i * F::TPL, buf0[o]);
+          if (op.src_ok(t + i * F::TPL)) buf0[o] = op.xform_tile(tp, t + i * F::TPL, buf0[o]);
         }
       }
       const int xs = col_fx<F, NCOL>(buf0, t, c, tw);

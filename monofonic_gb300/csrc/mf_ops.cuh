@@ -212,13 +212,13 @@ struct ConvXInvOp {
   }
   template <class I>
   __device__ __forceinline__ C xform_tile(const Tile& t, I x, C v0) const {
-    const T gi = G::template row_comp<T>(x) * kfac;
-    if (t.grad) {
-      const T f = t.c1 * gi + t.c0;
-      return mkc<T>(-f * v0.y, f * v0.x);
+    T f = t.c0;
+    // (in FP64 the operands without an x direction skip the factor's four operations)
+    if (sizeof(T) == 4 || t.c1 != T(0) || t.c2 != T(0)) {
+      const T gi = G::template row_comp<T>(x) * kfac;
+      f = (t.c2 * gi + t.c1) * gi + t.c0;
     }
-    const T f = (t.c2 * gi + t.c1) * gi + t.c0;
-    return mkc<T>(v0.x * f, v0.y * f);
+    return t.grad ? mkc<T>(-f * v0.y, f * v0.x) : mkc<T>(v0.x * f, v0.y * f);
   }
   template <class I>
   __device__ __forceinline__ void store_z(int z, int j, I x, int kz, C v) const {
@@ -341,8 +341,9 @@ struct ConvXFwdOp {
     else if (out_op == OUT_SUB) r = csub(r, v);
     else r = mkc<T>(r.x + v.x * x, r.y + v.y * x);
     if (post_invlap) {
-      const T kx = kcomp<T>(i, g.N, kfac), ky = kcomp<T>(j, g.N, kfac), kzz = kcomp<T>(kz, g.N, kfac);
-      const T k2 = kx * kx + ky * ky + kzz * kzz;
+      // k^2 from the integer components (exact: below 2^24)
+      const int ii = i - ((i > nh) ? g.N : 0), jj = j - ((j > nh) ? g.N : 0);
+      const T k2 = T(ii * ii + jj * jj + kz * kz) * (kfac * kfac);
       const T m = -rcp_rn(k2);
       r = (idx == 0) ? mkc<T>(T(0), T(0)) : mkc<T>(r.x * m, r.y * m);
     }
