@@ -171,5 +171,82 @@ __device__ __forceinline__ bool normal_pair_f32(uint64_t p, uint64_t seed, float
   return ok;
 }
 
+// The draws in FP64: the operations of normal_pair (mf_noise.h) that round, in
+// its order, with those that are exact done on integers -- the conversions of
+// the 53-bit integers, the halving and the powers of two, nine of ~66
+// operations on the FP64 pipe, which bounds it.
+__device__ __forceinline__ double exact_double(long long x, int sh) {  // x 2^-sh, |x| < 2^53
+  const long long s = x >> 63;
+  const unsigned long long a = (unsigned long long)((x ^ s) - s);
+  const int lz = __clzll((long long)a);
+  const long long b = (long long)((a << (lz & 63)) >> 11) + ((long long)(1085 - lz - sh) << 52);
+  return __longlong_as_double(a ? (b | (s & (long long)0x8000000000000000ull)) : 0ll);
+}
+__device__ __forceinline__ void normal_pair_f64(uint64_t p, uint64_t seed, double* z0, double* z1) {
+  uint32_t c[4] = {(uint32_t)(p & 0xFFFFFFFFu), (uint32_t)(p >> 32), 0u, 0u};
+  philox4x32_10(c, (uint32_t)(seed & 0xFFFFFFFFu), (uint32_t)(seed >> 32));
+  const uint64_t b1 = ((((uint64_t)c[1]) << 32) | c[0]) >> 11;
+  const uint64_t b2 = ((((uint64_t)c[3]) << 32) | c[2]) >> 11;
+  const uint64_t u = (b1 >> 52) ? 2 * (b1 + (b1 & 1)) : 2 * b1 + 1;  // as in normal_pair_f32
+  if (u >> 54) {
+    normal_pair(p, seed, z0, z1);
+    return;
+  }
+  // log_pos: u = m 2^e
+  const int lz = __clzll((long long)u);
+  const uint64_t mant = ((u << lz) >> 11) & 0x000FFFFFFFFFFFFFull;
+  int e = 9 - lz;
+  const bool half = mant > 0x6a09e667f3bcdull;  // m > sqrt(2)
+  e += half;
+  const double m = from_bits(mant | ((half ? 0x3FEull : 0x3FFull) << 52));
+  const double s = div_(sub(m, 1.0), add(m, 1.0));
+  const double z = mul(s, s);
+  double q = 0x1.642c8590b2164p-4;
+  q = fma_(q, z, 0x1.8618618618618p-4);
+  q = fma_(q, z, 0x1.af286bca1af28p-4);
+  q = fma_(q, z, 0x1.e1e1e1e1e1e1ep-4);
+  q = fma_(q, z, 0x1.1111111111111p-3);
+  q = fma_(q, z, 0x1.3b13b13b13b14p-3);
+  q = fma_(q, z, 0x1.745d1745d1746p-3);
+  q = fma_(q, z, 0x1.c71c71c71c71cp-3);
+  q = fma_(q, z, 0x1.2492492492492p-2);
+  q = fma_(q, z, 0x1.999999999999ap-2);
+  q = fma_(q, z, 0x1.5555555555555p-1);
+  q = fma_(q, z, 2.0);
+  const double ln = fma_(exact_double(e, 0), 0x1.62e42fefa39efp-1, mul(s, q));
+  // -2 ln: exact (ln is negative and normal for u < 1)
+  const double r = sqrt_(from_bits((bits(ln) ^ 0x8000000000000000ull) + (1ull << 52)));
+  // sincos_turn53 with its exact argument
+  const uint64_t t = (b2 + (1ull << 50)) >> 51;
+  const double f = exact_double((long long)(2 * b2 + 1) - (long long)(t << 52), 52);
+  const double w = mul(f, f);
+  double ps = -0x1.8a404211f9547p-45;
+  ps = fma_(ps, w, 0x1.aaec32af93359p-38);
+  ps = fma_(ps, w, -0x1.6fadb9f155744p-31);
+  ps = fma_(ps, w, 0x1.e8f434d018d63p-25);
+  ps = fma_(ps, w, -0x1.e3074fde8871fp-19);
+  ps = fma_(ps, w, 0x1.50783487ee782p-13);
+  ps = fma_(ps, w, -0x1.32d2cce62bd86p-8);
+  ps = fma_(ps, w, 0x1.466bc6775aae2p-4);
+  ps = fma_(ps, w, -0x1.4abbce625be53p-1);
+  ps = fma_(ps, w, 0x1.921fb54442d18p+0);
+  double pc = -0x1.2a0c591af8314p-41;
+  pc = fma_(pc, w, 0x1.20c62c2f2d7f5p-34);
+  pc = fma_(pc, w, -0x1.b6e24f44b128fp-28);
+  pc = fma_(pc, w, 0x1.f9d38a3763cc3p-22);
+  pc = fma_(pc, w, -0x1.a6d1f2a204a8cp-16);
+  pc = fma_(pc, w, 0x1.e1f506891babbp-11);
+  pc = fma_(pc, w, -0x1.55d3c7e3cbffap-6);
+  pc = fma_(pc, w, 0x1.03c1f081b5ac4p-2);
+  pc = fma_(pc, w, -0x1.3bd3cc9be45dep+0);
+  pc = fma_(pc, w, 1.0);
+  const double sn = mul(f, ps);
+  const int k = (int)(t & 3);
+  const double a = mul(r, (k & 1) ? sn : pc), b = mul(r, (k & 1) ? pc : sn);
+  // quadrants: (sin, cos) = (s, c), (c, -s), (-s, -c), (-c, s); signs are exact
+  *z0 = (k == 1 || k == 2) ? -a : a;
+  *z1 = (k >= 2) ? -b : b;
+}
+
 }  // namespace noise
 }  // namespace mf

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kThreads) k_white_noise(T* d, int n, unsigned 
     if constexpr (std::is_same<T, float>::value) done = noise::normal_pair_f32(p, sd, &v.x, &v.y);
     if (!done) {
       double z0, z1;
-      noise::normal_pair(p, sd, &z0, &z1);
+      noise::normal_pair_f64(p, sd, &z0, &z1);
       v.x = (T)z0;
       v.y = (T)z1;
     }
