@@ -23,31 +23,15 @@
 #ifndef MF_COL_MAXR
 #define MF_COL_MAXR 8
 #endif
-// threads per CTA up to which the pipelined strided passes are compiled for two
-// resident CTAs per SM (a register cap of 65536 / (2 x threads)); a build-time knob.
-// 512 puts two 512-thread CTAs of the FP32 length-512 passes on an SM (64
-// registers, no spills): 0.4 ms less per 512^3 3LPT IC than one CTA at 256.
-#ifndef MF_COL_MINB_LIMIT
-#define MF_COL_MINB_LIMIT 512
-#endif
-// 1: the pipelined strided passes' resident CTAs per SM sized from the
-// registers the plan needs (~4 per scalar held, plus 32) instead of the rule
-// above, at most 4; a build-time knob.  The 128-thread CTAs of the FP32
-// length-96..384 passes were compiled for two CTAs per SM and took up to 255
-// registers (8 warps per SM); sized for four (128 registers, no spills) the
-// N=256 3LPT IC takes 10.9 instead of 11.7 ms and the 96-realization batch
-// 215 instead of 231 ms.  M=768 and N=512 passes compile as before.
-#ifndef MF_COL_REG_SIZED
-#define MF_COL_REG_SIZED 1
-#endif
 
 namespace mf {
 
-// minimum resident CTAs per SM a pipelined strided pass is compiled for
-// (its __launch_bounds__): threads per CTA, values per thread E of the plan,
-// bytes per scalar
+// minimum resident CTAs per SM a pipelined strided pass is compiled for (its
+// __launch_bounds__): threads per CTA, values per thread E of the plan, bytes
+// per scalar.  Sized from the registers the plan needs (~4 per scalar held,
+// plus 32), at most 4: without the bound the 128-thread FP32 CTAs took up to
+// 255 registers (8 warps per SM).
 __host__ __device__ constexpr int col_minb(int threads, int e, int scalar_bytes) {
-  if (!MF_COL_REG_SIZED) return threads <= MF_COL_MINB_LIMIT ? 2 : 1;
   int need = 4 * e * (scalar_bytes / 4) + 32;
   if (scalar_bytes == 8 && need > 168) need = 168;  // fixed-point FP64 columns: three 128-thread CTAs
   need = need < 64 ? 64 : (need > 255 ? 255 : need);
@@ -168,7 +152,8 @@ k_colfft3s(OP op, const cplx<T>* __restrict__ tw, int ncols) {
 }
 
 // ---------------------------------------------------------------------------
-// persistent, double-buffered strided pass.  Each CTA walks tiles
+// persistent strided pass of the FP64 lines and of the FP32 lengths without a
+// two-stage plan (k_col2 below; double-buffered in FP32).  Each CTA walks tiles
 // (column tile, slab, operand) with stride gridDim.x; while a tile is being
 // transformed, the raw elements of the CTA's next tile are already being
 // copied into the other shared-memory buffer with cp.async.  Every thread
@@ -533,7 +518,7 @@ k_col2_trunc(OP op, const cplx<T>* __restrict__ tw, int ncols, int ntc, int nsla
 
 // ---------------------------------------------------------------------------
 // strided forward transform, truncation and inverse transform of one column in
-// one pass (ConvXTruncOp), persistent and double-buffered as k_colfft_pipe
+// one pass (ConvXTruncOp), for the lengths that k_colfft_pipe takes and as there
 // ---------------------------------------------------------------------------
 template <typename T, int L, int NCOL, class OP>
 __global__ void __launch_bounds__(NCOL * LineFFT<T, L, false, MF_COL_MAXR>::TPL,
@@ -1012,7 +997,9 @@ __global__ void __launch_bounds__(NT, MINB) k_zconv(ZConvArgs<T> a, const cplx<T
 // asynchronous copies (cp.async.bulk, one per operand, completion counted on
 // an mbarrier) into the other half of a double buffer while the current batch
 // is transformed, so HBM traffic overlaps the FFT work.
-// Shared memory: [2 mbarriers | stage[2][nop][LPB][kin] | exchange[LPB][H+1]]
+// Shared memory: [2 mbarriers | stage[2][nop][LPB][line stride] | exchange[LPB][line stride]],
+// the exchange only where the staged lines cannot hold it; FP64 lines, bound by
+// the integer pipes, are transformed in place in one stage.
 // ---------------------------------------------------------------------------
 template <typename T, int H>
 __device__ __forceinline__ cplx<T> c2r_pre_s(const cplx<T>* src, int k, int kin, const cplx<T>* __restrict__ twM) {

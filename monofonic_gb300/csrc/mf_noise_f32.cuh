@@ -13,7 +13,7 @@
 // Why: the sequence takes ~61 FP64 operations per pair at 1.68 per clock and
 // SM; the float pairs take ~300 FP32 operations at ~120.  A noise field and its
 // potential on a 384^3 grid: 4.60 ms with the FP64 sequence (3.64 ms of it the
-// noise), 1.37 ms with the pairs.
+// noise), 1.37 ms with the pairs (1.13 ms with the transform passes of today).
 #pragma once
 
 #include "mf_noise.h"

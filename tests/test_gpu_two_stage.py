@@ -1,4 +1,4 @@
-"""FP32 strided passes in two stages (pass lengths 128..768 but 256) against the
+"""FP32 strided passes in two stages (pass lengths 128..768) against the
 FP64 transforms: every output operator of a padded product, the N-grid
 transforms, and a 3LPT run, whose pair products go through the truncation pass.
 
