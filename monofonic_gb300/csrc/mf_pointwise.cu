@@ -125,7 +125,10 @@ __global__ void __launch_bounds__(32) k_pk_table(double* kval, int* bin, int nk2
 // binned |delta_k|^2 (grid_fft.cc:1133-1181): per-block shared histograms, one
 // copy per kPkWarps warps.  The bins and |k| come from the table: per mode that
 // leaves ~6 of ~35 FP64 operations (the square root, the division and the
-// conversions bounded the pass: 778 -> 330 us at N=256).
+// conversions bounded the pass: 778 -> 330 us at N=256).  The shared-memory
+// atomics bounded what was left, so a thread takes the up to eight modes
+// (+-a, +-b, kz), (+-b, +-a, kz), 0 <= a, b <= n/2, of one |k| and bin together
+// (330 -> 130 us at N=256).
 constexpr int kPkWarps = 2;
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_pk(const cplx<T>* d, int n, double kfac, int nbins, double* acc,
@@ -139,32 +142,53 @@ __global__ void __launch_bounds__(kThreads) k_pk(const cplx<T>* d, int n, double
   const int copy = threadIdx.x / (32 * kPkWarps);
   double* h = sh + copy * 3 * nbins;
   unsigned* cnt = cnt0 + copy * nbins;
-  const unsigned Kz = n / 2 + 1;
-  const unsigned tot = (unsigned)n * n * Kz;  // n <= 1024
+  const int h1 = n / 2, M = h1 + 1;
+  const unsigned Kz = h1 + 1;
+  // unordered pairs of [0, M): (a, a + e mod M), e <= M/2 (at e = M/2, M even, each twice)
+  const unsigned ne = M / 2 + 1;
+  const unsigned tot = (unsigned)M * ne * Kz;
   const double kmin = kfac, kmax = kfac * (n / 2), dk = kmin;
   for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < tot; idx += gridDim.x * blockDim.x) {
     const unsigned line = idx / Kz;
     const int kz = (int)(idx - line * Kz);
-    const int i = (int)(line / (unsigned)n);
-    const int j = (int)(line - (unsigned)i * (unsigned)n);
-    const int ii = i - (i > n / 2 ? n : 0), jj = j - (j > n / 2 ? n : 0);
-    const int k2 = ii * ii + jj * jj + kz * kz;
+    const int i = (int)(line / ne);
+    const int e = (int)(line - (unsigned)i * ne);
+    int j = i + e;
+    if (j >= M) j -= M;
+    if (2 * e == M && i >= e) continue;
+    const int k2 = i * i + j * j + kz * kz;
     int b = bin[k2];
     double k = kval[k2];
     if (b == -1) {
       const double kx = kcomp<double>(i, n, kfac), ky = kcomp<double>(j, n, kfac), kk = kcomp<double>(kz, n, kfac);
-      // |k| without contraction into FMAs (the bin follows the exact rounding of x*x + y*y + z*z)
+      // |k| without contraction into FMAs (the bin follows the exact rounding of
+      // x*x + y*y + z*z, the same for either sign and order of x and y)
       k = sqrt(__dadd_rn(__dadd_rn(__dmul_rn(kx, kx), __dmul_rn(ky, ky)), __dmul_rn(kk, kk)));
       b = (k >= kmin && k < kmax) ? (int)(k / dk) : -2;
     }
     if (b >= 0 && b < nbins) {
-      const cplx<T> z = d[idx];
-      const double v = (double)z.x * (double)z.x + (double)z.y * (double)z.y;
-      const double wv = (kz == 0) ? v : v + v;
-      atomicAdd(&h[b], wv);
-      atomicAdd(&h[nbins + b], wv * v);
-      atomicAdd(&h[2 * nbins + b], (kz == 0) ? k : k + k);
-      atomicAdd(&cnt[b], (kz == 0) ? 1u : 2u);
+      const bool pi = i > 0 && i < h1, pj = j > 0 && j < h1;  // has a mirror image
+      const int m = (pi ? 2 : 1) * (pj ? 2 : 1) * (e ? 2 : 1);
+      cplx<T> z[8];  // all in flight before the first use
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int x = (q & 1) ? n - i : i, y = (q & 2) ? n - j : j;
+        const size_t row = (q & 4) ? (size_t)y * n + x : (size_t)x * n + y;
+        z[q] = mkc<T>(T(0), T(0));
+        if ((!(q & 1) || pi) && (!(q & 2) || pj) && (!(q & 4) || e)) z[q] = d[row * Kz + kz];
+      }
+      double s1 = 0.0, s2 = 0.0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const double v = (double)z[q].x * (double)z[q].x + (double)z[q].y * (double)z[q].y;
+        s1 += v;
+        s2 += v * v;
+      }
+      const double w = (kz == 0) ? 1.0 : 2.0;
+      atomicAdd(&h[b], w * s1);
+      atomicAdd(&h[nbins + b], w * s2);
+      atomicAdd(&h[2 * nbins + b], w * m * k);
+      atomicAdd(&cnt[b], (kz == 0) ? (unsigned)m : 2u * m);
     }
   }
   __syncthreads();
@@ -233,7 +257,7 @@ cudaError_t pw_power_spectrum(const cplx<T>* d, int n, double kfac, int nbins, d
     if (e != cudaSuccess) return e;
   }
   // a few blocks per SM: every block adds its histogram to the result
-  unsigned grid = grid_for((size_t)n * n * (n / 2 + 1), 8);
+  unsigned grid = grid_for((size_t)(n / 2 + 1) * (n / 4 + 1) * (n / 2 + 1));
   if (grid > 152u * 8u) grid = 152u * 8u;
   k_pk<T><<<grid, kThreads, smem, s>>>(d, n, kfac, nbins, acc, kval, bin);
   return cudaGetLastError();
