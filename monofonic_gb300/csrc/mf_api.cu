@@ -375,6 +375,7 @@ extern "C" int mf_ctx_destroy(mf_ctx* c) {
   for (auto& rec : c->prof_events) { cudaEventDestroy(rec.second.first); cudaEventDestroy(rec.second.second); }
   for (auto e : c->event_pool) cudaEventDestroy(e);
   cudaFree(c->d_err);
+  cudaFree(c->ws);
   cudaStreamDestroy(c->stream);
   delete c;
   return MF_OK;
@@ -588,7 +589,23 @@ extern "C" int mf_grid_power_spectrum(mf_grid* g, double* bin_k, double* bin_P, 
     return set_err(c, MF_ERR_ARG, "mf_grid_power_spectrum: output arrays too small");
   double* acc = nullptr;
   const size_t acc_bytes = sizeof(double) * 4 * nbins;  // the sums, then the scratch tables
-  cudaError_t e = cudaMallocAsync(&acc, acc_bytes + pw_power_spectrum_scratch(g->n), c->stream);
+  const size_t need = acc_bytes + pw_power_spectrum_scratch(g->n);
+  // the context's scratch, unless another thread's call has it or the stream is captured
+  std::unique_lock<std::mutex> own(c->ws_mu, std::try_to_lock);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(c->stream, &cap);
+  const bool kept = own.owns_lock() && e == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+  if (e == cudaSuccess && kept && c->ws_bytes < need) {
+    if (c->ws) cudaFreeAsync(c->ws, c->stream);
+    c->ws = nullptr;
+    c->ws_bytes = 0;
+    e = cudaMallocAsync(&c->ws, need, c->stream);
+    if (e == cudaSuccess) c->ws_bytes = need;
+  }
+  if (e == cudaSuccess) {
+    if (kept) acc = (double*)c->ws;
+    else e = cudaMallocAsync(&acc, need, c->stream);
+  }
   void* scratch = (char*)acc + acc_bytes;
   if (e == cudaSuccess) e = cudaMemsetAsync(acc, 0, sizeof(double) * 4 * nbins, c->stream);
   if (e == cudaSuccess)
@@ -596,8 +613,9 @@ extern "C" int mf_grid_power_spectrum(mf_grid* g, double* bin_k, double* bin_P, 
                                  : pw_power_spectrum<float>((cplx<float>*)g->d, g->n, kfac, nbins, acc, scratch, c->stream);
   std::vector<double> h(4 * (size_t)nbins);
   if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), acc, sizeof(double) * 4 * nbins, cudaMemcpyDeviceToHost, c->stream);
-  if (acc) cudaFreeAsync(acc, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  if (acc && !kept) cudaFreeAsync(acc, c->stream);
+  const cudaError_t es = cudaStreamSynchronize(c->stream);  // (also before another call may take the scratch)
+  if (e == cudaSuccess) e = es;
   if (e != cudaSuccess) return cuda_err(c, e, "mf_grid_power_spectrum");
   // normalisation (grid_fft.cc:1198-1209)
   const double volfac = g->L * g->L * g->L / std::pow(2.0 * M_PI, 3.0);
