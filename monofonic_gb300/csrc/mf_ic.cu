@@ -477,41 +477,21 @@ int shared_sources(mf_ic* ic, bool timed) {
     if (e != cudaSuccess) return cuda_err(c, e, #x);     \
   } while (0)
 
-  // padded c2r of up to three operands into real fields dst[k]
-  auto c2r = [&](int nop, const Operand<T>* ops, const int* dst) -> cudaError_t {
-    ConvXInvOp<T> xo{};
-    for (int k = 0; k < nop; ++k) { xo.opnd[k] = ops[k]; xo.dst[k] = W[k]; }
-    xo.g = g;
-    xo.kfac = kfac;
-    xo.scale = scale_in;
-    cudaError_t e2;
-    {
-      LaunchScope ls(c, KK_CONV_XINV);
-      if ((e2 = Launch<T>::conv_xinv(M, xo, N, Kz, nop, twM, s)) != cudaSuccess) return e2;
-    }
-    ConvYInvOp<T> yo{};
-    for (int k = 0; k < nop; ++k) { yo.src[k] = W[k]; yo.dst[k] = W[k]; }
-    yo.g = g;
-    {
-      LaunchScope ls(c, KK_CONV_YINV);
-      if ((e2 = Launch<T>::conv_yinv(M, yo, M, Kz, nop, twM, s)) != cudaSuccess) return e2;
-    }
-    for (int k = 0; k < nop; ++k) {
-      ZConvArgs<T> za{};
-      za.in[0] = W[k];
-      za.out = R(dst[k]);
-      za.nop = 1;
-      za.kin = Kz;
-      za.kout = H;
-      za.in_stride = Kz;
-      za.out_stride = H;
-      za.nlines = M * M;
-      za.out_scale = T(1);
-      za.err = c->d_err;
-      LaunchScope ls(c, KK_CONV_Z);
-      if ((e2 = Launch<T>::z_c2r_tma(H, za, twH, twM, s)) != cudaSuccess) return e2;
-    }
-    return cudaSuccess;
+  // z pass of an operand's c2r, from a buffer of padded rows into real field dst
+  auto z_c2r = [&](const cplx<T>* in, int dst) -> cudaError_t {
+    ZConvArgs<T> za{};
+    za.in[0] = in;
+    za.out = R(dst);
+    za.nop = 1;
+    za.kin = Kz;
+    za.kout = H;
+    za.in_stride = Kz;
+    za.out_stride = H;
+    za.nlines = M * M;
+    za.out_scale = T(1);
+    za.err = c->d_err;
+    LaunchScope ls(c, KK_CONV_Z);
+    return Launch<T>::z_c2r_tma(H, za, twH, twM, s);
   };
   // product-sum scratch fields (after the 17 operand fields)
   const int P0 = (p.lpt_order > 2) ? 17 : 6;
@@ -563,24 +543,98 @@ int shared_sources(mf_ic* ic, bool timed) {
     LaunchScope ls(c, KK_POINTWISE);
     return pw_sources<T>(set, fields, outs, 2 * rl, s);
   };
-  // Hessian fields in the order (0,0) (1,1) (2,2) (0,1) (0,2) (1,2)
-  const int HD[6][2] = {{0, 0}, {1, 1}, {2, 2}, {0, 1}, {0, 2}, {1, 2}};
-  auto hessians = [&](int fi, int base) -> cudaError_t {
+  // The six padded Hessians of field fi into real fields base + 0..5, in the
+  // order (0,0) (1,1) (2,2) (0,1) (0,2) (1,2).
+  // FP64: two passes of three operands.
+  auto hessians6 = [&](int fi, int base) -> cudaError_t {
+    const int HD[6][2] = {{0, 0}, {1, 1}, {2, 2}, {0, 1}, {0, 2}, {1, 2}};
     for (int half = 0; half < 2; ++half) {
-      Operand<T> ops[3];
-      int dst[3];
+      ConvXInvOp<T> xo{};
+      ConvYInvOp<T> yo{};
       for (int k = 0; k < 3; ++k) {
-        ops[k] = Operand<T>{};
-        ops[k].f = (const cplx<T>*)ic->f[fi]->d;
-        ops[k].kind = OPND_HESS;
-        ops[k].d[0] = HD[3 * half + k][0];
-        ops[k].d[1] = HD[3 * half + k][1];
-        dst[k] = base + 3 * half + k;
+        xo.opnd[k] = Operand<T>{};
+        xo.opnd[k].f = (const cplx<T>*)ic->f[fi]->d;
+        xo.opnd[k].kind = OPND_HESS;
+        xo.opnd[k].d[0] = HD[3 * half + k][0];
+        xo.opnd[k].d[1] = HD[3 * half + k][1];
+        xo.dst[k] = W[k];
+        yo.src[k] = W[k];
+        yo.dst[k] = W[k];
       }
-      cudaError_t e2 = c2r(3, ops, dst);
-      if (e2 != cudaSuccess) return e2;
+      xo.g = g;
+      xo.kfac = kfac;
+      xo.scale = scale_in;
+      yo.g = g;
+      cudaError_t e2;
+      {
+        LaunchScope ls(c, KK_CONV_XINV);
+        if ((e2 = Launch<T>::conv_xinv(M, xo, N, Kz, 3, twM, s)) != cudaSuccess) return e2;
+      }
+      {
+        LaunchScope ls(c, KK_CONV_YINV);
+        if ((e2 = Launch<T>::conv_yinv(M, yo, M, Kz, 3, twM, s)) != cudaSuccess) return e2;
+      }
+      for (int k = 0; k < 3; ++k)
+        if ((e2 = z_c2r(W[k], base + 3 * half + k)) != cudaSuccess) return e2;
     }
     return cudaSuccess;
+  };
+  // FP32: along an x column only g_x varies, so three x transforms serve all
+  // six: of f, i g_x f and -g_x^2 f; the other factors are constant on the column
+  // and multiply it on the way into the y pass.  The x pass so writes three
+  // padded grids instead of six (3LPT runs: 61.9 -> 59.4 ms at N=512 BCC, 7.05 ->
+  // 6.77 at 256).  Fields that are still to be written hold what the three work
+  // buffers cannot.  In FP64 the factors on the y rows, half as many again as
+  // the x rows, cost what the transforms save (N=256 32.4 -> 32.0 ms, N=64 2LPT
+  // 0.68-0.72 -> 0.73 ms).
+  auto hessians3 = [&](int fi, int base) -> cudaError_t {
+    ConvXInvOp<T> xo{};
+    for (int k = 0; k < 3; ++k) {
+      xo.opnd[k] = Operand<T>{};
+      xo.opnd[k].f = (const cplx<T>*)ic->f[fi]->d;
+      xo.opnd[k].kind = k == 0 ? OPND_PLAIN : (k == 1 ? OPND_GRAD : OPND_HESS);
+      xo.dst[k] = W[k];
+    }
+    xo.g = g;
+    xo.kfac = kfac;
+    xo.scale = scale_in;
+    cudaError_t e2;
+    {
+      LaunchScope ls(c, KK_CONV_XINV);
+      if ((e2 = Launch<T>::conv_xinv(M, xo, N, Kz, 3, twM, s)) != cudaSuccess) return e2;
+    }
+    struct Part {
+      const cplx<T>* src;
+      cplx<T>* dst;
+      int y_pow, kz_pow, field;
+    };
+    // a part's destination is read by its z pass before the next launch or
+    // field overwrites it; no part's source is another's destination
+    const Part parts[2][3] = {
+        {{W[2], W[2], 0, 0, base}, {W[1], R(base + 5), 1, 0, base + 3}, {W[0], R(base + 2), 2, 0, base + 1}},
+        {{W[1], W[1], 0, 1, base + 4}, {W[0], R(base + 5), 0, 2, base + 2}, {W[0], W[2], 1, 1, base + 5}}};
+    for (const auto& ps : parts) {
+      ConvYHessOp<T> yo{};
+      for (int k = 0; k < 3; ++k) {
+        yo.src[k] = ps[k].src;
+        yo.dst[k] = ps[k].dst;
+        yo.y_pow[k] = ps[k].y_pow;
+        yo.kz_pow[k] = ps[k].kz_pow;
+      }
+      yo.g = g;
+      yo.kfac = kfac;
+      {
+        LaunchScope ls(c, KK_CONV_YINV);
+        if ((e2 = Launch<T>::conv_yhess(M, yo, M, Kz, 3, twM, s)) != cudaSuccess) return e2;
+      }
+      for (int k = 0; k < 3; ++k)
+        if ((e2 = z_c2r(ps[k].dst, ps[k].field)) != cudaSuccess) return e2;
+    }
+    return cudaSuccess;
+  };
+
+  auto hessians = [&](int fi, int base) -> cudaError_t {
+    return sizeof(T) == 4 ? hessians3(fi, base) : hessians6(fi, base);
   };
 
   // convolve3's first stage for one pair product held as a padded real field:
@@ -624,19 +678,7 @@ int shared_sources(mf_ic* ic, bool timed) {
       LaunchScope ls(c, KK_CONV_YINV);
       if ((e2 = Launch<T>::conv_yinv(M, yo, M, Kz, 1, twM, s)) != cudaSuccess) return e2;
     }
-    ZConvArgs<T> zc{};
-    zc.in[0] = W[0];
-    zc.out = R(dstf);
-    zc.nop = 1;
-    zc.kin = Kz;
-    zc.kout = H;
-    zc.in_stride = Kz;
-    zc.out_stride = H;
-    zc.nlines = M * M;
-    zc.out_scale = T(1);
-    zc.err = c->d_err;
-    LaunchScope ls(c, KK_CONV_Z);
-    return Launch<T>::z_c2r_tma(H, zc, twH, twM, s);
+    return z_c2r(W[0], dstf);
   };
 
   // ---- phi(2) (ic_generator.cc:471-488) ----------------------------------

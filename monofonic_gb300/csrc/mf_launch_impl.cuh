@@ -471,6 +471,21 @@ cudaError_t Launch<T>::conv_yinv(int L, ConvYInvOp<T> op, int nslab, int ncols, 
 #undef CASE
 }
 template <typename T>
+cudaError_t Launch<T>::conv_yhess(int L, ConvYHessOp<T> op, int nslab, int ncols, int nops, const cplx<T>* tw,
+                                  cudaStream_t s) {
+#define CASE(LL)                                                                                        \
+  case LL:                                                                                             \
+    if constexpr (sizeof(T) == 4 && orszag_len(LL)) {                                                  \
+      using G = CGeom<LL, true>;                                                                       \
+      if (!geom_matches<G>(op.g)) return cudaErrorInvalidValue;                                        \
+      return launch_col<T, LL, true>(op.template with_geom<G>(), nslab, ncols, nops, tw, s, KK_CONV_YINV); \
+    } else {                                                                                           \
+      return cudaErrorInvalidValue;                                                                    \
+    }
+  switch (L) { MF_LEN_CONV(CASE) default: return cudaErrorInvalidValue; }
+#undef CASE
+}
+template <typename T>
 cudaError_t Launch<T>::conv_yfwd(int L, ConvYFwdOp<T> op, int nslab, int ncols, const cplx<T>* tw,
                                  cudaStream_t s) {
 #define CASE(LL)                                                                                        \
@@ -479,6 +494,7 @@ cudaError_t Launch<T>::conv_yfwd(int L, ConvYFwdOp<T> op, int nslab, int ncols, 
   switch (L) { MF_LEN_CONV(CASE) default: return cudaErrorInvalidValue; }
 #undef CASE
 }
+template cudaError_t Launch<MF_T>::conv_yhess(int, ConvYHessOp<MF_T>, int, int, int, const cplx<MF_T>*, cudaStream_t);
 template cudaError_t Launch<MF_T>::conv_yinv(int, ConvYInvOp<MF_T>, int, int, int, const cplx<MF_T>*, cudaStream_t);
 template cudaError_t Launch<MF_T>::conv_yfwd(int, ConvYFwdOp<MF_T>, int, int, const cplx<MF_T>*, cudaStream_t);
 #endif

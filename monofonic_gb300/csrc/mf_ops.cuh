@@ -263,6 +263,69 @@ struct ConvYInvOp {
   }
 };
 
+// y pass of Hessians whose x pass left the factor of g_x in (1, i g_x or -g_x^2): the
+// operand's factor of g_y and g_kz multiplies the column on the way in.  Source
+// and destination may be one buffer (in place per column) or two.
+// kz_pow, y_pow: the powers of g_kz and g_y; their sum is the number of
+// factors of i still to apply (mod 4, i.e. i^2 = -1).
+template <typename T, class G = ConvGeom>
+struct ConvYHessOp {
+  using C = cplx<T>;
+  const C* src[3];  // compact rows j < N of each x slab
+  C* dst[3];        // rows y < M
+  int y_pow[3], kz_pow[3];
+  G g;
+  T kfac;
+  static constexpr bool kPrefetch = false;
+  template <class G2>
+  ConvYHessOp<T, G2> with_geom() const {
+    ConvYHessOp<T, G2> o{};
+    for (int k = 0; k < 3; ++k) {
+      o.src[k] = src[k];
+      o.dst[k] = dst[k];
+      o.y_pow[k] = y_pow[k];
+      o.kz_pow[k] = kz_pow[k];
+    }
+    o.kfac = kfac;
+    return o;
+  }
+  static constexpr bool kColSwizzle = true;
+  template <class I>
+  __device__ __forceinline__ bool src_ok(I y) const { return g.src_row(y) >= 0; }
+  template <class I>
+  __device__ __forceinline__ bool gap(I y) const { return g.gap(y); }
+  template <class I>
+  __device__ __forceinline__ const C* srcp(int z, int x, I y, int kz) const {
+    const C* s0 = z == 0 ? src[0] : (z == 1 ? src[1] : src[2]);
+    return s0 + ((long long)x * g.M * g.Kz + kz) + g.row_off(y, g.Kz);
+  }
+  // the factor c0 + c1 g_y + c2 g_y^2 of a column, times i if grad
+  struct Tile {
+    T c0, c1, c2;
+    bool grad;
+  };
+  __device__ __forceinline__ Tile tile_prep(int z, int, int kz) const {
+    const int p = z == 0 ? y_pow[0] : (z == 1 ? y_pow[1] : y_pow[2]);
+    const int q = z == 0 ? kz_pow[0] : (z == 1 ? kz_pow[1] : kz_pow[2]);
+    const T gk = gradk<T>(kz, g.N, kfac);
+    T f = p + q == 2 ? T(-1) : T(1);
+    if (q > 0) f *= gk;
+    if (q > 1) f *= gk;
+    return Tile{p == 0 ? f : T(0), p == 1 ? f : T(0), p == 2 ? f : T(0), p + q == 1};
+  }
+  template <class I>
+  __device__ __forceinline__ C xform_tile(const Tile& t, I y, C v0) const {
+    const T gj = G::template row_comp<T>(y) * kfac;
+    const T f = (t.c2 * gj + t.c1) * gj + t.c0;
+    return t.grad ? mkc<T>(-f * v0.y, f * v0.x) : mkc<T>(v0.x * f, v0.y * f);
+  }
+  template <class I>
+  __device__ __forceinline__ void store_z(int z, int x, I y, int kz, C v) const {
+    C* d = z == 0 ? dst[0] : (z == 1 ? dst[1] : dst[2]);
+    d[((long long)x * g.M * g.Kz + kz) + idx_off(y, g.Kz)] = v;
+  }
+};
+
 // y pass of the product's r2c: keeps only the rows unpad reads
 template <typename T, class G = ConvGeom>
 struct ConvYFwdOp {
