@@ -137,9 +137,9 @@ class Clocks:
 def algorithmic_bytes_ic(n: int, prec_bytes: int, overload: int = 2, plt: bool = True) -> dict:
     """Unique bytes each kernel kind must read and write for one 3LPT IC of the
     shared-source pipeline (each element once; re-reads not counted):
-    17 operands through the padded c2r (y and z passes; x passes: FP32 three per
-    field for its six Hessians, FP64 six; the five pair products' x passes are
-    their truncations), 10 product sums through the padded r2c (z and y passes;
+    17 operands through the padded c2r (y and z passes; three x passes
+    per field for its six Hessians; the five pair products' x passes are their
+    truncations), 10 product sums through the padded r2c (z and y passes;
     x passes of five, and the five truncations), the streaming source products,
     and the assembly of `overload` sub-lattices for positions and velocities."""
     cs = 2 * prec_bytes
@@ -149,7 +149,7 @@ def algorithmic_bytes_ic(n: int, prec_bytes: int, overload: int = 2, plt: bool =
     S_N = n * n * (n + 2) * prec_bytes  # N-grid
     npart = overload * n ** 3
     out = {
-        "conv_xinv": (6 if prec_bytes == 4 else 12) * (S_NK + S_MNK),
+        "conv_xinv": 6 * (S_NK + S_MNK),
         "conv_yinv": 17 * (S_MNK + S_MMK),
         "conv_z": 27 * (S_MMK + S_R),
         "conv_yfwd": 10 * (S_MMK + S_MNK),

@@ -545,49 +545,13 @@ int shared_sources(mf_ic* ic, bool timed) {
   };
   // The six padded Hessians of field fi into real fields base + 0..5, in the
   // order (0,0) (1,1) (2,2) (0,1) (0,2) (1,2).
-  // FP64: two passes of three operands.
-  auto hessians6 = [&](int fi, int base) -> cudaError_t {
-    const int HD[6][2] = {{0, 0}, {1, 1}, {2, 2}, {0, 1}, {0, 2}, {1, 2}};
-    for (int half = 0; half < 2; ++half) {
-      ConvXInvOp<T> xo{};
-      ConvYInvOp<T> yo{};
-      for (int k = 0; k < 3; ++k) {
-        xo.opnd[k] = Operand<T>{};
-        xo.opnd[k].f = (const cplx<T>*)ic->f[fi]->d;
-        xo.opnd[k].kind = OPND_HESS;
-        xo.opnd[k].d[0] = HD[3 * half + k][0];
-        xo.opnd[k].d[1] = HD[3 * half + k][1];
-        xo.dst[k] = W[k];
-        yo.src[k] = W[k];
-        yo.dst[k] = W[k];
-      }
-      xo.g = g;
-      xo.kfac = kfac;
-      xo.scale = scale_in;
-      yo.g = g;
-      cudaError_t e2;
-      {
-        LaunchScope ls(c, KK_CONV_XINV);
-        if ((e2 = Launch<T>::conv_xinv(M, xo, N, Kz, 3, twM, s)) != cudaSuccess) return e2;
-      }
-      {
-        LaunchScope ls(c, KK_CONV_YINV);
-        if ((e2 = Launch<T>::conv_yinv(M, yo, M, Kz, 3, twM, s)) != cudaSuccess) return e2;
-      }
-      for (int k = 0; k < 3; ++k)
-        if ((e2 = z_c2r(W[k], base + 3 * half + k)) != cudaSuccess) return e2;
-    }
-    return cudaSuccess;
-  };
-  // FP32: along an x column only g_x varies, so three x transforms serve all
-  // six: of f, i g_x f and -g_x^2 f; the other factors are constant on the column
-  // and multiply it on the way into the y pass.  The x pass so writes three
-  // padded grids instead of six (3LPT runs: 61.9 -> 59.4 ms at N=512 BCC, 7.05 ->
-  // 6.77 at 256).  Fields that are still to be written hold what the three work
-  // buffers cannot.  In FP64 the factors on the y rows, half as many again as
-  // the x rows, cost what the transforms save (N=256 32.4 -> 32.0 ms, N=64 2LPT
-  // 0.68-0.72 -> 0.73 ms).
-  auto hessians3 = [&](int fi, int base) -> cudaError_t {
+  // Along an x column only g_x varies, so three x transforms serve all six: of
+  // f, i g_x f and -g_x^2 f; the other factors are constant on the column and
+  // multiply it on the way into the y pass.  The x pass so writes three padded
+  // grids instead of six (3LPT runs: FP32 61.9 -> 59.4 ms at N=512 BCC, 7.05 ->
+  // 6.77 at 256, 0.597 -> 0.577 at 64; FP64 32.4 -> 31.9 at 256).  Fields that are
+  // still to be written hold what the three work buffers cannot.
+  auto hessians = [&](int fi, int base) -> cudaError_t {
     ConvXInvOp<T> xo{};
     for (int k = 0; k < 3; ++k) {
       xo.opnd[k] = Operand<T>{};
@@ -631,10 +595,6 @@ int shared_sources(mf_ic* ic, bool timed) {
         if ((e2 = z_c2r(ps[k].dst, ps[k].field)) != cudaSuccess) return e2;
     }
     return cudaSuccess;
-  };
-
-  auto hessians = [&](int fi, int base) -> cudaError_t {
-    return sizeof(T) == 4 ? hessians3(fi, base) : hessians6(fi, base);
   };
 
   // convolve3's first stage for one pair product held as a padded real field:

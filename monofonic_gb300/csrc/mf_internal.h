@@ -67,7 +67,7 @@ struct Launch {
                                const cplx<T>* tw, cudaStream_t s);
   static cudaError_t conv_yinv(int L, ConvYInvOp<T> op, int nslab, int ncols, int nops,
                                const cplx<T>* tw, cudaStream_t s);
-  // (FP32, Orszag lengths)
+  // (Orszag lengths)
   static cudaError_t conv_yhess(int L, ConvYHessOp<T> op, int nslab, int ncols, int nops, const cplx<T>* tw,
                                 cudaStream_t s);
   static cudaError_t conv_yfwd(int L, ConvYFwdOp<T> op, int nslab, int ncols, const cplx<T>* tw,

@@ -475,7 +475,7 @@ cudaError_t Launch<T>::conv_yhess(int L, ConvYHessOp<T> op, int nslab, int ncols
                                   cudaStream_t s) {
 #define CASE(LL)                                                                                        \
   case LL:                                                                                             \
-    if constexpr (sizeof(T) == 4 && orszag_len(LL)) {                                                  \
+    if constexpr (orszag_len(LL)) {                                                                    \
       using G = CGeom<LL, true>;                                                                       \
       if (!geom_matches<G>(op.g)) return cudaErrorInvalidValue;                                        \
       return launch_col<T, LL, true>(op.template with_geom<G>(), nslab, ncols, nops, tw, s, KK_CONV_YINV); \

@@ -299,7 +299,7 @@ struct ConvYHessOp {
     const C* s0 = z == 0 ? src[0] : (z == 1 ? src[1] : src[2]);
     return s0 + ((long long)x * g.M * g.Kz + kz) + g.row_off(y, g.Kz);
   }
-  // the factor c0 + c1 g_y + c2 g_y^2 of a column, times i if grad
+  // the factor c0 + c1 m + c2 m^2 of a column, m = g_y / kfac, times i if grad
   struct Tile {
     T c0, c1, c2;
     bool grad;
@@ -311,12 +311,15 @@ struct ConvYHessOp {
     T f = p + q == 2 ? T(-1) : T(1);
     if (q > 0) f *= gk;
     if (q > 1) f *= gk;
-    return Tile{p == 0 ? f : T(0), p == 1 ? f : T(0), p == 2 ? f : T(0), p + q == 1};
+    return Tile{p == 0 ? f : T(0), p == 1 ? f * kfac : T(0), p == 2 ? f * kfac * kfac : T(0), p + q == 1};
   }
   template <class I>
   __device__ __forceinline__ C xform_tile(const Tile& t, I y, C v0) const {
-    const T gj = G::template row_comp<T>(y) * kfac;
-    const T f = (t.c2 * gj + t.c1) * gj + t.c0;
+    T f = t.c0;
+    if (sizeof(T) == 4 || t.c1 != T(0) || t.c2 != T(0)) {  // (as in ConvXInvOp)
+      const T gj = G::template row_comp<T>(y);
+      f = (t.c2 * gj + t.c1) * gj + t.c0;
+    }
     return t.grad ? mkc<T>(-f * v0.y, f * v0.x) : mkc<T>(v0.x * f, v0.y * f);
   }
   template <class I>
