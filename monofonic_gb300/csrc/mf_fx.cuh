@@ -17,7 +17,7 @@
 // ~1.4 2^-53.
 //
 // Measured (N=256, FP64): z c2r of a padded operand 1734 -> 386 us, y c2r 1000
-// -> 262 us per operand, a 3LPT run 114.0 -> 35.0 ms (32.4 with the cheaper
+// -> 262 us per operand, a 3LPT run 114.0 -> 35.0 ms (31.9 with the cheaper
 // operand factors and sources since); a forward transform of
 // white noise is 1.1e-16 (N=256) and 1.7e-16 (N=384) off in relative L2, FP64
 // butterflies were 3.2e-16 and 3.3e-16 off.  What bounds it now is instruction
