@@ -325,7 +325,10 @@ __device__ __forceinline__ int col_fx(double2* tile, int t, int c, const double2
   return xs;
 }
 
-// norm of each line of a contiguous-line pass, TPL threads per line
+// norm of each line of a contiguous-line pass, TPL threads per line, to all of
+// them.  Summed in an order that is fixed by the line alone: the sum decides the
+// scale, so another order could round every output of the line differently.
+// (At most 256 threads per CTA; the callers have a barrier between two calls.)
 template <int TPL, class SYNC>
 __device__ __forceinline__ fx::Norm line_norm(fx::Norm n, int t, int lg, SYNC sync) {
   if constexpr (std::is_same<SYNC, SyncWarp>::value) {
@@ -335,15 +338,15 @@ __device__ __forceinline__ fx::Norm line_norm(fx::Norm n, int t, int lg, SYNC sy
   } else {
     __shared__ float l1[256];
     __shared__ int mx[256];
-    sync();
-    if (t == 0) { l1[lg] = 0.f; mx[lg] = 0; }
-    sync();
-    atomicAdd(&l1[lg], n.l1);
-    atomicMax(&mx[lg], n.mx);
+    l1[lg * TPL + t] = n.l1;
+    mx[lg * TPL + t] = n.mx;
     sync();
     fx::Norm r;
-    r.l1 = l1[lg];
-    r.mx = mx[lg];
+#pragma unroll
+    for (int i = 0; i < TPL; ++i) {
+      r.l1 += l1[lg * TPL + i];
+      r.mx = max(r.mx, mx[lg * TPL + i]);
+    }
     return r;
   }
 }
