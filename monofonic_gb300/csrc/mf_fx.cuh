@@ -352,16 +352,21 @@ __device__ __forceinline__ fx::Norm line_norm(fx::Norm n, int t, int lg, SYNC sy
 }
 
 // a staged half-complex line (kin values, kz >= kin zero) to fixed point in
-// place; returns its scale
+// place; returns its scale.  A c2r ignores the imaginary parts of kz = 0 and
+// kz = H, however large they are: they count in neither the norm nor the
+// transform.
 template <int H, int TPL, class SYNC>
 __device__ __forceinline__ int c2r_line_to_fx(double2* src, int kin, int t, int lg, SYNC sync) {
   fx::Norm n;
 #pragma unroll 2
-  for (int k = t; k < kin; k += TPL) n.add(src[k]);
+  for (int k = t; k < kin; k += TPL) {
+    double2 v = src[k];
+    if (k == 0 || k == H) v.y = 0.0;
+    n.add(v);
+  }
   n = line_norm<TPL>(n, t, lg, sync);
   // inputs of the transform are E + iO: at most twice the moduli of two terms each
   const int xs = fx::scale(n.l1, n.mx, fx::ceil_log2(H), 2);
-  // the imaginary parts of kz = 0 and kz = H do not count
 #pragma unroll 2
   for (int k = t; k < kin; k += TPL) {
     longlong2 q = fx::from_c(src[k], xs);

@@ -60,3 +60,39 @@ def test_batch_equals_standalone(ctx, n):
         for i, r in enumerate(reqs):
             assert _same(b.particles(i), _standalone(ctx, r)), i
     b.close()
+
+
+@pytest.mark.parametrize("n", [16, 32, 96, 256])
+@pytest.mark.parametrize("size", [1e12, 1e200])
+def test_dropped_imaginary_parts_do_not_count(ctx, n, size):
+    """A c2r ignores the imaginary parts of its lines' kz = 0 and, unless the
+    lines are padded, kz = N/2 values, so however large they are the result
+    keeps every bit.  The modes (0, 0, 0) and (0, 0, N/2) have columns of their
+    own."""
+    import monofonic_gb300 as mf
+    L = 50.0
+    rng = np.random.default_rng(n)
+    s = rng.standard_normal((n, n, n // 2 + 1)) + 1j * rng.standard_normal((n, n, n // 2 + 1))
+    s[:, :, 0] = 0
+    s[:, :, n // 2] = 0
+    g = mf.Grid_FFT(ctx, n, L, "f64", "k")
+    h = mf.Grid_FFT(ctx, n, L, "f64", "k")
+    out = mf.Grid_FFT(ctx, n, L, "f64", "k")
+    padded, aliased = mf.OrszagConvolver(ctx, n, L, "f64"), mf.NaiveConvolver(ctx, n, L, "f64")
+    h.set_k(s)
+    res = []
+    for im in (0.0, size):
+        one = []
+        s[0, 0, 0] = 1j * im
+        g.set_k(s)
+        padded.multiply_field(g, h, mf.op.assign_to(out))
+        one.append(out.get_k())
+        s[0, 0, n // 2] = 1j * im
+        g.set_k(s)
+        aliased.multiply_field(g, h, mf.op.assign_to(out))
+        one.append(out.get_k())
+        g.FourierTransformBackward()
+        one.append(g.get_real())
+        res.append(one)
+    for a, b in zip(*res):
+        assert np.array_equal(a, b)
