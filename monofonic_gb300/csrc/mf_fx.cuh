@@ -26,7 +26,7 @@
 // Lines holding an infinity or a NaN come out NaN.  A line whose norm is
 // outside the float range that the bound is summed in takes its scale from
 // its largest exponent (the bound is then L times that value), and extreme
-// results are scaled by FP64 products.  Subnormal inputs count as zeros.
+// results are scaled by FP64 products.
 #pragma once
 
 #include <cmath>
@@ -102,21 +102,23 @@ __device__ __forceinline__ int scale(float l1, int maxhi, int len_bits, int grow
     const int X = (__float_as_int(l1 * 1.015625f) >> 23) - 126;
     return 62 - grow - X;
   }
-  const int e = max(maxhi >> 20, 1);
+  // every value below 2^(e-1022), subnormal ones among them
+  int e = maxhi >> 20;
   if (e == 0x7ff) return kNan;
+  if (e == 0) e = max(12 - __clz(maxhi), -(grow + len_bits));  // (xs <= 1083: from_double)
   return 62 - grow - (e - 1022 + 1 + len_bits);
 }
 
-// round(x 2^xs) for |x| 2^xs < 2^62, subnormal x as zero
+// round(x 2^xs) for |x| 2^xs < 2^62, xs <= 1083
 __device__ __forceinline__ long long from_double(double x, int xs) {
-  const int hi = __double2hiint(x);
+  const int hi = __double2hiint(x), h = hi & 0x7fffffff;
   const unsigned lo = (unsigned)__double2loint(x);
-  // the 53-bit mantissa at bits 10..62, shifted right to twice the value (a
-  // count of 64 or more leaves 0)
-  const unsigned mh = (((unsigned)hi & 0xfffffu) | 0x100000u) << 10 | (lo >> 22);
+  // |x| = m 2^(e-1084) for the 53-bit mantissa m at bits 10..62 (normal or, e = 0,
+  // subnormal), shifted right to twice the value (a count of 64 or more leaves 0)
+  const int e = max((h >> 20) - 1, 0);
+  const unsigned mh = __funnelshift_l(lo, (unsigned)(h - (e << 20)), 10);
   const unsigned long long m = ((unsigned long long)mh << 32) | (lo << 10);
-  const int e = (hi >> 20) & 0x7ff;
-  const unsigned r = e ? (unsigned)(1084 - xs - e) : 64u;
+  const unsigned r = (unsigned)(1083 - xs - e);
   unsigned long long q;
   asm("shr.u64 %0, %1, %2;" : "=l"(q) : "l"(m), "r"(r));
   const long long s = (long long)(hi >> 31);

@@ -96,3 +96,25 @@ def test_dropped_imaginary_parts_do_not_count(ctx, n, size):
         res.append(one)
     for a, b in zip(*res):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [16, 96, 128])
+@pytest.mark.parametrize("shift", [-1030, -1060])
+def test_subnormal_values_count(ctx, n, shift):
+    """A field of subnormal values is transformed like any other.  Every pass
+    rounds its results to the subnormal spacing 2^-1074: half of it per
+    component, at the last pass (the earlier ones' grow less than the values)
+    2^-1075 sqrt(2) of a field of r.m.s. 2^shift; four times that is allowed."""
+    import monofonic_gb300 as mf
+    x = np.ldexp(np.random.default_rng(n).standard_normal((n, n, n)), shift)
+    g = mf.Grid_FFT(ctx, n, 1.0, "f64")
+    g.set_real(x)
+    g.FourierTransformForward()
+    k = g.get_k()
+    up = np.ldexp(k.real, -shift) + 1j * np.ldexp(k.imag, -shift)
+    want = np.fft.rfftn(np.ldexp(x, -shift)) / np.sqrt(float(n) ** 3)
+    tol = 4e-15 + 4 * np.sqrt(2.0) * np.ldexp(1.0, -1075 - shift)
+    assert np.linalg.norm(up - want) <= tol * np.linalg.norm(want)
+    g.FourierTransformBackward()
+    back = np.ldexp(g.get_real(), -shift)
+    assert np.linalg.norm(back - np.ldexp(x, -shift)) <= 2 * tol * np.linalg.norm(np.ldexp(x, -shift))
