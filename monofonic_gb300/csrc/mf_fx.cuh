@@ -23,10 +23,10 @@
 // butterflies were 3.2e-16 and 3.3e-16 off.  What bounds it now is instruction
 // issue: ~100 instructions per element in the butterflies, ~100 in conversions.
 //
-// Lines holding an infinity or a NaN come out NaN.  A line whose norm is
-// outside the float range that the bound is summed in takes its scale from
-// its largest exponent (the bound is then L times that value), and extreme
-// results are scaled by FP64 products.
+// Lines holding an infinity or a NaN come out NaN.  The norm of a line outside
+// the float range that it is summed in is summed again relative to its largest
+// exponent, and extreme results are scaled by FP64 products: like FP64
+// arithmetic, the transform commutes with powers of two.
 #pragma once
 
 #include <cmath>
@@ -84,28 +84,63 @@ __device__ __forceinline__ long long mulc(long long a, int ch, int cl) {
   return join(wide(ah, ch), mad(ah, cl, mad(al, ch, 1ll << 29)));
 }
 
-// upper bound of |x| as a float: the exponent rebased and the mantissa
-// rounded up; 0 below the float range, infinity or NaN above it
-__device__ __forceinline__ float mag(int hi_abs) {
-  int h = hi_abs - (896 << 20);
+// upper bound of |x| 2^(896-off) as a float: the exponent rebased and the
+// mantissa rounded up; 0 below the float range, infinity or NaN above it
+__device__ __forceinline__ float mag(int hi_abs, int off = 896) {
+  int h = hi_abs - off * 0x100000;
   h = max(h, 0);
   h = min(h, 0x0ff00000);
   return __int_as_float((h << 3) + 8);
 }
 __device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
 
-// scale of a line from the bound of its L1 norm and its largest high word;
-// grow: bits of growth of the processing around the transform
-__device__ __forceinline__ int scale(float l1, int maxhi, int len_bits, int grow) {
-  if (l1 > 0x1p-100f && l1 < 0x1p120f) {
+// bound of a line: sum of the components' magnitudes times 2^-base, largest high word
+struct Norm {
+  float l1 = 0.f;
+  int mx = 0;
+  int base = 0;
+  __device__ __forceinline__ void add(double2 v) {
+    const int a = hi_abs(v.x), b = hi_abs(v.y);
+    l1 += mag(a) + mag(b);
+    mx = max(mx, max(a, b));
+  }
+  __device__ __forceinline__ void add(const Norm& o) {
+    l1 += o.l1;
+    mx = max(mx, o.mx);
+  }
+  __device__ __forceinline__ Norm shfl_xor(int o) const {
+    Norm r;
+    r.l1 = __shfl_xor_sync(0xffffffffu, l1, o);
+    r.mx = __shfl_xor_sync(0xffffffffu, mx, o);
+    return r;
+  }
+  __device__ __forceinline__ bool in_range() const { return l1 > 0x1p-100f && l1 < 0x1p120f; }
+  // whether the magnitudes are to be summed again relative to the largest
+  // exponent; of a part of a line: if no part's are, the whole is in range
+  __device__ __forceinline__ bool sum_again() const { return mx != 0 && !(l1 > 0x1p-100f && l1 < 0x1p110f); }
+  // the rebasing of that sum; the magnitudes of an exponent mx are then in [1, 2]
+  __device__ __forceinline__ int rebased() const { return (mx >> 20) - 127; }
+  // its result; lines of subnormal or with non-finite values keep theirs
+  __device__ __forceinline__ void set_rebased(float sum) {
+    const int e = mx >> 20;
+    if (in_range() || e == 0 || e == 0x7ff) return;
+    l1 = sum;
+    base = e - 1023;
+  }
+};
+
+// scale of a line from its norm; grow: bits of growth of the processing around
+// the transform
+__device__ __forceinline__ int scale(const Norm& n, int len_bits, int grow) {
+  if (n.in_range()) {
     // l1 (1 + 2^-6) < 2^X covers the rounding of the float sum
-    const int X = (__float_as_int(l1 * 1.015625f) >> 23) - 126;
-    return 62 - grow - X;
+    const int X = (__float_as_int(n.l1 * 1.015625f) >> 23) - 126;
+    return 62 - grow - X - n.base;
   }
   // every value below 2^(e-1022), subnormal ones among them
-  int e = maxhi >> 20;
+  int e = n.mx >> 20;
   if (e == 0x7ff) return kNan;
-  if (e == 0) e = max(12 - __clz(maxhi), -(grow + len_bits));  // (xs <= 1083: from_double)
+  if (e == 0) e = max(12 - __clz(n.mx), -(grow + len_bits));  // (xs <= 1083: from_double)
   return 62 - grow - (e - 1022 + 1 + len_bits);
 }
 
@@ -155,27 +190,6 @@ __device__ __forceinline__ longlong2 from_c(double2 v, int xs) {
 __device__ __forceinline__ double2 to_c(longlong2 v, int xs) {
   return make_double2(to_double(v.x, xs), to_double(v.y, xs));
 }
-
-// running bound of a line: sum of the components' magnitudes, largest high word
-struct Norm {
-  float l1 = 0.f;
-  int mx = 0;
-  __device__ __forceinline__ void add(double2 v) {
-    const int a = hi_abs(v.x), b = hi_abs(v.y);
-    l1 += mag(a) + mag(b);
-    mx = max(mx, max(a, b));
-  }
-  __device__ __forceinline__ void add(const Norm& o) {
-    l1 += o.l1;
-    mx = max(mx, o.mx);
-  }
-  __device__ __forceinline__ Norm shfl_xor(int o) const {
-    Norm r;
-    r.l1 = __shfl_xor_sync(0xffffffffu, l1, o);
-    r.mx = __shfl_xor_sync(0xffffffffu, mx, o);
-    return r;
-  }
-};
 
 __host__ __device__ constexpr int ceil_log2(int n) {
   int b = 0;
@@ -265,13 +279,30 @@ __device__ __forceinline__ const longlong2* fx_table(const double2* tw) {
   return reinterpret_cast<const longlong2*>(tw + L);
 }
 
-// norm of each column of a strided tile, block (NCOL, TPL), to all its threads
-template <int NCOL, int TPL>
-__device__ __forceinline__ fx::Norm col_norm(fx::Norm n, int t, int c) {
+// partial norms that the threads of a CTA exchange: one block of shared memory
+// per kernel, however many transforms it has (a second one cost the fused z pass
+// at H = 144 a CTA per SM, 6 % of five products at 192^3)
+template <int COUNT>
+struct NormParts {
+  float l1[COUNT];
+  int mx[COUNT];
+};
+template <int COUNT>
+__device__ __forceinline__ NormParts<COUNT>& norm_parts() {
+  __shared__ NormParts<COUNT> p;
+  return p;
+}
+
+// norm of each column of a strided tile, block (NCOL, TPL), to all its threads.
+// each(f) calls f with every value of the thread.
+template <int NCOL, int TPL, class EACH>
+__device__ __forceinline__ fx::Norm col_norm(int t, int c, EACH each) {
   constexpr bool WARP = NCOL < 32;  // a warp holds 32 / NCOL elements of a column
   constexpr int ROWS = WARP ? (NCOL * TPL + 31) / 32 : TPL;
-  __shared__ float l1[ROWS * NCOL];
-  __shared__ int mx[ROWS * NCOL];
+  float* l1 = norm_parts<ROWS * NCOL>().l1;
+  int* mx = norm_parts<ROWS * NCOL>().mx;
+  fx::Norm n;
+  each([&](double2 v) { n.add(v); });
   if constexpr (WARP) {
 #pragma unroll
     for (int o = NCOL; o < 32; o <<= 1) n.add(n.shfl_xor(o));
@@ -279,12 +310,26 @@ __device__ __forceinline__ fx::Norm col_norm(fx::Norm n, int t, int c) {
   const int row = WARP ? (t * NCOL + c) >> 5 : t;
   l1[row * NCOL + c] = n.l1;  // (a warp's lanes of one column write the same values)
   mx[row * NCOL + c] = n.mx;
-  __syncthreads();
+  const bool again = __syncthreads_or(n.sum_again());
   fx::Norm r;
 #pragma unroll 8
   for (int i = 0; i < ROWS; ++i) {
     r.l1 += l1[i * NCOL + c];
     r.mx = max(r.mx, mx[i * NCOL + c]);
+  }
+  if (again) {
+    float s = 0.f;
+    each([&](double2 v) { s += fx::mag(fx::hi_abs(v.x), r.rebased()) + fx::mag(fx::hi_abs(v.y), r.rebased()); });
+    if constexpr (WARP) {
+#pragma unroll
+      for (int o = NCOL; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    }
+    __syncthreads();  // the first sums have been read
+    l1[row * NCOL + c] = s;
+    __syncthreads();
+    s = 0.f;
+    for (int i = 0; i < ROWS; ++i) s += l1[i * NCOL + c];
+    r.set_rebased(s);
   }
   return r;
 }
@@ -313,11 +358,11 @@ __device__ __forceinline__ void col_fx_run(longlong2* tile, int t, int c, const 
 template <class F, int NCOL>
 __device__ __forceinline__ int col_fx(double2* tile, int t, int c, const double2* tw) {
   longlong2* tx = reinterpret_cast<longlong2*>(tile);
-  fx::Norm n;
+  const fx::Norm n = col_norm<NCOL, F::TPL>(t, c, [&](auto f) {
 #pragma unroll 2
-  for (int i = 0; i < F::E; ++i) n.add(tile[tile_slot<F, NCOL>(t, i) + c]);
-  n = col_norm<NCOL, F::TPL>(n, t, c);
-  const int xs = fx::scale(n.l1, n.mx, fx::ceil_log2(F::LEN), 0);
+    for (int i = 0; i < F::E; ++i) f(tile[tile_slot<F, NCOL>(t, i) + c]);
+  });
+  const int xs = fx::scale(n, fx::ceil_log2(F::LEN), 0);
 #pragma unroll 2
   for (int i = 0; i < F::E; ++i) {
     const int o = tile_slot<F, NCOL>(t, i) + c;
@@ -331,23 +376,45 @@ __device__ __forceinline__ int col_fx(double2* tile, int t, int c, const double2
 // them.  Summed in an order that is fixed by the line alone: the sum decides the
 // scale, so another order could round every output of the line differently.
 // (At most 256 threads per CTA; the callers have a barrier between two calls.)
-template <int TPL, class SYNC>
-__device__ __forceinline__ fx::Norm line_norm(fx::Norm n, int t, int lg, SYNC sync) {
+template <int TPL, class SYNC, class EACH>
+__device__ __forceinline__ fx::Norm line_norm(int t, int lg, SYNC sync, EACH each) {
+  fx::Norm n;
+  each([&](double2 v) { n.add(v); });
+  auto again = [&](const fx::Norm& m) {
+    float s = 0.f;
+    each([&](double2 v) { s += fx::mag(fx::hi_abs(v.x), m.rebased()) + fx::mag(fx::hi_abs(v.y), m.rebased()); });
+    return s;
+  };
   if constexpr (std::is_same<SYNC, SyncWarp>::value) {
 #pragma unroll
     for (int o = 1; o < TPL; o <<= 1) n.add(n.shfl_xor(o));
+    if (__any_sync(0xffffffffu, n.sum_again())) {
+      float s = again(n);
+#pragma unroll
+      for (int o = 1; o < TPL; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      n.set_rebased(s);
+    }
     return n;
   } else {
-    __shared__ float l1[256];
-    __shared__ int mx[256];
+    float* l1 = norm_parts<256>().l1;
+    int* mx = norm_parts<256>().mx;
     l1[lg * TPL + t] = n.l1;
     mx[lg * TPL + t] = n.mx;
-    sync();
+    const bool any = __syncthreads_or(n.sum_again());
     fx::Norm r;
 #pragma unroll
     for (int i = 0; i < TPL; ++i) {
       r.l1 += l1[lg * TPL + i];
       r.mx = max(r.mx, mx[lg * TPL + i]);
+    }
+    if (any) {
+      const float s = again(r);
+      sync();  // the first sums have been read
+      l1[lg * TPL + t] = s;
+      sync();
+      float sum = 0.f;
+      for (int i = 0; i < TPL; ++i) sum += l1[lg * TPL + i];
+      r.set_rebased(sum);
     }
     return r;
   }
@@ -359,16 +426,16 @@ __device__ __forceinline__ fx::Norm line_norm(fx::Norm n, int t, int lg, SYNC sy
 // transform.
 template <int H, int TPL, class SYNC>
 __device__ __forceinline__ int c2r_line_to_fx(double2* src, int kin, int t, int lg, SYNC sync) {
-  fx::Norm n;
+  const fx::Norm n = line_norm<TPL>(t, lg, sync, [&](auto f) {
 #pragma unroll 2
-  for (int k = t; k < kin; k += TPL) {
-    double2 v = src[k];
-    if (k == 0 || k == H) v.y = 0.0;
-    n.add(v);
-  }
-  n = line_norm<TPL>(n, t, lg, sync);
+    for (int k = t; k < kin; k += TPL) {
+      double2 v = src[k];
+      if (k == 0 || k == H) v.y = 0.0;
+      f(v);
+    }
+  });
   // inputs of the transform are E + iO: at most twice the moduli of two terms each
-  const int xs = fx::scale(n.l1, n.mx, fx::ceil_log2(H), 2);
+  const int xs = fx::scale(n, fx::ceil_log2(H), 2);
 #pragma unroll 2
   for (int k = t; k < kin; k += TPL) {
     longlong2 q = fx::from_c(src[k], xs);
@@ -383,11 +450,11 @@ __device__ __forceinline__ int c2r_line_to_fx(double2* src, int kin, int t, int 
 // returns its scale (the post-processing doubles the values)
 template <int H, int TPL, int LIN, class SYNC>
 __device__ __forceinline__ int r2c_line_to_fx(double2* src, int t, int lg, SYNC sync) {
-  fx::Norm n;
+  const fx::Norm n = line_norm<TPL>(t, lg, sync, [&](auto f) {
 #pragma unroll 2
-  for (int k = t; k < H; k += TPL) n.add(src[pidx<LIN>(k)]);
-  n = line_norm<TPL>(n, t, lg, sync);
-  const int xs = fx::scale(n.l1, n.mx, fx::ceil_log2(H), 1);
+    for (int k = t; k < H; k += TPL) f(src[pidx<LIN>(k)]);
+  });
+  const int xs = fx::scale(n, fx::ceil_log2(H), 1);
 #pragma unroll 2
   for (int k = t; k < H; k += TPL)
     reinterpret_cast<longlong2*>(src)[pidx<LIN>(k)] = fx::from_c(src[pidx<LIN>(k)], xs);

@@ -118,3 +118,37 @@ def test_subnormal_values_count(ctx, n, shift):
     g.FourierTransformBackward()
     back = np.ldexp(g.get_real(), -shift)
     assert np.linalg.norm(back - np.ldexp(x, -shift)) <= 2 * tol * np.linalg.norm(np.ldexp(x, -shift))
+
+
+@pytest.mark.parametrize("n", [16, 32, 96, 128, 192])
+@pytest.mark.parametrize("kind", ["white", "spike", "lines"])
+def test_powers_of_two_factor_out(ctx, n, kind):
+    """Values times a power of two give results times that power, bit for bit,
+    as FP64 arithmetic does: the scale follows the line's norm however far it
+    is from 1, and whatever the lines beside it hold."""
+    import monofonic_gb300 as mf
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, n, n))
+    if kind == "spike":
+        x = np.zeros((n, n, n))
+        x[3, n // 2, n - 1], x[1, 2, 3] = -1.7, 0.3
+    elif kind == "lines":  # neighbouring lines 2^-100 .. 2^100 apart
+        x = np.ldexp(x, rng.integers(-100, 101, size=(n, n, 1)))
+    g = mf.Grid_FFT(ctx, n, 1.0, "f64")
+    h, out = mf.Grid_FFT(ctx, n, 1.0, "f64", "k"), mf.Grid_FFT(ctx, n, 1.0, "f64", "k")
+    cv = mf.OrszagConvolver(ctx, n, 1.0, "f64")
+
+    def run(shift):
+        g.set_real(np.ldexp(x, shift))
+        g.FourierTransformForward()
+        k = g.get_k()
+        h.set_k(np.ldexp(k.real, -shift // 2) + 1j * np.ldexp(k.imag, -shift // 2))
+        cv.multiply_field(h, h, mf.op.assign_to(out))
+        p = out.get_k()
+        g.FourierTransformBackward()
+        return [np.ldexp(a, -shift) for a in (k.real, k.imag, g.get_real(), p.real, p.imag)]
+
+    want = run(0)
+    for shift in (-400, -130, -104, 120, 400):
+        for a, b in zip(run(shift), want):
+            assert np.array_equal(a, b), shift
