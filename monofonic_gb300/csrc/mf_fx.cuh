@@ -8,19 +8,30 @@
 //
 // Scale.  Every value inside an unnormalised DFT is a sum of inputs times
 // phases, so its modulus is at most the line's L1 norm.  xs places an upper
-// bound of that norm at 2^62 (less the growth of a pre- or post-processing
-// step), so nothing overflows and no stage needs a shift.  The error: each
-// conversion and each product is rounded to half a unit of 2^-xs, which over
-// a transform of length L leaves ~0.4 L^(1/2) units; with |x|_1 <= L^(1/2)
-// |x|_2 that is at most ~0.4 L 2^-62 of the output's r.m.s. (0.6 2^-53 at
-// L = 768, less for lines dominated by few values), where FP64 rounding leaves
-// ~1.4 2^-53.
+// bound of that norm (moduli as max + 0.4142 min of the components, at most 8 %
+// too large) at 1.3125 2^62, less the growth of a pre- or post-processing step:
+// the sums of two components inside radix 8 stay below 2^63 then, so nothing
+// overflows and no stage needs a shift.  xs is lower where a single value would
+// pass 2^62.
 //
-// Measured (N=256, FP64): z c2r of a padded operand 1734 -> 386 us, y c2r 1000
-// -> 262 us per operand, a 3LPT run 114.0 -> 35.0 ms (31.9 with the cheaper
-// operand factors and sources since); a forward transform of
-// white noise is 1.1e-16 (N=256) and 1.7e-16 (N=384) off in relative L2, FP64
-// butterflies were 3.2e-16 and 3.3e-16 off.  What bounds it now is instruction
+// Error.  In units of 2^-xs a conversion is off by at most 1/2, a twiddle
+// product by 0.55 r.m.s. and at most 2.3 (the rounding and two products of low
+// words that are left out), a product with sqrt(3)/2 by at most 1.12.  The
+// largest terms are the conversions of a long line: a unit is 2^-62 to 2^-61 of
+// the L1 norm, which for L white values is 1.25 L of one's r.m.s.; the one or two
+// bits of growth of the real transforms make it two or four times as large.
+// Measured, relative L2 of a product with a field of one mode, the largest of
+// eight amplitudes, and what FP64 butterflies left: N=64 1.3e-16 / 3.1e-16, 128
+// 3.8 / 5.1, 256 1.3 / 3.5, 384 2.2 / 3.9, 512 (L = 768) 5.4 / 5.9.  With the norm
+// from |re| + |im| at 2^62 it was 7.1e-16 at N=512, more than the butterflies.
+//
+// Forward transforms of white values against extended precision: 0.9e-16 at
+// N=256, 1.0e-16 at 384, 1.4e-16 at 512, where FP64 butterflies are 3.6e-16, 2.8e-16
+// and 3.3e-16 off.
+//
+// Time (N=256, FP64): z c2r of a padded operand 1734 -> 386 us, y c2r 1000
+// -> 262 us per operand, a 3LPT run 114.0 -> 35.0 ms (32.0 with the cheaper
+// operand factors and sources since).  What bounds it now is instruction
 // issue: ~100 instructions per element in the butterflies, ~100 in conversions.
 //
 // Lines holding an infinity or a NaN come out NaN.  The norm of a line outside
@@ -76,8 +87,8 @@ __device__ __forceinline__ long long join(long long h, long long m) {
   const unsigned hi = __funnelshift_l((unsigned)lo32(u), (unsigned)hi32(u), 2);
   return (long long)(((unsigned long long)hi << 32) | lo);
 }
-// round(a c / 2^62) for a constant c in Q62, |a| < 2^62.5 (the product of the
-// low words, below half a unit, is left out: both are signed)
+// a c / 2^62 rounded, for a constant c in Q62, |a| < 2^63 (the product of the
+// low words, up to 0.62 units at sqrt(3)/2, is left out: both are signed)
 __device__ __forceinline__ long long mulc(long long a, int ch, int cl) {
   int ah, al;
   split(a, ah, al);
@@ -94,15 +105,24 @@ __device__ __forceinline__ float mag(int hi_abs, int off = 896) {
 }
 __device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
 
-// bound of a line: sum of the components' magnitudes times 2^-base, largest high word
+// bound of the modulus from the components' high words, a >= b
+__device__ __forceinline__ float modulus(int a, int b, int off = 896) {
+  return fmaf(mag(b, off), 0.41421357f, mag(a, off));  // sqrt(2) - 1, rounded up
+}
+// bound of a line: sum of the moduli times 2^-base, largest high word
 struct Norm {
   float l1 = 0.f;
   int mx = 0;
   int base = 0;
   __device__ __forceinline__ void add(double2 v) {
+    const int a = hi_abs(v.x), b = hi_abs(v.y), m = max(a, b);
+    l1 += modulus(m, min(a, b));
+    mx = max(mx, m);
+  }
+  // term of the sum relative to the largest exponent (of this, the line's norm)
+  __device__ __forceinline__ float rebased(double2 v) const {
     const int a = hi_abs(v.x), b = hi_abs(v.y);
-    l1 += mag(a) + mag(b);
-    mx = max(mx, max(a, b));
+    return modulus(max(a, b), min(a, b), (mx >> 20) - 127);
   }
   __device__ __forceinline__ void add(const Norm& o) {
     l1 += o.l1;
@@ -115,12 +135,10 @@ struct Norm {
     return r;
   }
   __device__ __forceinline__ bool in_range() const { return l1 > 0x1p-100f && l1 < 0x1p120f; }
-  // whether the magnitudes are to be summed again relative to the largest
+  // whether the moduli are to be summed again relative to the largest
   // exponent; of a part of a line: if no part's are, the whole is in range
   __device__ __forceinline__ bool sum_again() const { return mx != 0 && !(l1 > 0x1p-100f && l1 < 0x1p110f); }
-  // the rebasing of that sum; the magnitudes of an exponent mx are then in [1, 2]
-  __device__ __forceinline__ int rebased() const { return (mx >> 20) - 127; }
-  // its result; lines of subnormal or with non-finite values keep theirs
+  // the result of that; lines of subnormal or with non-finite values keep theirs
   __device__ __forceinline__ void set_rebased(float sum) {
     const int e = mx >> 20;
     if (in_range() || e == 0 || e == 0x7ff) return;
@@ -133,9 +151,10 @@ struct Norm {
 // the transform
 __device__ __forceinline__ int scale(const Norm& n, int len_bits, int grow) {
   if (n.in_range()) {
-    // l1 (1 + 2^-6) < 2^X covers the rounding of the float sum
-    const int X = (__float_as_int(n.l1 * 1.015625f) >> 23) - 126;
-    return 62 - grow - X - n.base;
+    // l1 (1 + 2^-6) covers the rounding of the float sum; at most 1.3125 2^62,
+    // and 2^62 for the largest value (from_double)
+    const int X = (__float_as_int(n.l1 * (1.015625f / 1.3125f)) >> 23) - 126;
+    return min(62 - grow - X - n.base, 1084 - max(n.mx >> 20, 1));
   }
   // every value below 2^(e-1022), subnormal ones among them
   int e = n.mx >> 20;
@@ -319,7 +338,7 @@ __device__ __forceinline__ fx::Norm col_norm(int t, int c, EACH each) {
   }
   if (again) {
     float s = 0.f;
-    each([&](double2 v) { s += fx::mag(fx::hi_abs(v.x), r.rebased()) + fx::mag(fx::hi_abs(v.y), r.rebased()); });
+    each([&](double2 v) { s += r.rebased(v); });
     if constexpr (WARP) {
 #pragma unroll
       for (int o = NCOL; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -382,7 +401,7 @@ __device__ __forceinline__ fx::Norm line_norm(int t, int lg, SYNC sync, EACH eac
   each([&](double2 v) { n.add(v); });
   auto again = [&](const fx::Norm& m) {
     float s = 0.f;
-    each([&](double2 v) { s += fx::mag(fx::hi_abs(v.x), m.rebased()) + fx::mag(fx::hi_abs(v.y), m.rebased()); });
+    each([&](double2 v) { s += m.rebased(v); });
     return s;
   };
   if constexpr (std::is_same<SYNC, SyncWarp>::value) {

@@ -152,3 +152,86 @@ def test_powers_of_two_factor_out(ctx, n, kind):
     for shift in (-400, -130, -104, 120, 400):
         for a, b in zip(run(shift), want):
             assert np.array_equal(a, b), shift
+
+
+# relative L2 that FP64 butterflies leave of the product below, measured
+BUTTERFLIES = {64: 3.1e-16, 96: 3.6e-16, 128: 5.0e-16, 192: 5.5e-16, 256: 3.4e-16, 384: 3.8e-16, 512: 5.8e-16}
+
+
+@pytest.mark.parametrize("n", list(BUTTERFLIES))
+@pytest.mark.parametrize("amp", [8, 12, 13])
+def test_products_are_as_accurate_as_butterflies(ctx, n, amp):
+    """A product with a field of one mode is the other field shifted both ways:
+    exact sums of 53-bit values here but for the normalisation.  The error of the
+    fixed-point lines depends on the amplitude (the scale is a power of two)."""
+    import monofonic_gb300 as mf
+    rng = np.random.default_rng(n)
+    h = n // 2
+    s = np.zeros((n, n, h + 1), complex)
+    s.real[:, :, 1:h] = rng.integers(-2 ** 48, 2 ** 48, size=(n, n, h - 1))
+    s.imag[:, :, 1:h] = rng.integers(-2 ** 48, 2 ** 48, size=(n, n, h - 1))
+    s[h] = s[:, h] = 0
+    s *= amp
+    f, g, out = (mf.Grid_FFT(ctx, n, 1.0, "f64", "k") for _ in range(3))
+    f.set_k(s)
+    q = np.zeros_like(s)
+    q[1, 1, 0] = q[-1, -1, 0] = 1
+    g.set_k(q)
+    mf.OrszagConvolver(ctx, n, 1.0, "f64").multiply_field(f, g, mf.op.assign_to(out))
+    got = out.get_k()
+    want = (np.roll(s, (1, 1), (0, 1)) + np.roll(s, (-1, -1), (0, 1))) / np.sqrt(float(n) ** 3)
+    for a in (got, want):
+        a[h] = a[:, h] = a[:, :, h] = 0
+    assert np.linalg.norm(got - want) <= BUTTERFLIES[n] * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("n, trials", [(16, 40), (32, 40), (64, 20), (96, 10), (128, 6), (192, 3), (256, 2), (512, 1)])
+def test_coherent_lines_do_not_overflow(ctx, n, trials):
+    """Lines whose values add up in phase reach the bound that the scale is set
+    by: single waves forward, single cells backward, and the product of two
+    cells' fields, at amplitudes all over an octave.  An overflow is an error
+    of order one; the bound is that of the other accuracy tests."""
+    import monofonic_gb300 as mf
+    rng = np.random.default_rng(n)
+    g, out = mf.Grid_FFT(ctx, n, 1.0, "f64"), mf.Grid_FFT(ctx, n, 1.0, "f64", "k")
+    cvs = [c(ctx, n, 1.0, "f64") for c in (mf.OrszagConvolver, mf.NaiveConvolver)]
+    w = 2 * np.pi * np.arange(n) / n
+    h = n // 2
+    norm = np.linalg.norm
+
+    def wave(p, sign, phase):
+        """exp(i sign (p . index) 2 pi / n + i phase)"""
+        a = [np.exp(1j * sign * ((p[d] * np.arange(n)) % n) * (2 * np.pi / n)) for d in range(3)]
+        return a[0][:, None, None] * a[1][None, :, None] * a[2][None, None, :] * np.exp(1j * phase)
+
+    for _ in range(trials):
+        amp, phase = 2 ** rng.uniform(0, 1), rng.integers(0, 8) * np.pi / 4
+        b = rng.integers(0, n, 3)
+        b[2] = rng.integers(1, h)
+        g.set_real(amp * wave(b, 1, phase).real)
+        g.FourierTransformForward()
+        k = g.get_k()
+        want = np.zeros_like(k)
+        want[tuple(b)] = amp / 2 * np.exp(1j * phase) * np.sqrt(float(n) ** 3)
+        assert norm(k - want) <= 4e-15 * norm(want)
+        # a cell: every mode has the same modulus (cells on even sites: the Nyquist planes are real)
+        p = 2 * rng.integers(0, h, 3)
+        cell = amp * wave(p, -1, 0.0)[:, :, : h + 1]
+        g.set_k(cell)
+        g.FourierTransformBackward()
+        r = g.get_real()
+        want = np.zeros_like(r)
+        want[tuple(p)] = amp * np.sqrt(float(n) ** 3)
+        assert norm(r - want) <= 4e-15 * norm(want)
+        g.set_k(cell)
+        cvs[1].multiply_field(g, g, mf.op.assign_to(out))
+        want = cell * (amp * np.sqrt(float(n) ** 3))
+        assert norm(out.get_k() - want) <= 8e-15 * norm(want)
+        cell[h] = cell[:, h] = cell[:, :, h] = 0  # padded: the modes with |K - k| < N/2 on every axis add up
+        g.set_k(cell)
+        cvs[0].multiply_field(g, g, mf.op.assign_to(out))
+        count = n - 1 - np.abs(np.fft.fftfreq(n) * n)
+        want = cell * (amp / np.sqrt(float(n) ** 3)) * (
+            count[:, None, None] * count[None, :, None] * count[None, None, : h + 1])
+        assert norm(out.get_k() - want) <= 8e-15 * norm(want)
+        g.set_real(np.zeros((n, n, n)))
