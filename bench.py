@@ -137,11 +137,11 @@ class Clocks:
 def algorithmic_bytes_ic(n: int, prec_bytes: int, overload: int = 2, plt: bool = True) -> dict:
     """Unique bytes each kernel kind must read and write for one 3LPT IC of the
     shared-source pipeline (each element once; re-reads not counted):
-    17 operands through the padded c2r (y and z passes; three x passes
-    per field for its six Hessians; the five pair products' x passes are their
-    truncations), 10 product sums through the padded r2c (z and y passes;
-    x passes of five, and the five truncations), the streaming source products,
-    and the assembly of `overload` sub-lattices for positions and velocities."""
+    17 operands through the padded c2r (y and z passes; one x launch of three
+    transforms per field for its six Hessians, whose second y launch reads two
+    of them; the five pair products' x passes are their truncations), 10 product
+    sums through the padded r2c (z and y passes; x passes of five, and the five
+    truncations), the streaming source products, and the assembly of `overload` sub-lattices for positions and velocities."""
     cs = 2 * prec_bytes
     M, Kz = 3 * n // 2, n // 2 + 1
     S_NK, S_MNK, S_MMK = n * n * Kz * cs, M * n * Kz * cs, M * M * Kz * cs
@@ -149,8 +149,8 @@ def algorithmic_bytes_ic(n: int, prec_bytes: int, overload: int = 2, plt: bool =
     S_N = n * n * (n + 2) * prec_bytes  # N-grid
     npart = overload * n ** 3
     out = {
-        "conv_xinv": 6 * (S_NK + S_MNK),
-        "conv_yinv": 17 * (S_MNK + S_MMK),
+        "conv_xinv": 2 * (S_NK + 3 * S_MNK),
+        "conv_yinv": 2 * (5 * S_MNK + 6 * S_MMK) + 5 * (S_MNK + S_MMK),
         "conv_z": 27 * (S_MMK + S_R),
         "conv_yfwd": 10 * (S_MMK + S_MNK),
         "conv_xfwd": 5 * (S_MNK + S_NK) + 5 * 2 * S_MNK,
