@@ -141,7 +141,8 @@ def algorithmic_bytes_ic(n: int, prec_bytes: int, overload: int = 2, plt: bool =
     transforms per field for its six Hessians, whose second y launch reads two
     of them; the five pair products' x passes are their truncations), 10 product
     sums through the padded r2c (z and y passes; x passes of five, and the five
-    truncations), the streaming source products, and the assembly of `overload` sub-lattices for positions and velocities."""
+    truncations), the streaming source products, and the assembly of `overload`
+    sub-lattices for positions and velocities."""
     cs = 2 * prec_bytes
     M, Kz = 3 * n // 2, n // 2 + 1
     S_NK, S_MNK, S_MMK = n * n * Kz * cs, M * n * Kz * cs, M * M * Kz * cs

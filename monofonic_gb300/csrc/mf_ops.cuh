@@ -44,23 +44,11 @@ struct Operand {
   int d[4];
 };
 
-__device__ __forceinline__ int sel3(int d, int i, int j, int k) { return d == 0 ? i : (d == 1 ? j : k); }
-
 struct ConvGeom {
   int N;       // unpadded size
   int M;       // padded size (3N/2, or N for the aliased convolver)
   int Kz;      // N/2 + 1 stored kz columns
   bool orszag;
-  // padded row index -> source row, -1 in the zero gap
-  __device__ __forceinline__ int src_row(int x) const {
-    if (!orszag) return x;
-    if (x <= (N >> 1)) return x;
-    if (x > N) return x - (N >> 1);
-    return -1;
-  }
-  // padded row kept by unpad -> original row, -1 otherwise
-  __device__ __forceinline__ int kept_row(int x) const { return src_row(x); }
-  __device__ __forceinline__ long long row_off(int x, long long stride) const { return (long long)src_row(x) * stride; }
 };
 
 // index of an element along a transform: t, from the thread, in [0, TPL), plus
@@ -83,16 +71,18 @@ __device__ __forceinline__ long long idx_off(LineIdx<TPL> x, long long stride) {
 // padded axis (M = L): Orszag 3/2 (N = 2L/3) or the aliased convolver
 // (N = L).  The strided passes are launched with it, so that their per-element
 // row maps and addresses fold into immediates (about a quarter fewer
-// instructions per element of the length-768 passes than with ConvGeom).
+// instructions per element of the length-768 passes than with a run-time one).
 template <int L, bool ORSZAG>
 struct CGeom {
   static constexpr int M = L;
   static constexpr int N = ORSZAG ? 2 * L / 3 : L;
   static constexpr int Kz = N / 2 + 1;
   static constexpr bool orszag = ORSZAG;
+  // padded row index -> source row, -1 in the zero gap
   __device__ __forceinline__ static constexpr int src_row(int x) {
     return !ORSZAG ? x : (x <= (N >> 1) ? x : (x > N ? x - (N >> 1) : -1));
   }
+  // padded row kept by unpad -> original row, -1 otherwise
   __device__ __forceinline__ static constexpr int kept_row(int x) { return src_row(x); }
   template <int TPL>
   __device__ __forceinline__ static int src_row(LineIdx<TPL> x) {
