@@ -80,11 +80,18 @@ constexpr int pipe_ncol() {
 // whether a strided pass takes the two-stage kernels
 template <typename T, int L>
 constexpr bool two_stage() { return sizeof(T) == 4 && col2_r1(L) > 0; }
-// columns per tile of the two-stage passes: 128-byte rows (16) for length 256 and
-// for the N-grid passes of length 384, where two tiles of a CTA leave room for
-// enough CTAs; else 64-byte rows.  Measured, 16 against 8 columns: five aliased
-// products at N=256 1309 / 1430 us, a 384^3 field 1138 / 1173 us, but padded
-// products at N=256 (length 384) 2158 / 2098 us, at N=128 (192) 388 / 370 us.
+// columns per tile of the two-stage passes: 128-byte rows (16) at length 256 and in
+// the N-grid passes of length 384, else 64-byte rows (8).  Measured, 8 / 16 columns
+// in every pass of the length, us:
+//   a forward and a backward transform: L = 128 44.6 / 45.2, 192 101.9 / 98.1,
+//     256 199 / 184, 384 664 / 628, 512 1531 / 1480
+//   an aliased product: 128 47.6 / 50.3, 192 126 / 125, 256 313 / 252, 384 986 / 975,
+//     512 2083 / 2008
+//   a padded product: 144 53.2 / 53.3, 192 72.4 / 75.8, 288 270 / 297, 384 519 / 532,
+//     576 2619 / 2118, 768 4650 / 4330
+// Wider rows are longer runs of memory but fewer CTAs per SM; which one counts was
+// measured, not derived.  512, 576 and 768, faster at 16 as well, stay at 8
+// until whole runs are compared there.
 template <int L, class OP>
 constexpr int col2_cols() { return (L == 256 || (L == 384 && plain_op<OP>::value)) ? 16 : 8; }
 
