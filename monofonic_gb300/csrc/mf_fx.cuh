@@ -21,7 +21,7 @@
 // the L1 norm, which for L white values is 1.25 L of one's r.m.s.; the one or two
 // bits of growth of the real transforms make it two or four times as large.
 // Measured, relative L2 of a product with a field of one mode, the largest of
-// eight amplitudes, and what FP64 butterflies left: N=64 1.3e-16 / 3.1e-16, 128
+// eight amplitudes, and what FP64 butterflies left: N=64 1.3e-16 / 3.2e-16, 128
 // 3.8 / 5.1, 256 1.3 / 3.5, 384 2.2 / 3.9, 512 (L = 768) 5.4 / 5.9.  With the norm
 // from |re| + |im| at 2^62 it was 7.1e-16 at N=512, more than the butterflies.
 //
