@@ -195,7 +195,6 @@ def test_coherent_lines_do_not_overflow(ctx, n, trials):
     rng = np.random.default_rng(n)
     g, out = mf.Grid_FFT(ctx, n, 1.0, "f64"), mf.Grid_FFT(ctx, n, 1.0, "f64", "k")
     cvs = [c(ctx, n, 1.0, "f64") for c in (mf.OrszagConvolver, mf.NaiveConvolver)]
-    w = 2 * np.pi * np.arange(n) / n
     h = n // 2
     norm = np.linalg.norm
 
@@ -204,8 +203,10 @@ def test_coherent_lines_do_not_overflow(ctx, n, trials):
         a = [np.exp(1j * sign * ((p[d] * np.arange(n)) % n) * (2 * np.pi / n)) for d in range(3)]
         return a[0][:, None, None] * a[1][None, :, None] * a[2][None, None, :] * np.exp(1j * phase)
 
-    for _ in range(trials):
+    for trial in range(trials):
         amp, phase = 2 ** rng.uniform(0, 1), rng.integers(0, 8) * np.pi / 4
+        if trial % 2 == 0:  # a single mode at the top of a scale (1.3125 / 1.015625), its components equal
+            amp, phase = 1.2922, np.pi / 4 + (trial // 2) % 4 * np.pi / 2
         b = rng.integers(0, n, 3)
         b[2] = rng.integers(1, h)
         g.set_real(amp * wave(b, 1, phase).real)
@@ -214,6 +215,10 @@ def test_coherent_lines_do_not_overflow(ctx, n, trials):
         want = np.zeros_like(k)
         want[tuple(b)] = amp / 2 * np.exp(1j * phase) * np.sqrt(float(n) ** 3)
         assert norm(k - want) <= 4e-15 * norm(want)
+        g.set_k(want)
+        g.FourierTransformBackward()
+        want = amp * wave(b, 1, phase).real
+        assert norm(g.get_real() - want) <= 4e-15 * norm(want)
         # a cell: every mode has the same modulus (cells on even sites: the Nyquist planes are real)
         p = 2 * rng.integers(0, h, 3)
         cell = amp * wave(p, -1, 0.0)[:, :, : h + 1]
